@@ -163,6 +163,27 @@ struct BarrierTest {
   int withhold_cta;
   unsigned spin_limit;
 };
+// ---- cluster solve (k_cluster.cu) --------------------------------------------
+// Plan rows = 5: the whole solve in one launch of one thread-block cluster of
+// plan.xc CTAs, the iterate in their shared memory.  Any sz.  Bit for bit the
+// other plans.
+long long cluster_solve_units(const Dims& d);  // units of 2 x 1 x 4 cells: entries of umap and list
+int cluster_solve_width(const Dims& d);   // CTAs of the default plan
+bool cluster_solve_takes(const Dims& d, int width);               // the launch's limits
+bool cluster_solve_fits(const Dims& d, long long particles);      // the default plan's rule
+// fixed_sweeps > 0: that many sweeps then one residual; else residual mode.
+// part: one double per 32 units.  Starts from pa, result in pa.  r2_only (may
+// be null): the squared residual goes there and *ss is only read.
+cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, float* pb, const float* rhs,
+                                 const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
+                                 int fixed_sweeps, int check, int max_iters, double tol, double* r2_only);
+// The same for scenes order[0 .. scenes) of a batch, one cluster each;
+// scratch[s]: scene s's first entry in umap and list, and in part.
+int batch_cluster_width(const Dims& d, long long particles);  // 0: the scene does not fit a cluster
+cudaError_t launch_batch_cluster_solve(cudaStream_t st, const BatchIndex& bi, int scenes, int width, const int* order,
+                                       const int2* scratch, float* pa, float* pb, const float* rhs,
+                                       const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
+                                       int fixed_sweeps, int check, int max_iters, double tol);
 // ---- resident solve (k_resident.cu) ------------------------------------------
 // Plan rows = 4: the whole solve in one cooperative launch, one CTA per SM;
 // a CTA keeps a tile (plan.xc selects the TX x TY x TZ shape) plus a K-cell

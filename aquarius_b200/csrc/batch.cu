@@ -76,6 +76,18 @@ struct aq_batch {
   int* n_row_list = nullptr;
   int row_list_cap = 0;
 
+  // Cluster solve (when every scene fits one): scenes by cluster width, largest
+  // first; each width is a launch on a stream of its own inside the step.
+  static constexpr int kWidths = 5;  // 1, 2, 4, 8, 16 CTAs
+  bool clusters = false;
+  int cl_first[kWidths + 1] = {0};
+  int* cl_order = nullptr;
+  int2* cl_scratch = nullptr;
+  int *cl_map = nullptr, *cl_list = nullptr;
+  double* cl_part = nullptr;
+  cudaStream_t cl_stream[kWidths] = {nullptr};
+  cudaEvent_t cl_event[kWidths + 1] = {nullptr};
+
   Particles cur{}, tmp{};
   int *key = nullptr, *slot = nullptr, *perm_u = nullptr, *sort_index = nullptr;
   int *count = nullptr, *off = nullptr, *tile_sums = nullptr;
@@ -100,6 +112,10 @@ struct aq_batch {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
     if (exec) cudaGraphExecDestroy(exec);
+    for (cudaEvent_t e : cl_event)
+      if (e) cudaEventDestroy(e);
+    for (cudaStream_t q : cl_stream)
+      if (q) cudaStreamDestroy(q);
     for (void* p : allocs) cudaFree(p);
     if (own_stream && stream) cudaStreamDestroy(stream);
   }
@@ -129,6 +145,8 @@ struct aq_batch {
   }
 
   aq_status allocate();
+  aq_status plan_clusters();
+  aq_status enq_clusters();
   aq_status add_scene(int s, aq_fluid* f);
   aq_status enq_pre_solve();
   aq_status enq_sweeps(int sweeps);
@@ -182,7 +200,63 @@ aq_status aq_batch::allocate() {
   bi.slayer = pre_d + 3 * (ns + 1);
   bi.flat = pre_d + 4 * (ns + 1);
   bi.rows = pre_d + 5 * (ns + 1);
+  AQB_TRY(plan_clusters());
   return set_sweep_plan(xs, pipe);
+}
+
+// Sorts the scenes into clusters of 1 to 16 CTAs, if each fits one.
+aq_status aq_batch::plan_clusters() {
+  std::vector<std::vector<int>> by(kWidths);
+  std::vector<int2> scratch((size_t)ns);
+  long long units = 0, parts = 0;
+  for (int s = 0; s < ns; ++s) {
+    const SceneDesc& S = scenes[s];
+    const int w = batch_cluster_width(S.d, S.n);
+    if (w == 0) return AQ_OK;
+    int k = 0;
+    while ((1 << k) < w) ++k;
+    by[k].push_back(s);
+    scratch[s] = make_int2((int)units, (int)parts);
+    const long long u = cluster_solve_units(S.d);
+    units += u;
+    parts += u / 32 + 1;
+  }
+  std::vector<int> order;
+  for (int k = 0; k < kWidths; ++k) {
+    std::stable_sort(by[k].begin(), by[k].end(), [&](int a, int b) { return scenes[a].n > scenes[b].n; });
+    cl_first[k] = (int)order.size();
+    order.insert(order.end(), by[k].begin(), by[k].end());
+    if (!by[k].empty()) AQB_CUDA(cudaStreamCreateWithFlags(&cl_stream[k], cudaStreamNonBlocking));
+  }
+  cl_first[kWidths] = ns;
+  for (cudaEvent_t& e : cl_event) AQB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  AQB_TRY(alloc(&cl_order, (size_t)ns));
+  AQB_TRY(alloc(&cl_scratch, (size_t)ns));
+  AQB_TRY(alloc(&cl_map, (size_t)units));
+  AQB_TRY(alloc(&cl_list, (size_t)units));
+  AQB_TRY(alloc(&cl_part, (size_t)parts));
+  AQB_CUDA(cudaMemcpyAsync(cl_order, order.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, stream));
+  AQB_CUDA(cudaMemcpyAsync(cl_scratch, scratch.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, stream));
+  AQB_CUDA(cudaStreamSynchronize(stream));
+  clusters = true;
+  return AQ_OK;
+}
+
+// The solves of all scenes; widest clusters first.
+aq_status aq_batch::enq_clusters() {
+  const int fixed = solver.solve_mode == AQ_SOLVE_RESIDUAL ? 0 : solver.pressure_iterations;
+  AQB_CUDA(cudaEventRecord(cl_event[kWidths], stream));
+  for (int k = kWidths - 1; k >= 0; --k) {
+    const int n = cl_first[k + 1] - cl_first[k];
+    if (n == 0) continue;
+    AQB_CUDA(cudaStreamWaitEvent(cl_stream[k], cl_event[kWidths], 0));
+    AQB_CUDA(launch_batch_cluster_solve(cl_stream[k], bi, n, 1 << k, cl_order + cl_first[k], cl_scratch, pa, pb, rhs,
+                                        type, cl_map, cl_list, cl_part, ss, fixed, solver.check_interval,
+                                        solver.max_iterations, (double)solver.rel_residual));
+    AQB_CUDA(cudaEventRecord(cl_event[k], cl_stream[k]));
+    AQB_CUDA(cudaStreamWaitEvent(stream, cl_event[k], 0));
+  }
+  return AQ_OK;
 }
 
 // Packed-row Jacobi items depend on the x planes per item: rebuild their
@@ -252,7 +326,7 @@ aq_status aq_batch::enq_pre_solve() {
   AQB_CUDA(launch_batch_divergence(stream, bi, tb, grid512(), off, type, density, un1, vn1, wn1, pcount, div, rhs,
                                    pa, pb, solver.pressure_init == AQ_PRESSURE_ZERO, bact, part_b2, part_nf));
   AQB_CUDA(launch_batch_b2_finalize(stream, bi, part_b2, part_nf, ss, live));
-  AQB_TRY(enq_row_list());
+  if (!clusters) AQB_TRY(enq_row_list());
   return AQ_OK;
 }
 
@@ -269,6 +343,7 @@ aq_status aq_batch::enq_sweeps(int sweeps) {
 aq_status aq_batch::enq_solve_fixed() {
   const int K = solver.pressure_iterations;
   if (K <= 0) return AQ_OK;
+  if (clusters) return enq_clusters();
   AQB_TRY(enq_sweeps(K));
   AQB_CUDA(launch_batch_resid_flat(stream, bi, pre_f[ns], grid(), live, K % 2 ? pb : pa, rhs, type, bact, rpart));
   if (K % 2) {
@@ -312,10 +387,22 @@ aq_status aq_batch::build_graph() {
     if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
     return AQ_OK;
   };
+  // counted as the row sweeps run; the cluster solve does a step's blocks in
+  // one launch per cluster width instead
   const int pre_launches = (N > 0 ? 6 : 3) + 5;  // sort; p2g, s-layer, divergence, b2, row list
   const int post_launches = 4;
   aq_status st;
-  if (solver.solve_mode == AQ_SOLVE_RESIDUAL) {
+  if (solver.solve_mode == AQ_SOLVE_RESIDUAL && clusters) {
+    st = capture(g, nullptr, 0, [&]() {
+      aq_status s2 = enq_pre_solve();
+      if (s2 != AQ_OK) return s2;
+      s2 = enq_clusters();
+      if (s2 != AQ_OK) return s2;
+      return enq_post_solve();
+    });
+    body_launches = solver.check_interval + 3;
+    graph_launches = pre_launches + post_launches;
+  } else if (solver.solve_mode == AQ_SOLVE_RESIDUAL) {
     st = capture(g, nullptr, 0, [&]() { return enq_pre_solve(); });
     if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
     size_t nn = 0;
@@ -678,6 +765,7 @@ aq_status aq_batch_benchmark_pressure(aq_batch* b, int32_t sweeps, float* ms, in
   // every scene takes part
   std::vector<int> ones((size_t)b->ns, 1);
   AQB_CUDA(cudaMemcpyAsync(b->live, ones.data(), sizeof(int) * ones.size(), cudaMemcpyHostToDevice, b->stream));
+  AQB_TRY(b->enq_row_list());  // the row sweeps are timed, whichever solve the steps use
   AQB_CUDA(cudaStreamSynchronize(b->stream));
   const int k = sweeps + (sweeps % 2);  // even: the iterate stays in pa
   AQB_CUDA(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));

@@ -235,6 +235,9 @@ aq_status aqb::set_last_error(aq_status st, const std::string& msg) {
 // last launch as an extra level.
 static bool separate_residual(const aqb::JacobiPlan& p) { return p.by == 0 || p.by == 2 || p.by == 3; }
 
+// Plans that run the whole solve in one launch.
+static bool whole_solve(const aqb::JacobiPlan& p) { return p.by == 1 || p.by == 4 || p.by == 5; }
+
 // =================================================================== fluid
 // ------------------------------------------------------------- allocation
 aq_status aq_fluid::allocate() {
@@ -301,7 +304,20 @@ aq_status aq_fluid::allocate() {
     AQ_TRY(alloc(&jpart, (size_t)jpart_cap));
   }
   memset(ss_host, 0, sizeof(SolveState));
+  // small grids: the whole solve in one thread-block cluster
+  if (cluster_solve_fits(d, n)) {
+    AQ_TRY(alloc_cluster());
+    plan = JacobiPlan{1, 5, cluster_solve_width(d)};
+  }
   return AQ_OK;
+}
+
+aq_status aq_fluid::alloc_cluster() {
+  if (cl_map) return AQ_OK;
+  const size_t q = (size_t)cluster_solve_units(d);
+  AQ_TRY(alloc(&cl_list, q));
+  AQ_TRY(alloc(&cl_part, q / 32 + 1));
+  return alloc(&cl_map, q);
 }
 
 // ------------------------------------------------------------------ stages
@@ -347,6 +363,7 @@ static std::vector<int> split_sweeps(int sweeps, int levels) {
 
 static int jacobi_launches(const JacobiPlan& plan, int sweeps) {
   if (plan.by == 1 || plan.by == 4) return 2;  // work list + the cooperative solve
+  if (plan.by == 5) return 1;
   const int k = (int)split_sweeps(sweeps, plan.levels).size();
   // sweeps, parity copy, finalize, separate residual pass (flat, cube and list plans)
   return k + (k % 2) + 1 + (separate_residual(plan) ? 1 : 0);
@@ -419,14 +436,21 @@ int aq_fluid::solve_sweeps_done() const { return cfg.pressure_init == AQ_PRESSUR
 aq_status aq_fluid::enq_learned_start() {
   if (!net || !net_acts) return fail(AQ_ERR_INVALID_CONFIG, "AQ_PRESSURE_LEARNED needs a network (aq_fluid_set_warm_start)");
   AQ_TRY(unet_predict(net, stream, net_acts, rhs, type, pa));
-  // the two short starts run one sweep per launch (the list plan) when the
-  // solve itself is the resident plan
-  const JacobiPlan wp = plan.by == 4 ? JacobiPlan{1, 3, 1} : plan;
-  AQ_TRY(enqueue_sweeps_on(this, wp, pa, pb, kWarmSweeps, true, jpart));
+  // the two short starts: a cluster solve each where that is the plan, else
+  // one sweep per launch (the list plan when the solve itself is one launch)
+  const JacobiPlan wp = whole_solve(plan) ? JacobiPlan{1, 3, 1} : plan;
+  const bool cluster = plan.by == 5;
+  auto start = [&](float* a, float* b, double* part) -> aq_status {
+    if (!cluster) return enqueue_sweeps_on(this, wp, a, b, kWarmSweeps, true, part);
+    AQ_CUDA(launch_cluster_solve(stream, d, plan.xc, a, b, rhs, type, cl_map, cl_list, cl_part, ss, kWarmSweeps, 0, 0,
+                                 0.0, part));
+    return AQ_OK;
+  };
+  AQ_TRY(start(pa, pb, jpart));
   AQ_CUDA(cudaMemsetAsync(za, 0, sizeof(float) * d.C, stream));
   AQ_CUDA(cudaMemsetAsync(zb, 0, sizeof(float) * d.C, stream));
-  AQ_TRY(enqueue_sweeps_on(this, wp, za, zb, kWarmSweeps, true, jpart2));
-  k_pick_start<<<1, 1024, 0, stream>>>(jpart, jpart2, last_parts_of(this, wp, kWarmSweeps), ss, pick,
+  AQ_TRY(start(za, zb, jpart2));
+  k_pick_start<<<1, 1024, 0, stream>>>(jpart, jpart2, cluster ? 1 : last_parts_of(this, wp, kWarmSweeps), ss, pick,
                                        cfg.solve_mode == AQ_SOLVE_RESIDUAL ? (double)cfg.rel_residual : 0.0);
   AQ_CUDA(cudaGetLastError());
   k_copy_if<<<std::min((d.C + 255) / 256, 148 * 8), 256, 0, stream>>>(pick, za, pa, d.C);
@@ -452,10 +476,24 @@ static aq_status enqueue_resident(aq_fluid* f, int fixed_sweeps) {
   return AQ_OK;
 }
 
+// The whole solve as one launch of one cluster (plan.by == 5).
+static aq_status enqueue_cluster(aq_fluid* f, int fixed_sweeps) {
+  AQ_CUDA(launch_cluster_solve(f->stream, f->d, f->plan.xc, f->pa, f->pb, f->rhs, f->type, f->cl_map, f->cl_list,
+                               f->cl_part, f->ss, fixed_sweeps, f->cfg.check_interval, f->cfg.max_iterations,
+                               (double)f->cfg.rel_residual, nullptr));
+  return AQ_OK;
+}
+
+// A plan that is one launch: fixed_sweeps sweeps, or (0) residual mode.
+static aq_status enqueue_whole(aq_fluid* f, int fixed_sweeps) {
+  return f->plan.by == 1   ? enqueue_persistent(f, fixed_sweeps)
+         : f->plan.by == 4 ? enqueue_resident(f, fixed_sweeps)
+                           : enqueue_cluster(f, fixed_sweeps);
+}
+
 aq_status aq_fluid::enq_solve_fixed(int sweeps) {
   if (sweeps <= 0) return AQ_OK;
-  if (plan.by == 1) return enqueue_persistent(this, sweeps);
-  if (plan.by == 4) return enqueue_resident(this, sweeps);
+  if (whole_solve(plan)) return enqueue_whole(this, sweeps);
   AQ_TRY(enqueue_sweeps(this, sweeps));
   AQ_CUDA(launch_resid_finalize(stream, jpart, last_parts(this, sweeps), ss, sweeps, 0.0, 0, false, 0));
   return AQ_OK;
@@ -484,8 +522,7 @@ aq_status aq_fluid::enq_solve_body(bool set_cond, unsigned long long handle, int
 
 // Residual mode without a graph: the host reads the solve state after each block.
 aq_status aq_fluid::enq_solve_residual_eager() {
-  if (plan.by == 1) return enqueue_persistent(this, 0);
-  if (plan.by == 4) return enqueue_resident(this, 0);
+  if (whole_solve(plan)) return enqueue_whole(this, 0);
   for (int guard = 0; guard < 1000000; ++guard) {
     AQ_TRY(enq_solve_body(false, 0, nullptr));
     AQ_CUDA(cudaMemcpyAsync(ss_host, ss, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
@@ -668,15 +705,15 @@ aq_status aq_fluid::build_graph() {
   };
   aq_status st = AQ_OK;
   launches += (n > 0 ? 6 : 3) + 2 + 2;  // particles (+3 scan kernels), p2g, slayer, divergence, b2
-  if (cfg.solve_mode == AQ_SOLVE_RESIDUAL && (plan.by == 1 || plan.by == 4)) {
+  if (cfg.solve_mode == AQ_SOLVE_RESIDUAL && whole_solve(plan)) {
     st = capture(g, nullptr, 0, [&]() {
       aq_status s2 = enq_pre_solve();
       if (s2 != AQ_OK) return s2;
-      s2 = plan.by == 1 ? enqueue_persistent(this, 0) : enqueue_resident(this, 0);
+      s2 = enqueue_whole(this, 0);
       if (s2 != AQ_OK) return s2;
       return enq_post_solve();
     });
-    launches += 2;
+    launches += count_jacobi_launches(0);
     body_launches = 0;
   } else if (cfg.solve_mode == AQ_SOLVE_RESIDUAL) {
     st = capture(g, nullptr, 0, [&]() { return enq_pre_solve(); });
@@ -718,7 +755,7 @@ aq_status aq_fluid::build_graph() {
   if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
   if (cfg.pressure_init == AQ_PRESSURE_LEARNED)  // network, two 20-sweep starts, pick, copy
     launches += kUNetForwardLaunches +
-                2 * (jacobi_launches(plan.by == 4 ? JacobiPlan{1, 3, 1} : plan, kWarmSweeps) - 1) + 2;
+                2 * (plan.by == 5 ? 1 : jacobi_launches(plan.by == 4 ? JacobiPlan{1, 3, 1} : plan, kWarmSweeps) - 1) + 2;
   launches += 1 + 3 + (multiphase ? cfg.diffusion_iterations : 0) + (ink_on && n_ink > 0 ? 1 : 0);
   graph_launches = launches;
   cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
@@ -1553,6 +1590,17 @@ aq_status aq_fluid_set_jacobi_plan(aq_fluid* f, int32_t levels, int32_t rows, in
     f->invalidate_graph();
     return AQ_OK;
   }
+  if (rows == 5) {  // one cluster of x_planes CTAs
+    if (levels != 1 || !cluster_solve_takes(f->d, x_planes))
+      return fail(AQ_ERR_INVALID_ARGUMENT,
+                  "the cluster plan is (1, 5, 1/2/4/8/16) and takes at most 16384 units of 2 x 1 x 4 cells per CTA");
+    cudaSetDevice(f->device);
+    AQ_CUDA(cudaStreamSynchronize(f->stream));
+    AQ_TRY(f->alloc_cluster());
+    f->plan = JacobiPlan{1, 5, x_planes};
+    f->invalidate_graph();
+    return AQ_OK;
+  }
   if (rows == 3) {  // list of active warp rows, one sweep per launch
     if (f->d.sz % 4 != 0 || levels != 1 || x_planes != 1)
       return fail(AQ_ERR_INVALID_ARGUMENT, "the list plan is (1, 3, 1) and needs sz % 4 == 0");
@@ -1634,9 +1682,7 @@ aq_status aq_fluid_benchmark_pressure(aq_fluid* f, int32_t sweeps, float* ms, in
   // The sweeps are captured into a graph and replayed, as inside a step.
   cudaGraph_t g = nullptr;
   AQ_CUDA(cudaStreamBeginCapture(f->stream, cudaStreamCaptureModeThreadLocal));
-  aq_status st = f->plan.by == 1   ? enqueue_persistent(f, sweeps)
-                 : f->plan.by == 4 ? enqueue_resident(f, sweeps)
-                                   : enqueue_sweeps(f, sweeps, false);
+  aq_status st = whole_solve(f->plan) ? enqueue_whole(f, sweeps) : enqueue_sweeps(f, sweeps, false);
   cudaGraph_t got = nullptr;
   cudaError_t ce = cudaStreamEndCapture(f->stream, &got);
   if (st != AQ_OK) { if (got) cudaGraphDestroy(got); return st; }
@@ -1662,13 +1708,13 @@ aq_status aq_fluid_benchmark_pressure(aq_fluid* f, int32_t sweeps, float* ms, in
   const std::vector<int> parts = split_sweeps(sweeps, f->plan.levels);
   if (ms) *ms = t;
   if (launches)
-    *launches = f->plan.by == 1 || f->plan.by == 4 ? 2 : (int32_t)(parts.size() + parts.size() % 2);
+    *launches = whole_solve(f->plan) ? jacobi_launches(f->plan, sweeps) : (int32_t)(parts.size() + parts.size() % 2);
   if (cells_per_sweep) {
     std::vector<uint8_t> act((size_t)f->nbricks);
     AQ_CUDA(cudaMemcpy(act.data(), f->bact, act.size(), cudaMemcpyDeviceToHost));
     *cells_per_sweep =
         f->plan.by == 4 ? resident_cells_updated(f->d, f->plan.xc, act.data())
-                        : jacobi_cells_updated(f->d, f->plan.by == 1 || f->plan.by == 3 ? JacobiPlan{1, 0, 1} : f->plan,
+                        : jacobi_cells_updated(f->d, f->plan.by == 1 || f->plan.by == 3 || f->plan.by == 5 ? JacobiPlan{1, 0, 1} : f->plan,
                                                act.data());
   }
   return AQ_OK;
@@ -1743,7 +1789,8 @@ aq_status aq_fluid_autotune(aq_fluid* f, int32_t sweeps_per_trial, const char* c
   }
   const int cands[][3] = {{1, 0, 1}, {1, 0, 2}, {1, 1, 1},  {1, 16, 8}, {2, 16, 16}, {2, 32, 16}, {4, 32, 16},
                           {2, 2, 8},  {3, 2, 8},  {4, 2, 8},  {2, 2, 16}, {4, 2, 16},  {1, 3, 1},   {4, 4, 0},
-                          {4, 4, 1},  {4, 4, 2},  {4, 4, 3},  {4, 4, 4},  {4, 4, 5},   {4, 4, 6}};
+                          {4, 4, 1},  {4, 4, 2},  {4, 4, 3},  {4, 4, 4},  {4, 4, 5},   {4, 4, 6},  {1, 5, 1},
+                          {1, 5, 8},  {1, 5, 16}};
   float best = 1e30f;
   int bestp[3] = {f->plan.levels, f->plan.by, f->plan.xc};
   for (const auto& c : cands) {

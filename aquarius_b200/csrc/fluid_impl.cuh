@@ -94,6 +94,9 @@ struct aq_fluid {
   int* tiles = nullptr;
   int* n_tiles = nullptr;
   int res_ctas = 0;
+  // cluster solve (plan rows 5): numbering of the fluid quads, residual partials
+  int *cl_map = nullptr, *cl_list = nullptr;
+  double* cl_part = nullptr;
 
   JacobiPlan plan{4, 16, 32};
   // learned warm start (AQ_PRESSURE_LEARNED)
@@ -154,6 +157,7 @@ struct aq_fluid {
   uint8_t* hb(int which) const { return which == 1 ? h1 : h2; }
 
   aq_status allocate();
+  aq_status alloc_cluster();
   aq_status seed_and_init();
   // stage enqueues (eager or under capture)
   aq_status enq_particles(bool move);

@@ -284,7 +284,10 @@ aq_status aq_selfcheck_division(int32_t device, uint64_t* mismatches);
  * 4 8x16x24, 5 24x16x24 cells, 6 8x40x24 with twice the threads) with a
  * `levels`-cell halo (4) in
  * shared memory for the whole solve and exchanges halos every `levels`
- * sweeps (sz % 4 == 0).  rows = 8, 16, 32:
+ * sweeps (sz % 4 == 0).  rows = 5: the whole solve in one launch of one
+ * thread-block cluster of x_planes (1, 2, 4, 8 or 16) CTAs with the iterate in
+ * their shared memory (levels 1, any sz, at most 16384 units of 2 x 1 x 4
+ * cells per CTA; the default where the fluid fits).  rows = 8, 16, 32:
  * the temporally blocked kernel with `levels` sweeps (1, 2, 4, 8) per launch
  * over tiles of that many rows and x_planes planes.  Chosen per grid by the
  * tuner; invalid plans are rejected. */
@@ -374,13 +377,17 @@ aq_status aq_batch_totals(const aq_batch* b, int64_t* cells, int64_t* nodes, int
  * (cell tables and sort indices relative to the scene). */
 aq_status aq_batch_download_scene(aq_batch* b, int32_t scene, aq_host_state* s);
 aq_status aq_batch_solve_stats(aq_batch* b, int32_t scene, aq_solve_stats* st);
-/* Kernel launches per step outside the residual loop, and per loop block. */
+/* Kernel launches per step outside the residual loop, and per loop block, of
+ * a step whose solve runs as row sweeps.  When every scene fits a
+ * thread-block cluster the step's whole solve is at most five launches (one
+ * per cluster size) instead, and no block launches anything. */
 aq_status aq_batch_launch_counts(const aq_batch* b, int32_t* per_step, int32_t* per_block);
 /* Caps every batched launch at multiple x SMs CTAs (default 64, i.e. as many
  * as are resident at once; a batched launch never exceeds one resident wave).
  * Results do not depend on it. */
 aq_status aq_batch_set_grid_multiple(aq_batch* b, int32_t multiple);
-/* Shape of the batched Jacobi sweep: x planes each warp streams (1, 2, 4 or
+/* Shape of the batched row sweep, which solves batches with a scene too large
+ * for a thread-block cluster: x planes each warp streams (1, 2, 4 or
  * 8; default 1) and, for more than one plane, whether the next plane's loads
  * are issued before the current plane's arithmetic.  Results do not depend
  * on it. */
