@@ -2,6 +2,8 @@
 // of its launch; all work is enqueued on `st`.
 #pragma once
 
+#include <cuda_bf16.h>
+
 #include <string>
 
 #include "../../include/aquarius_b200.h"
@@ -338,12 +340,14 @@ cudaError_t launch_absmax(cudaStream_t st, const float* a, int n, float* part /*
 cudaError_t launch_unet_input(cudaStream_t st, const float* rhs, const int8_t* type, const float* scale, void* out,
                               int V);
 cudaError_t launch_pool2(cudaStream_t st, const void* in, void* out, int sx, int sy, int sz, int C);
-cudaError_t launch_pool2_bwd(cudaStream_t st, const void* dout, void* din, int sx, int sy, int sz, int C,
-                             bool accumulate);
+// din += dout / 8, then relu'(y)
+cudaError_t launch_pool2_bwd(cudaStream_t st, const void* dout, void* din, const void* y, int sx, int sy, int sz,
+                             int C);
 cudaError_t launch_upcat(cudaStream_t st, const void* coarse, const void* skip, void* out, int sx, int sy, int sz,
                          int Cu, int Cs);
-cudaError_t launch_upcat_bwd(cudaStream_t st, const void* dout, void* dcoarse, void* dskip, int sx, int sy, int sz,
-                             int Cu, int Cs);
+// y: the coarse layer's output, whose ReLU dcoarse goes through
+cudaError_t launch_upcat_bwd(cudaStream_t st, const void* dout, void* dcoarse, const void* y, void* dskip, int sx,
+                             int sy, int sz, int Cu, int Cs);
 cudaError_t launch_relu_bwd(cudaStream_t st, void* dy, const void* y, int n);
 int chan_sum_parts(int V);
 cudaError_t launch_chan_sum(cudaStream_t st, const void* dy, int V, int C, float* part, float* out);
@@ -358,8 +362,23 @@ cudaError_t launch_unet_loss_bwd(cudaStream_t st, const float* out, const float*
                                  const void* h, const float* w, float alpha, int k, void* dh, int sx, int sy, int sz,
                                  float* e, float* p0, float* p1, float* p2, float* p3, float* g, float* part,
                                  float* sums, float* head_part, float* head_sums);
-cudaError_t launch_adam(cudaStream_t st, float* w, const float* g, float* m, float* v, int n, float lr, float b1,
-                        float b2, float eps, int t, void* wb);
+// The tensors of one Adam step, concatenated: tensor k holds elements first[k]
+// to first[k + 1].  wb and wt (may be null): bf16 copies of a weight tensor
+// [27][cout][cin], as it is and [26 - tap][cin][cout].
+struct AdamTensor {
+  float* w;
+  const float* g;
+  float *m, *v;
+  __nv_bfloat16 *wb, *wt;
+  int cin, cout;
+};
+struct AdamTensors {
+  static constexpr int kMax = 24;
+  AdamTensor t[kMax];
+  int first[kMax + 1];
+  int count;
+};
+cudaError_t launch_adam(cudaStream_t st, const AdamTensors& T, float lr, float b1, float b2, float eps, int t);
 cudaError_t launch_f32_to_bf16(cudaStream_t st, const float* a, void* b, int n);
 cudaError_t launch_unet_to_pressure(cudaStream_t st, const float* out, const float* scale, float out_scale,
                                     const int8_t* type, float* p, int V);

@@ -185,27 +185,22 @@ aq_status backward(aq_unet* net, cudaStream_t st, UActs* a, const float* target,
   const int V = sx * sy * sz, V2 = V / 8, V4 = V / 64;
   UN_CUDA(launch_unet_loss_bwd(st, a->out, target, type, a->d1, net->hp, alpha, k, a->g_d1, sx, sy, sz, a->le, a->l0,
                                a->l1, a->l2, a->l3, a->lg, a->lpart, a->lsums, a->hpart, net->hg));
-  UN_CUDA(launch_relu_bwd(st, a->g_d1, a->d1, V * 16));
   UN_TRY(conv_bwd(net, st, a, 9, a->d1a, a->g_d1, a->g_d1a, sx, sy, sz));
   UN_CUDA(launch_relu_bwd(st, a->g_d1a, a->d1a, V * 16));
   UN_TRY(conv_bwd(net, st, a, 8, a->u1, a->g_d1a, a->g_u1, sx, sy, sz));
-  UN_CUDA(launch_upcat_bwd(st, a->g_u1, a->g_d2, a->g_e1, sx, sy, sz, 32, 16));
-  UN_CUDA(launch_relu_bwd(st, a->g_d2, a->d2, V2 * 32));
+  UN_CUDA(launch_upcat_bwd(st, a->g_u1, a->g_d2, a->d2, a->g_e1, sx, sy, sz, 32, 16));
   UN_TRY(conv_bwd(net, st, a, 7, a->d2a, a->g_d2, a->g_d2a, hx, hy, hz));
   UN_CUDA(launch_relu_bwd(st, a->g_d2a, a->d2a, V2 * 32));
   UN_TRY(conv_bwd(net, st, a, 6, a->u2, a->g_d2a, a->g_u2, hx, hy, hz));
-  UN_CUDA(launch_upcat_bwd(st, a->g_u2, a->g_b2, a->g_e2, hx, hy, hz, 64, 32));
-  UN_CUDA(launch_relu_bwd(st, a->g_b2, a->b2, V4 * 64));
+  UN_CUDA(launch_upcat_bwd(st, a->g_u2, a->g_b2, a->b2, a->g_e2, hx, hy, hz, 64, 32));
   UN_TRY(conv_bwd(net, st, a, 5, a->b1, a->g_b2, a->g_b1, qx, qy, qz));
   UN_CUDA(launch_relu_bwd(st, a->g_b1, a->b1, V4 * 64));
   UN_TRY(conv_bwd(net, st, a, 4, a->p2, a->g_b1, a->g_p2, qx, qy, qz));
-  UN_CUDA(launch_pool2_bwd(st, a->g_p2, a->g_e2, hx, hy, hz, 32, true));
-  UN_CUDA(launch_relu_bwd(st, a->g_e2, a->e2, V2 * 32));
+  UN_CUDA(launch_pool2_bwd(st, a->g_p2, a->g_e2, a->e2, hx, hy, hz, 32));
   UN_TRY(conv_bwd(net, st, a, 3, a->e2a, a->g_e2, a->g_e2a, hx, hy, hz));
   UN_CUDA(launch_relu_bwd(st, a->g_e2a, a->e2a, V2 * 32));
   UN_TRY(conv_bwd(net, st, a, 2, a->p1, a->g_e2a, a->g_p1, hx, hy, hz));
-  UN_CUDA(launch_pool2_bwd(st, a->g_p1, a->g_e1, sx, sy, sz, 16, true));
-  UN_CUDA(launch_relu_bwd(st, a->g_e1, a->e1, V * 16));
+  UN_CUDA(launch_pool2_bwd(st, a->g_p1, a->g_e1, a->e1, sx, sy, sz, 16));
   UN_TRY(conv_bwd(net, st, a, 1, a->e1a, a->g_e1, a->g_e1a, sx, sy, sz));
   UN_CUDA(launch_relu_bwd(st, a->g_e1a, a->e1a, V * 16));
   UN_TRY(conv_bwd(net, st, a, 0, a->in0, a->g_e1a, nullptr, sx, sy, sz));
@@ -213,15 +208,23 @@ aq_status backward(aq_unet* net, cudaStream_t st, UActs* a, const float* target,
 }
 
 aq_status adam_step(aq_unet* net, cudaStream_t st, float lr) {
-  const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
   const int t = ++net->adam_t;
+  AdamTensors T;
+  T.count = 0;
+  T.first[0] = 0;
+  auto add = [&](const AdamTensor& x, int n) {
+    T.t[T.count] = x;
+    T.first[T.count + 1] = T.first[T.count] + n;
+    ++T.count;
+  };
+  static_assert(2 * 10 + 1 <= AdamTensors::kMax, "every tensor of the network");
   for (UConv& c : net->L) {
-    UN_CUDA(launch_adam(st, c.w, c.g, c.m, c.v, c.nw(), lr, b1, b2, eps, t, c.wb));
-    UN_CUDA(launch_adam(st, c.b, c.gb, c.mb, c.vb, c.cout, lr, b1, b2, eps, t, nullptr));
-    UN_CUDA(launch_flip_transpose(st, c.wb, c.wt, c.cin, c.cout));
+    add({c.w, c.g, c.m, c.v, c.wb, c.wt, c.cin, c.cout}, c.nw());
+    add({c.b, c.gb, c.mb, c.vb, nullptr, nullptr, 0, 0}, c.cout);
   }
   // head: hg holds [dw 16, db, loss]; the first 17 are the gradient
-  UN_CUDA(launch_adam(st, net->hp, net->hg, net->hm, net->hv, 17, lr, b1, b2, eps, t, nullptr));
+  add({net->hp, net->hg, net->hm, net->hv, nullptr, nullptr, 0, 0}, 17);
+  UN_CUDA(launch_adam(st, T, lr, 0.9f, 0.999f, 1e-8f, t));
   return AQ_OK;
 }
 
