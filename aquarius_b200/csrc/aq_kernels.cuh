@@ -37,6 +37,8 @@ struct SphParams {
   int gx, gy, gz;           // hash grid
   float s_corr_den, s_corr_k, leave;  // PBF: cubic_spline_kernel(0), 1e-6, wall leave speed
   float skip_r2;            // pairs with r^2 above it are outside both kernels' support
+  // the kernels' constant divisors and their correctly rounded reciprocals
+  float poly6_den, poly6_rcp, spikey_den, spikey_rcp, s_corr_rcp;
 };
 constexpr int kSphArrays = 6;
 struct SphArrays {
@@ -47,17 +49,22 @@ cudaError_t launch_sph_keys(cudaStream_t st, const SphParams& p, const float4* p
 cudaError_t launch_sph_gather(cudaStream_t st, const int* key, const int* off, const int* perm_u, const SphArrays& src,
                               const SphArrays& dst, int n);
 cudaError_t launch_pbf_predict(cudaStream_t st, const SphParams& p, float4* P, const float4* L, float4* V, int n);
+// Neighbour lists a density pass keeps for the pass after it: count[i]
+// neighbours of particle i, the first kSphList of them at lists[i * kSphList].
+// Null: nothing is kept, and the second pass searches again.
+constexpr int kSphList = 64;
 cudaError_t launch_pbf_lambda(cudaStream_t st, const SphParams& p, const int* off, float4* P, float4* V, float4* Q,
-                              bool set_rest, int n);
-cudaError_t launch_pbf_delta(cudaStream_t st, const SphParams& p, const int* off, const float4* Q, float4* P, int n);
+                              int* count, int* lists, bool set_rest, int n);
+cudaError_t launch_pbf_delta(cudaStream_t st, const SphParams& p, const int* off, const float4* Q, float4* P,
+                             const int* count, const int* lists, int n);
 cudaError_t launch_pbf_update(cudaStream_t st, const SphParams& p, const float4* P, float4* L, float4* V, int n);
 cudaError_t launch_pci_init(cudaStream_t st, float4* W, float4* F, int n);
 cudaError_t launch_pci_predict(cudaStream_t st, const SphParams& p, float4* P, float4* V, float4* Q, float4* W,
                                const float4* F, bool actual, int n);
 cudaError_t launch_pci_density(cudaStream_t st, const SphParams& p, const int* off, float4* P, float4* V,
-                               const float4* Q, float4* W, float4* R, bool set_rest, int n);
+                               const float4* Q, float4* W, float4* R, int* count, int* lists, bool set_rest, int n);
 cudaError_t launch_pci_force(cudaStream_t st, const SphParams& p, const int* off, const float4* P, const float4* R,
-                             float4* F, int n);
+                             float4* F, const int* count, const int* lists, int n);
 
 // Surface mesher (k_mesh.cu).  SDF grid SX*SY*SZ (cell hs), its hash grid
 // HX*HY*HZ = (SX-2)*(SY-2)*(SZ-2), marching-cubes grid MX*MY*MZ (cell hm).

@@ -24,9 +24,6 @@
 namespace aqb {
 namespace {
 
-constexpr float kPi = 3.14159265358979323846f;  // PI (Fluid/WeightKernels.cuh:8)
-constexpr float k64Pi = 64.f * kPi;
-
 inline int blocks(int n, int t) { return (n + t - 1) / t; }
 
 __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
@@ -44,25 +41,58 @@ __device__ __forceinline__ float dot3(float x, float y, float z) { return add(ad
 // 85% of the 27-cell candidates are such pairs.
 __device__ __forceinline__ bool outside(float r2, const SphParams& p) { return r2 > p.skip_r2; }
 
+// Division by a divisor used many times (a constant of the kernels, a
+// distance, a rest density): with y the correctly rounded reciprocal of b, two
+// residual corrections of a * y round as the IEEE division does (Markstein's
+// theorem: the first makes the quotient faithful, the second correct), where
+// nothing over- or underflows: |a| and |b| within 2^-60 .. 2^60, or a = 0.
+// Five FMAs and a check shared by up to three quotients, against a dozen
+// instructions and a branch each.
+struct Divisor {
+  float b, y;
+  bool ok;
+};
+__device__ __forceinline__ Divisor divisor(float b, float y) {
+  return {b, y, fabsf(b) >= 0x1p-60f && fabsf(b) <= 0x1p60f};
+}
+__device__ __forceinline__ float dvd_fast(float a, const Divisor& d) {
+  const float q0 = __fmul_rn(a, d.y);
+  const float q1 = __fmaf_rn(__fmaf_rn(-q0, d.b, a), d.y, q0);
+  return __fmaf_rn(__fmaf_rn(-q1, d.b, a), d.y, q1);
+}
+// 2 bits - 1 orders magnitudes, with 0 above all of them
+__device__ __forceinline__ unsigned mag_key(float a) { return 2u * __float_as_uint(a) - 1u; }
+constexpr unsigned kLeastKey = 0x42ffffffu;  // of 2^-60
+__device__ __forceinline__ float dvd(float a, const Divisor& d) {
+  return d.ok && mag_key(a) >= kLeastKey && fabsf(a) <= 0x1p60f ? dvd_fast(a, d) : dvd(a, d.b);
+}
+__device__ __forceinline__ float3 dvd(const float3& a, const Divisor& d) {
+  const unsigned least = min(min(mag_key(a.x), mag_key(a.y)), mag_key(a.z));
+  const float most = fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fabsf(a.z));
+  if (d.ok && least >= kLeastKey && most <= 0x1p60f)
+    return make_float3(dvd_fast(a.x, d), dvd_fast(a.y, d), dvd_fast(a.z, d));
+  return make_float3(dvd(a.x, d.b), dvd(a.y, d.b), dvd(a.z, d.b));
+}
+
 // poly6 (Fluid/WeightKernels.cuh:13-26)
-__device__ __forceinline__ float poly6(float vx, float vy, float vz, const SphParams& p) {
-  const float r2 = dot3(vx, vy, vz);
+__device__ __forceinline__ float poly6(float r2, const SphParams& p) {
   if (r2 <= p.kr2) {
     const float t = sub(p.kr2, r2);
-    return dvd(mul(mul(mul(t, t), t), 315.f), mul(k64Pi, p.kr9));
+    return dvd(mul(mul(mul(t, t), t), 315.f), divisor(p.poly6_den, p.poly6_rcp));
   }
   return 0.f;
 }
 
-// spikey_grad (Fluid/WeightKernels.cuh:43-58)
-__device__ __forceinline__ float3 spikey(float vx, float vy, float vz, const SphParams& p) {
-  const float r = __fsqrt_rn(dot3(vx, vy, vz));
-  float ux = vx, uy = vy, uz = vz;
-  if (r != 0.f) { ux = dvd(ux, r); uy = dvd(uy, r); uz = dvd(uz, r); }
+// spikey_grad (Fluid/WeightKernels.cuh:43-58); r2 = v . v
+__device__ __forceinline__ float3 spikey(float vx, float vy, float vz, float r2, const SphParams& p) {
+  const float r = __fsqrt_rn(r2);
+  float3 u = make_float3(vx, vy, vz);
+  if (r != 0.f) u = dvd(u, divisor(r, __frcp_rn(r)));
   if (0.f <= r && r <= p.kr) {
-    const float hr = sub(p.kr, r), d = mul(kPi, p.kr6);
-    return make_float3(dvd(mul(mul(mul(-ux, hr), hr), 45.f), d), dvd(mul(mul(mul(-uy, hr), hr), 45.f), d),
-                       dvd(mul(mul(mul(-uz, hr), hr), 45.f), d));
+    const float hr = sub(p.kr, r);
+    return dvd(make_float3(mul(mul(mul(-u.x, hr), hr), 45.f), mul(mul(mul(-u.y, hr), hr), 45.f),
+                           mul(mul(mul(-u.z, hr), hr), 45.f)),
+               divisor(p.spikey_den, p.spikey_rcp));
   }
   return make_float3(0.f, 0.f, 0.f);
 }
@@ -71,51 +101,125 @@ __device__ __forceinline__ int3 cell_of(const SphParams& p, float x, float y, fl
   return make_int3((int)dvd(x, p.kr), (int)dvd(y, p.kr), (int)dvd(z, p.kr));
 }
 
-// The 27 cells around c, dx, dy, dz from -1 to 1, outside ones skipped
-// (Fluid/Fluid_3D_PBF.cu:37-58); body(j) for every particle j in them.
-template <typename Body>
-__device__ __forceinline__ void for_neighbours(const SphParams& p, int3 c, const int* __restrict__ off, Body&& body) {
-  for (int dx = -1; dx <= 1; ++dx) {
-    const int x = c.x + dx;
-    if (x < 0 || x >= p.gx) continue;
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int y = c.y + dy;
-      if (y < 0 || y >= p.gy) continue;
-      const int row = (x * p.gy + y) * p.gz;
-      for (int dz = -1; dz <= 1; ++dz) {
-        const int z = c.z + dz;
-        if (z < 0 || z >= p.gz) continue;
-        const int j1 = __ldg(off + row + z + 1);
-        for (int j = __ldg(off + row + z); j < j1; ++j) body(j);
-      }
-    }
+// The neighbour walk: the 27 cells around c, dx, dy, dz from -1 to 1, outside
+// ones skipped (Fluid/Fluid_3D_PBF.cu:37-58), particles in sorted order.  The
+// up to three cells of a (dx, dy) are consecutive in the cell order, so their
+// particles are one run.
+//
+// Four lanes work on a particle.  They scan four candidates of a run at a time
+// and append the inside ones (about 15%) to the particle's list in order (a
+// ballot), then evaluate four of its terms at a time, and lane k adds component
+// k (and k + 4) of the terms in list order: the reference's sums, term for
+// term.  Evaluated in the scan, one thread a particle, the costly terms ran
+// with 13.9 of 32 lanes on the average; one thread a particle with lists of
+// its own leaves the machine short of warps at the reference's default of
+// 60k particles (PBF step 1290 us against 826 us).
+//
+// The density pass keeps the lists for the pass that follows it on the same
+// positions (PBF's delta, PCISPH's force), which then scans nothing.
+constexpr int kThreads = 128, kPart = kThreads / 4;  // particles per CTA
+constexpr int kList = 64;                            // listed at a time
+template <int NC>
+struct WalkShared {
+  int list[kPart][kList];
+  float4 term[kPart][NC];
+};
+
+// Adds the terms of up to four list entries: this lane's is t (zeros past the
+// end, which change no sum).
+template <int NC>
+__device__ __forceinline__ void add_terms(WalkShared<NC>& sm, const float (&t)[NC], float (&sum)[2]) {
+  const int l = threadIdx.x & 3, g = threadIdx.x >> 2;
+#pragma unroll
+  for (int k = 0; k < NC; ++k) reinterpret_cast<float*>(&sm.term[g][k])[l] = t[k];
+  __syncwarp();
+  if (l < NC) {
+    const float4 v = sm.term[g][l];
+    sum[0] = add(add(add(add(sum[0], v.x), v.y), v.z), v.w);
   }
+  if (l + 4 < NC) {
+    const float4 v = sm.term[g][l + 4];
+    sum[1] = add(add(add(add(sum[1], v.x), v.y), v.z), v.w);
+  }
+  __syncwarp();
 }
 
-// The neighbour walk in two phases, still in the reference's order: a cheap
-// scan keeps the candidates inside the support (their indices, in shared
-// memory, kBuf per thread), then the costly terms are evaluated from that
-// list.  Inside candidates are about 15% of the scan and fall on different
-// lanes; evaluated in the scan the warp would run the costly arithmetic with
-// a few lanes at a time, from the lists all lanes run it together.  Used by
-// the two PBF passes, whose terms cost most (measured: 1.5x); PCISPH's were
-// faster evaluated in the scan.
-constexpr int kBuf = 48;  // 48 x 256 threads x 4 B = the 48 KB of static shared memory
-
-template <typename Inside, typename Eval>
-__device__ __forceinline__ void walk_inside(const SphParams& p, int3 c, const int* __restrict__ off, int* buf,
-                                            Inside&& inside, Eval&& eval) {
-  const int stride = blockDim.x, tid = threadIdx.x;
-  int cnt = 0;
-  for_neighbours(p, c, off, [&](int j) {
-    if (!inside(j)) return;
-    buf[cnt * stride + tid] = j;
-    if (++cnt == kBuf) {
-      for (int q = 0; q < kBuf; ++q) eval(buf[q * stride + tid]);
-      cnt = 0;
+// All lanes of the warp call this together; lanes of a missing particle
+// (!valid) walk nothing.  sum[0], sum[1]: components k and k + 4 in lane k.
+// keep (may be null): where the particle's first kSphList neighbours go;
+// returns how many there are.
+template <int NC, typename Inside, typename Term>
+__device__ __forceinline__ int walk(const SphParams& p, int3 c, bool valid, const int* __restrict__ off,
+                                    int* __restrict__ keep, WalkShared<NC>& sm, float (&sum)[2], Inside&& inside,
+                                    Term&& term) {
+  const int l = threadIdx.x & 3, g = threadIdx.x >> 2, shift = threadIdx.x & 28;
+  int cnt = 0, total = 0;
+  sum[0] = sum[1] = 0.f;
+  auto flush = [&]() {
+    __syncwarp();
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    for (int b = 0; b < most; b += 4) {
+      float t[NC];
+#pragma unroll
+      for (int k = 0; k < NC; ++k) t[k] = 0.f;
+      if (b + l < cnt) {
+        const int j = sm.list[g][b + l];
+        if (keep && total + b + l < kSphList) keep[total + b + l] = j;
+        term(j, t);
+      }
+      add_terms<NC>(sm, t, sum);
     }
-  });
-  for (int q = 0; q < cnt; ++q) eval(buf[q * stride + tid]);
+    total += cnt;
+    cnt = 0;
+  };
+  const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, p.gz - 1) + 1;
+  for (int dx = -1; dx <= 1; ++dx)
+    for (int dy = -1; dy <= 1; ++dy) {
+      const int x = c.x + dx, y = c.y + dy;
+      int j = 0, j1 = 0;
+      if (valid && z1 > z0 && x >= 0 && x < p.gx && y >= 0 && y < p.gy) {
+        const int row = (x * p.gy + y) * p.gz;
+        j = __ldg(off + row + z0) + l;
+        j1 = __ldg(off + row + z1);
+      }
+      while (__any_sync(0xffffffffu, j < j1)) {
+        const bool in = j < j1 && inside(j);
+        const unsigned m = (__ballot_sync(0xffffffffu, in) >> shift) & 15u;
+        if (in) sm.list[g][cnt + __popc(m & ((1u << l) - 1u))] = j;
+        cnt += __popc(m);
+        j += 4;
+        if (__any_sync(0xffffffffu, cnt > kList - 4)) flush();
+      }
+    }
+  flush();
+  return total;
+}
+
+// The same sums from the lists a walk on the same positions kept; a warp with
+// a particle of more than kSphList neighbours (or without lists) walks.
+template <int NC, typename Inside, typename Term>
+__device__ __forceinline__ void walk_kept(const SphParams& p, int3 c, int i, bool valid, const int* __restrict__ off,
+                                          const int* __restrict__ count, const int* __restrict__ lists,
+                                          WalkShared<NC>& sm, float (&sum)[2], Inside&& inside, Term&& term) {
+  const int cnt = valid && count ? __ldg(count + i) : 0;
+  const int most = __reduce_max_sync(0xffffffffu, cnt);
+  if (!count || most > kSphList) {
+    walk<NC>(p, c, valid, off, nullptr, sm, sum, inside, term);
+    return;
+  }
+  const int l = threadIdx.x & 3;
+  const int* __restrict__ row = lists + (size_t)i * kSphList;
+  sum[0] = sum[1] = 0.f;
+  int j = l < cnt ? __ldg(row + l) : 0;
+  for (int b = 0; b < most; b += 4) {
+    const int next = b + 4 + l < cnt ? __ldg(row + b + 4 + l) : 0;
+    float t[NC];
+#pragma unroll
+    for (int k = 0; k < NC; ++k) t[k] = 0.f;
+    if (b + l < cnt) term(j, t);
+    add_terms<NC>(sm, t, sum);
+    j = next;
+  }
 }
 
 // --------------------------------------------------------------- sorting
@@ -185,30 +289,37 @@ __global__ void __launch_bounds__(256) k_pbf_predict(SphParams p, float4* __rest
 
 // computeDensityAndLambdaImpl (Fluid_3D_PBF.cu:28-110): reads P, writes
 // Q = (position, lambda), the density into V.w and, on the rest-density
-// pass, P.w.
-__global__ void __launch_bounds__(256) k_pbf_lambda(SphParams p, const int* __restrict__ off, float4* __restrict__ P,
-                                                   float4* __restrict__ V, float4* __restrict__ Q, int set_rest, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  __shared__ int buf[kBuf * 256];
-  const float4 me = P[i];
-  float gx = 0.f, gy = 0.f, gz = 0.f, sdot = 0.f, density = 0.f;
-  walk_inside(
-      p, cell_of(p, me.x, me.y, me.z), off, buf,
+// pass, P.w.  A term: poly6, spikey_grad and its square.
+__device__ __forceinline__ void lambda_term(const SphParams& p, const float4& me, const float4& o, float (&t)[5]) {
+  const float dx = sub(me.x, o.x), dy = sub(me.y, o.y), dz = sub(me.z, o.z);
+  const float r2 = dot3(dx, dy, dz);
+  const float3 w = spikey(dx, dy, dz, r2, p);
+  t[0] = w.x;
+  t[1] = w.y;
+  t[2] = w.z;
+  t[3] = poly6(r2, p);
+  t[4] = dot3(w.x, w.y, w.z);
+}
+__global__ void __launch_bounds__(kThreads) k_pbf_lambda(SphParams p, const int* __restrict__ off,
+                                                        float4* __restrict__ P, float4* __restrict__ V,
+                                                        float4* __restrict__ Q, int* __restrict__ count,
+                                                        int* __restrict__ lists, int set_rest, int n) {
+  __shared__ WalkShared<5> sm;
+  const int i = (blockIdx.x * kThreads + threadIdx.x) >> 2;
+  const float4 me = i < n ? P[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  float s[2];
+  const int found = walk<5>(
+      p, cell_of(p, me.x, me.y, me.z), i < n, off, lists ? lists + (size_t)i * kSphList : nullptr, sm, s,
       [&](int j) {
-        const float4 o = __ldg(P + j);
+        const float4 o = P[j];
         return !outside(dot3(sub(me.x, o.x), sub(me.y, o.y), sub(me.z, o.z)), p);
       },
-      [&](int j) {
-        const float4 o = __ldg(P + j);
-        const float dx = sub(me.x, o.x), dy = sub(me.y, o.y), dz = sub(me.z, o.z);
-        density = add(density, poly6(dx, dy, dz, p));
-        const float3 w = spikey(dx, dy, dz, p);
-        gx = add(gx, w.x);
-        gy = add(gy, w.y);
-        gz = add(gz, w.z);
-        sdot = add(sdot, dot3(w.x, w.y, w.z));
-      });
+      [&](int j, float (&t)[5]) { lambda_term(p, me, P[j], t); });
+  const int first = threadIdx.x & 28;
+  const float gx = s[0], gy = __shfl_sync(0xffffffffu, s[0], first + 1), gz = __shfl_sync(0xffffffffu, s[0], first + 2);
+  const float density = __shfl_sync(0xffffffffu, s[0], first + 3), sdot = s[1];
+  if ((threadIdx.x & 3) || i >= n) return;
+  if (count) count[i] = found;
   const float rho0 = set_rest ? density : me.w;
   const float ci = sub(dvd(density, rho0), 1.f);
   const float q = dvd(add(sdot, dot3(gx, gy, gz)), mul(rho0, rho0));
@@ -222,35 +333,42 @@ __global__ void __launch_bounds__(256) k_pbf_lambda(SphParams p, const int* __re
 
 // computeDeltaPositionImpl + applyDeltaPositionImpl (Fluid_3D_PBF.cu:114-206):
 // reads Q, writes the moved position into P (its w, the rest density, kept).
-__global__ void __launch_bounds__(256) k_pbf_delta(SphParams p, const int* __restrict__ off,
-                                                  const float4* __restrict__ Q, float4* __restrict__ P, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  __shared__ int buf[kBuf * 256];
-  const float4 me = Q[i];
-  const float rho0 = P[i].w;
-  float ax = 0.f, ay = 0.f, az = 0.f;
-  walk_inside(
-      p, cell_of(p, me.x, me.y, me.z), off, buf,
+__global__ void __launch_bounds__(kThreads) k_pbf_delta(SphParams p, const int* __restrict__ off,
+                                                       const float4* __restrict__ Q, float4* __restrict__ P,
+                                                       const int* __restrict__ count, const int* __restrict__ lists,
+                                                       int n) {
+  __shared__ WalkShared<3> sm;
+  const int i = (blockIdx.x * kThreads + threadIdx.x) >> 2;
+  const float4 me = i < n ? Q[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float rho0 = i < n ? P[i].w : 1.f;
+  const Divisor by_rho0 = divisor(rho0, __frcp_rn(rho0)), by_corr = divisor(p.s_corr_den, p.s_corr_rcp);
+  float s[2];
+  walk_kept<3>(
+      p, cell_of(p, me.x, me.y, me.z), i, i < n, off, count, lists, sm, s,
       [&](int j) {
         const float4 o = __ldg(Q + j);
         return !outside(dot3(sub(me.x, o.x), sub(me.y, o.y), sub(me.z, o.z)), p);
       },
-      [&](int j) {
+      [&](int j, float (&t)[3]) {
         const float4 o = __ldg(Q + j);
         const float dx = sub(me.x, o.x), dy = sub(me.y, o.y), dz = sub(me.z, o.z);
-        const float3 w = spikey(dx, dy, dz, p);
-        const float t = dvd(poly6(dx, dy, dz, p), p.s_corr_den);
-        const float t2 = mul(t, t);
-        const float sc = mul(mul(t2, t2), -p.s_corr_k);
+        const float r2 = dot3(dx, dy, dz);
+        const float3 w = spikey(dx, dy, dz, r2, p);
+        const float c = dvd(poly6(r2, p), by_corr);
+        const float c2 = mul(c, c);
+        const float sc = mul(mul(c2, c2), -p.s_corr_k);
         const float f = add(add(me.w, o.w), sc);
-        ax = add(ax, dvd(mul(w.x, f), rho0));
-        ay = add(ay, dvd(mul(w.y, f), rho0));
-        az = add(az, dvd(mul(w.z, f), rho0));
+        const float3 q = dvd(make_float3(mul(w.x, f), mul(w.y, f), mul(w.z, f)), by_rho0);
+        t[0] = q.x;
+        t[1] = q.y;
+        t[2] = q.z;
       });
+  const int first = threadIdx.x & 28;
+  const float ay = __shfl_sync(0xffffffffu, s[0], first + 1), az = __shfl_sync(0xffffffffu, s[0], first + 2);
+  if ((threadIdx.x & 3) || i >= n) return;
   const float hi = sub(p.size, p.md);
-  P[i] = make_float4(clampw(add(me.x, ax), p.md, hi), clampw(add(me.y, ay), p.md, hi), clampw(add(me.z, az), p.md, hi),
-                     rho0);
+  P[i] = make_float4(clampw(add(me.x, s[0]), p.md, hi), clampw(add(me.y, ay), p.md, hi),
+                     clampw(add(me.z, az), p.md, hi), rho0);
 }
 
 // updatePositionAndVelocityImpl (Fluid_3D_PBF.cu:209-267)
@@ -312,21 +430,29 @@ __global__ void __launch_bounds__(256) k_pci_predict(SphParams p, float4* __rest
 // - rest density), the coefficient the kernel ends with.  Writes the density
 // into V.w, the pressure into W.w, R = (predicted position, p / rho^2) and, on
 // the rest-density pass, P.w.
-__global__ void __launch_bounds__(256) k_pci_density(SphParams p, const int* __restrict__ off, float4* __restrict__ P,
-                                                    float4* __restrict__ V, const float4* __restrict__ Q,
-                                                    float4* __restrict__ W, float4* __restrict__ R, int set_rest,
-                                                    int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 me = P[i];
-  const float4 pq = Q[i];
-  float density = 0.f;
-  for_neighbours(p, cell_of(p, me.x, me.y, me.z), off, [&](int j) {
-    const float4 o = __ldg(Q + j);
-    const float dx = sub(pq.x, o.x), dy = sub(pq.y, o.y), dz = sub(pq.z, o.z);
-    if (outside(dot3(dx, dy, dz), p)) return;
-    density = add(density, poly6(dx, dy, dz, p));
-  });
+__global__ void __launch_bounds__(kThreads) k_pci_density(SphParams p, const int* __restrict__ off,
+                                                         float4* __restrict__ P, float4* __restrict__ V,
+                                                         const float4* __restrict__ Q, float4* __restrict__ W,
+                                                         float4* __restrict__ R, int* __restrict__ count,
+                                                         int* __restrict__ lists, int set_rest, int n) {
+  __shared__ WalkShared<1> sm;
+  const int i = (blockIdx.x * kThreads + threadIdx.x) >> 2;
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 me = i < n ? P[i] : none, pq = i < n ? Q[i] : none;
+  float s[2];
+  const int found = walk<1>(
+      p, cell_of(p, me.x, me.y, me.z), i < n, off, lists ? lists + (size_t)i * kSphList : nullptr, sm, s,
+      [&](int j) {
+        const float4 o = __ldg(Q + j);
+        return !outside(dot3(sub(pq.x, o.x), sub(pq.y, o.y), sub(pq.z, o.z)), p);
+      },
+      [&](int j, float (&t)[1]) {
+        const float4 o = __ldg(Q + j);
+        t[0] = poly6(dot3(sub(pq.x, o.x), sub(pq.y, o.y), sub(pq.z, o.z)), p);
+      });
+  if ((threadIdx.x & 3) || i >= n) return;
+  if (count) count[i] = found;
+  const float density = s[0];
   const float err = sub(density, me.w);
   const float pressure = add(W[i].w, mul(50.0f, err));
   V[i].w = density;
@@ -335,26 +461,36 @@ __global__ void __launch_bounds__(256) k_pci_density(SphParams p, const int* __r
   R[i] = make_float4(pq.x, pq.y, pq.z, dvd(pressure, mul(density, density)));
 }
 
-// computePressureForceImpl (Fluid_3D_PCISPH.cu:161-202)
-__global__ void __launch_bounds__(256) k_pci_force(SphParams p, const int* __restrict__ off,
-                                                  const float4* __restrict__ P, const float4* __restrict__ R,
-                                                  float4* __restrict__ F, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float4 me = P[i];
-  const float4 r = R[i];
-  float fx = 0.f, fy = 0.f, fz = 0.f;
-  for_neighbours(p, cell_of(p, me.x, me.y, me.z), off, [&](int j) {
-    const float4 o = __ldg(R + j);
-    const float dx = sub(r.x, o.x), dy = sub(r.y, o.y), dz = sub(r.z, o.z);
-    if (outside(dot3(dx, dy, dz), p)) return;
-    const float3 w = spikey(dx, dy, dz, p);
-    const float s = add(o.w, r.w);
-    fx = sub(fx, mul(w.x, s));
-    fy = sub(fy, mul(w.y, s));
-    fz = sub(fz, mul(w.z, s));
-  });
-  F[i] = make_float4(fx, fy, fz, 0.f);
+// computePressureForceImpl (Fluid_3D_PCISPH.cu:161-202); the reference
+// subtracts each term, and adding its negative rounds the same.
+__global__ void __launch_bounds__(kThreads) k_pci_force(SphParams p, const int* __restrict__ off,
+                                                       const float4* __restrict__ P, const float4* __restrict__ R,
+                                                       float4* __restrict__ F, const int* __restrict__ count,
+                                                       const int* __restrict__ lists, int n) {
+  __shared__ WalkShared<3> sm;
+  const int i = (blockIdx.x * kThreads + threadIdx.x) >> 2;
+  const float4 none = make_float4(0.f, 0.f, 0.f, 0.f);
+  const float4 me = i < n ? P[i] : none, r = i < n ? R[i] : none;
+  float s[2];
+  walk_kept<3>(
+      p, cell_of(p, me.x, me.y, me.z), i, i < n, off, count, lists, sm, s,
+      [&](int j) {
+        const float4 o = __ldg(R + j);
+        return !outside(dot3(sub(r.x, o.x), sub(r.y, o.y), sub(r.z, o.z)), p);
+      },
+      [&](int j, float (&t)[3]) {
+        const float4 o = __ldg(R + j);
+        const float dx = sub(r.x, o.x), dy = sub(r.y, o.y), dz = sub(r.z, o.z);
+        const float3 w = spikey(dx, dy, dz, dot3(dx, dy, dz), p);
+        const float q = add(o.w, r.w);
+        t[0] = -mul(w.x, q);
+        t[1] = -mul(w.y, q);
+        t[2] = -mul(w.z, q);
+      });
+  const int first = threadIdx.x & 28;
+  const float fy = __shfl_sync(0xffffffffu, s[0], first + 1), fz = __shfl_sync(0xffffffffu, s[0], first + 2);
+  if ((threadIdx.x & 3) || i >= n) return;
+  F[i] = make_float4(s[0], fy, fz, 0.f);
 }
 
 // initPressureImpl (Fluid_3D_PCISPH.cu:22-30): pressure and pressure force 0.
@@ -388,15 +524,16 @@ cudaError_t launch_pbf_predict(cudaStream_t st, const SphParams& p, float4* P, c
 }
 
 cudaError_t launch_pbf_lambda(cudaStream_t st, const SphParams& p, const int* off, float4* P, float4* V, float4* Q,
-                              bool set_rest, int n) {
+                              int* count, int* lists, bool set_rest, int n) {
   if (n <= 0) return cudaSuccess;
-  k_pbf_lambda<<<blocks(n, 256), 256, 0, st>>>(p, off, P, V, Q, set_rest ? 1 : 0, n);
+  k_pbf_lambda<<<blocks(n, kPart), kThreads, 0, st>>>(p, off, P, V, Q, count, lists, set_rest ? 1 : 0, n);
   return cudaGetLastError();
 }
 
-cudaError_t launch_pbf_delta(cudaStream_t st, const SphParams& p, const int* off, const float4* Q, float4* P, int n) {
+cudaError_t launch_pbf_delta(cudaStream_t st, const SphParams& p, const int* off, const float4* Q, float4* P,
+                             const int* count, const int* lists, int n) {
   if (n <= 0) return cudaSuccess;
-  k_pbf_delta<<<blocks(n, 256), 256, 0, st>>>(p, off, Q, P, n);
+  k_pbf_delta<<<blocks(n, kPart), kThreads, 0, st>>>(p, off, Q, P, count, lists, n);
   return cudaGetLastError();
 }
 
@@ -420,16 +557,16 @@ cudaError_t launch_pci_predict(cudaStream_t st, const SphParams& p, float4* P, f
 }
 
 cudaError_t launch_pci_density(cudaStream_t st, const SphParams& p, const int* off, float4* P, float4* V,
-                               const float4* Q, float4* W, float4* R, bool set_rest, int n) {
+                               const float4* Q, float4* W, float4* R, int* count, int* lists, bool set_rest, int n) {
   if (n <= 0) return cudaSuccess;
-  k_pci_density<<<blocks(n, 256), 256, 0, st>>>(p, off, P, V, Q, W, R, set_rest ? 1 : 0, n);
+  k_pci_density<<<blocks(n, kPart), kThreads, 0, st>>>(p, off, P, V, Q, W, R, count, lists, set_rest ? 1 : 0, n);
   return cudaGetLastError();
 }
 
 cudaError_t launch_pci_force(cudaStream_t st, const SphParams& p, const int* off, const float4* P, const float4* R,
-                             float4* F, int n) {
+                             float4* F, const int* count, const int* lists, int n) {
   if (n <= 0) return cudaSuccess;
-  k_pci_force<<<blocks(n, 256), 256, 0, st>>>(p, off, P, R, F, n);
+  k_pci_force<<<blocks(n, kPart), kThreads, 0, st>>>(p, off, P, R, F, count, lists, n);
   return cudaGetLastError();
 }
 

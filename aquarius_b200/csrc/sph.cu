@@ -33,6 +33,7 @@ using namespace aqb;
 
 namespace {
 
+constexpr int kListedParticles = 1 << 26;  // neighbour lists up to this many particles (17 GB)
 constexpr float kSize = 10.f;  // gridPhysicalSize (Fluid_3D_PBF.cuh:63, Fluid_3D_PCISPH.cuh:59)
 constexpr float kPiHost = 3.14159265358979323846f;
 
@@ -109,6 +110,9 @@ struct aq_sph {
   }
 
   // Fluid::simulationStep (Fluid_3D_PBF.cu:489-517, Fluid_3D_PCISPH.cu:424-448)
+  // neighbour lists of the density pass (null: not kept)
+  int *near_count = nullptr, *near_list = nullptr;
+
   aq_status enq_step() {
     if (method == AQ_SPH_PBF) {
       AQS_TRY(enq_sort());
@@ -116,8 +120,8 @@ struct aq_sph {
         AQS_CUDA(launch_pbf_predict(stream, sp, A(A_P), A(A_L), A(A_V), n));
         AQS_TRY(enq_sort());
         for (int it = 0; it < cfg.iterations; ++it) {
-          AQS_CUDA(launch_pbf_lambda(stream, sp, off, A(A_P), A(A_V), A(A_Q), false, n));
-          AQS_CUDA(launch_pbf_delta(stream, sp, off, A(A_Q), A(A_P), n));
+          AQS_CUDA(launch_pbf_lambda(stream, sp, off, A(A_P), A(A_V), A(A_Q), near_count, near_list, false, n));
+          AQS_CUDA(launch_pbf_delta(stream, sp, off, A(A_Q), A(A_P), near_count, near_list, n));
         }
         AQS_CUDA(launch_pbf_update(stream, sp, A(A_P), A(A_L), A(A_V), n));
       }
@@ -127,8 +131,9 @@ struct aq_sph {
         AQS_CUDA(launch_pci_init(stream, A(A_W), A(A_F), n));
         for (int it = 0; it < cfg.iterations; ++it) {
           AQS_CUDA(launch_pci_predict(stream, sp, A(A_P), A(A_V), A(A_Q), A(A_W), A(A_F), false, n));
-          AQS_CUDA(launch_pci_density(stream, sp, off, A(A_P), A(A_V), A(A_Q), A(A_W), A(A_R), false, n));
-          AQS_CUDA(launch_pci_force(stream, sp, off, A(A_P), A(A_R), A(A_F), n));
+          AQS_CUDA(launch_pci_density(stream, sp, off, A(A_P), A(A_V), A(A_Q), A(A_W), A(A_R), near_count,
+                                      near_list, false, n));
+          AQS_CUDA(launch_pci_force(stream, sp, off, A(A_P), A(A_R), A(A_F), near_count, near_list, n));
         }
         AQS_CUDA(launch_pci_predict(stream, sp, A(A_P), A(A_V), A(A_Q), A(A_W), A(A_F), true, n));
       }
@@ -313,6 +318,11 @@ aq_status aq_sph_create(const aq_sph_config* cfg, aq_sph** out) {
   p.gx = p.gy = p.gz = (int)std::ceil(kSize / kr);
   p.s_corr_den = cubic_spline(0, kr, kr3);
   p.s_corr_k = 1e-6f;
+  p.poly6_den = (64.f * 3.14159265358979323846f) * p.kr9;  // Fluid/WeightKernels.cuh:13-58
+  p.spikey_den = 3.14159265358979323846f * p.kr6;
+  p.poly6_rcp = 1.f / p.poly6_den;
+  p.spikey_rcp = 1.f / p.spikey_den;
+  p.s_corr_rcp = 1.f / p.s_corr_den;
   p.leave = (float)((double)p.md / ((double)p.dt * 1e2));
   {
     // the largest r^2 whose IEEE square root is still <= kernelRadius
@@ -338,6 +348,11 @@ aq_status aq_sph_create(const aq_sph_config* cfg, aq_sph** out) {
   if (st == AQ_OK) st = s->alloc(&s->count, (size_t)s->cells + 1);
   if (st == AQ_OK) st = s->alloc(&s->off, (size_t)s->cells + 1);
   if (st == AQ_OK) st = s->alloc(&s->tiles, cell_scan_tiles(s->cells));
+  // neighbour lists, 260 bytes a particle; without them each pass searches
+  if (st == AQ_OK && n <= kListedParticles) {
+    st = s->alloc(&s->near_count, (size_t)n);
+    if (st == AQ_OK) st = s->alloc(&s->near_list, (size_t)n * kSphList);
+  }
   if (st != AQ_OK) return bail(st);
   // Particle(float3): position = lastPosition = predictedPosition, velocity 0
   std::vector<float4> h4((size_t)n);
@@ -350,9 +365,10 @@ aq_status aq_sph_create(const aq_sph_config* cfg, aq_sph** out) {
   st = s->enq_sort();
   if (st == AQ_OK) {
     cudaError_t e = s->method == AQ_SPH_PBF
-                        ? launch_pbf_lambda(s->stream, p, s->off, s->A(A_P), s->A(A_V), s->A(A_Q), true, n)
+                        ? launch_pbf_lambda(s->stream, p, s->off, s->A(A_P), s->A(A_V), s->A(A_Q), s->near_count,
+                                            s->near_list, true, n)
                         : launch_pci_density(s->stream, p, s->off, s->A(A_P), s->A(A_V), s->A(A_Q), s->A(A_W),
-                                             s->A(A_R), true, n);
+                                             s->A(A_R), s->near_count, s->near_list, true, n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
     if (e != cudaSuccess) st = fail(AQ_ERR_CUDA, std::string("init: ") + cudaGetErrorString(e));
   }
