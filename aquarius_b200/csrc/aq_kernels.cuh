@@ -58,6 +58,8 @@ cudaError_t launch_pbf_lambda(cudaStream_t st, const SphParams& p, const int* of
 cudaError_t launch_pbf_delta(cudaStream_t st, const SphParams& p, const int* off, const float4* Q, float4* P,
                              const int* count, const int* lists, int n);
 cudaError_t launch_pbf_update(cudaStream_t st, const SphParams& p, const float4* P, float4* L, float4* V, int n);
+// planes[k * n + i] = component k of a[i]
+cudaError_t launch_sph_planes(cudaStream_t st, const float4* a, float* planes, int n);
 cudaError_t launch_pci_init(cudaStream_t st, float4* W, float4* F, int n);
 cudaError_t launch_pci_predict(cudaStream_t st, const SphParams& p, float4* P, float4* V, float4* Q, float4* W,
                                const float4* F, bool actual, int n);

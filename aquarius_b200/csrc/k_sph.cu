@@ -501,7 +501,24 @@ __global__ void __launch_bounds__(256) k_pci_init(float4* __restrict__ W, float4
   F[i] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+__global__ void __launch_bounds__(256) k_sph_planes(const float4* __restrict__ a, float* __restrict__ planes, int n) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 v = a[i];
+  const size_t m = (size_t)n;
+  planes[i] = v.x;
+  planes[m + i] = v.y;
+  planes[2 * m + i] = v.z;
+  planes[3 * m + i] = v.w;
+}
+
 }  // namespace
+
+cudaError_t launch_sph_planes(cudaStream_t st, const float4* a, float* planes, int n) {
+  if (n <= 0) return cudaSuccess;
+  k_sph_planes<<<blocks(n, 256), 256, 0, st>>>(a, planes, n);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_sph_keys(cudaStream_t st, const SphParams& p, const float4* pos, int* key, int* slot, int* count,
                             int n) {

@@ -110,6 +110,7 @@ struct aq_sph {
   }
 
   // Fluid::simulationStep (Fluid_3D_PBF.cu:489-517, Fluid_3D_PCISPH.cu:424-448)
+  float* planes = nullptr;  // one particle array as planes (made by the first download)
   // neighbour lists of the density pass (null: not kept)
   int *near_count = nullptr, *near_list = nullptr;
 
@@ -415,29 +416,26 @@ aq_status aq_sph_download_state(aq_sph* s, aq_sph_state* st) {
   AQS_CUDA(cudaStreamSynchronize(s->stream));
   const size_t n = (size_t)s->n;
   st->physical_time = s->time;
-  std::vector<float4> h(n);
-  auto get = [&](int role) -> aq_status {
-    if (n) AQS_CUDA(cudaMemcpy(h.data(), s->A(role), sizeof(float4) * n, cudaMemcpyDeviceToHost));
+  if (n && !s->planes) AQS_TRY(s->alloc(&s->planes, 4 * n));
+  // one array, split into planes on the device; only what is asked for
+  auto get = [&](int role, float* xyz, float* w) -> aq_status {
+    if (!n || (!xyz && !w)) return AQ_OK;
+    AQS_CUDA(launch_sph_planes(s->stream, s->A(role), s->planes, s->n));
+    if (xyz) AQS_CUDA(cudaMemcpyAsync(xyz, s->planes, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost, s->stream));
+    if (w) AQS_CUDA(cudaMemcpyAsync(w, s->planes + 3 * n, sizeof(float) * n, cudaMemcpyDeviceToHost, s->stream));
     return AQ_OK;
   };
-  auto xyz = [&](float* dst) {
-    if (!dst) return;
-    for (size_t i = 0; i < n; ++i) { dst[i] = h[i].x; dst[n + i] = h[i].y; dst[2 * n + i] = h[i].z; }
-  };
-  auto w = [&](float* dst) {
-    if (!dst) return;
-    for (size_t i = 0; i < n; ++i) dst[i] = h[i].w;
-  };
-  AQS_TRY(get(A_P)); xyz(st->position); w(st->rest_density);
-  AQS_TRY(get(A_V)); xyz(st->velocity); w(st->density);
+  AQS_TRY(get(A_P, st->position, st->rest_density));
+  AQS_TRY(get(A_V, st->velocity, st->density));
   if (s->method == AQ_SPH_PBF) {
-    AQS_TRY(get(A_L)); xyz(st->last_position);
-    AQS_TRY(get(A_Q)); w(st->lambda);
+    AQS_TRY(get(A_L, st->last_position, nullptr));
+    AQS_TRY(get(A_Q, nullptr, st->lambda));
   } else {
-    AQS_TRY(get(A_Q)); xyz(st->predicted_position);
-    AQS_TRY(get(A_W)); xyz(st->predicted_velocity); w(st->pressure);
-    AQS_TRY(get(A_F)); xyz(st->pressure_force);
+    AQS_TRY(get(A_Q, st->predicted_position, nullptr));
+    AQS_TRY(get(A_W, st->predicted_velocity, st->pressure));
+    AQS_TRY(get(A_F, st->pressure_force, nullptr));
   }
+  AQS_CUDA(cudaStreamSynchronize(s->stream));
   return AQ_OK;
 }
 
