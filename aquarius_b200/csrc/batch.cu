@@ -105,13 +105,21 @@ struct aq_batch {
   int* live = nullptr;
 
   cudaGraphExec_t exec = nullptr;
+  // the step in two graphs, split behind the sort (as aq_fluid's)
+  cudaGraphExec_t exec_sort = nullptr, exec_rest = nullptr;
+  cudaStream_t copy = nullptr;
+  cudaEvent_t sorted = nullptr, copied = nullptr;
   int graph_launches = 0, body_launches = 0;
   std::vector<void*> allocs;
 
   ~aq_batch() {
     cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    if (exec) cudaGraphExecDestroy(exec);
+    invalidate_graph();
+    if (copy) cudaStreamSynchronize(copy);
+    if (copy) cudaStreamDestroy(copy);
+    if (sorted) cudaEventDestroy(sorted);
+    if (copied) cudaEventDestroy(copied);
     for (cudaEvent_t e : cl_event)
       if (e) cudaEventDestroy(e);
     for (cudaStream_t q : cl_stream)
@@ -148,16 +156,18 @@ struct aq_batch {
   aq_status plan_clusters();
   aq_status enq_clusters();
   aq_status add_scene(int s, aq_fluid* f);
-  aq_status enq_pre_solve();
+  aq_status enq_sort();       // the step's particle stage
+  aq_status enq_pre_solve();  // the rest up to the solve
   aq_status enq_sweeps(int sweeps);
   aq_status enq_solve_fixed();
   aq_status enq_solve_body(unsigned long long handle);
   aq_status enq_post_solve();
+  aq_status capture_step(bool sort, bool rest, cudaGraphExec_t* out);
   aq_status build_graph();
   void invalidate_graph() {
-    if (exec) {
-      cudaGraphExecDestroy(exec);
-      exec = nullptr;
+    for (cudaGraphExec_t* e : {&exec, &exec_sort, &exec_rest}) {
+      if (*e) cudaGraphExecDestroy(*e);
+      *e = nullptr;
     }
   }
 };
@@ -310,8 +320,8 @@ aq_status aq_batch::add_scene(int s, aq_fluid* f) {
 }
 
 // ------------------------------------------------------------------ stages
-aq_status aq_batch::enq_pre_solve() {
-  const int tp = pre_p[ns], tn = pre_n[ns], tb = pre_b[ns], tsl = pre_s[ns];
+aq_status aq_batch::enq_sort() {
+  const int tp = pre_p[ns];
   if (N > 0) {
     AQB_CUDA(launch_batch_particles_advance(stream, bi, tp, grid(), true, cur, tmp, u0, v0, w0, un2, vn2, wn2, key,
                                             slot, count));
@@ -321,6 +331,11 @@ aq_status aq_batch::enq_pre_solve() {
   } else {
     AQB_CUDA(launch_cell_scan(stream, C, count, off, tile_sums));
   }
+  return AQ_OK;
+}
+
+aq_status aq_batch::enq_pre_solve() {
+  const int tn = pre_n[ns], tb = pre_b[ns], tsl = pre_s[ns];
   AQB_CUDA(launch_batch_p2g(stream, bi, tn, grid(), true, cur, off, u0, v0, w0, un1, vn1, wn1, type, density));
   AQB_CUDA(launch_batch_slayer(stream, bi, tsl, grid(), type, un2, vn2, wn2, un1, vn1, wn1, un2, vn2, wn2));
   AQB_CUDA(launch_batch_divergence(stream, bi, tb, grid512(), off, type, density, un1, vn1, wn1, pcount, div, rhs,
@@ -376,6 +391,10 @@ aq_status aq_batch::enq_post_solve() {
 
 aq_status aq_batch::build_graph() {
   invalidate_graph();
+  return capture_step(true, true, &exec);
+}
+
+aq_status aq_batch::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   AQB_CUDA(cudaGraphCreate(&g, 0));
   auto capture = [&](cudaGraph_t into, const cudaGraphNode_t* deps, size_t nd, auto&& body) -> aq_status {
@@ -391,10 +410,16 @@ aq_status aq_batch::build_graph() {
   // one launch per cluster width instead
   const int pre_launches = (N > 0 ? 6 : 3) + 5;  // sort; p2g, s-layer, divergence, b2, row list
   const int post_launches = 4;
+  auto before_solve = [&]() -> aq_status {
+    if (sort) AQB_TRY(enq_sort());
+    return rest ? enq_pre_solve() : AQ_OK;
+  };
   aq_status st;
-  if (solver.solve_mode == AQ_SOLVE_RESIDUAL && clusters) {
+  if (!rest) {
+    st = capture(g, nullptr, 0, before_solve);
+  } else if (solver.solve_mode == AQ_SOLVE_RESIDUAL && clusters) {
     st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = enq_pre_solve();
+      aq_status s2 = before_solve();
       if (s2 != AQ_OK) return s2;
       s2 = enq_clusters();
       if (s2 != AQ_OK) return s2;
@@ -403,7 +428,7 @@ aq_status aq_batch::build_graph() {
     body_launches = solver.check_interval + 3;
     graph_launches = pre_launches + post_launches;
   } else if (solver.solve_mode == AQ_SOLVE_RESIDUAL) {
-    st = capture(g, nullptr, 0, [&]() { return enq_pre_solve(); });
+    st = capture(g, nullptr, 0, before_solve);
     if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
     size_t nn = 0;
     cudaGraphGetNodes(g, nullptr, &nn);
@@ -435,7 +460,7 @@ aq_status aq_batch::build_graph() {
     graph_launches = pre_launches + post_launches;
   } else {
     st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = enq_pre_solve();
+      aq_status s2 = before_solve();
       if (s2 != AQ_OK) return s2;
       s2 = enq_solve_fixed();
       if (s2 != AQ_OK) return s2;
@@ -446,9 +471,9 @@ aq_status aq_batch::build_graph() {
     graph_launches = pre_launches + post_launches + (K > 0 ? K + 2 + (K % 2) : 0);
   }
   if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
-  cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+  cudaError_t e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
-  if (e != cudaSuccess) { exec = nullptr; return fail(AQ_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e)); }
+  if (e != cudaSuccess) { *out = nullptr; return fail(AQ_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e)); }
   return AQ_OK;
 }
 
@@ -610,13 +635,39 @@ aq_status aq_batch_step_host(aq_batch* b, int32_t n_steps, const float* pin, con
       if (vin) AQB_CUDA(cudaMemcpyAsync(dv[k], vin + k * N, 4 * N, cudaMemcpyHostToDevice, s));
     }
   }
-  AQB_TRY(aq_batch_step(b, n_steps));
-  if (N) {
-    for (int k = 0; k < 3; ++k) {
-      if (pout) AQB_CUDA(cudaMemcpyAsync(pout + k * N, dp[k], 4 * N, cudaMemcpyDeviceToHost, s));
-      if (vout) AQB_CUDA(cudaMemcpyAsync(vout + k * N, dv[k], 4 * N, cudaMemcpyDeviceToHost, s));
+  // copies out go beside the rest of the last step, as aq_fluid_step_host's
+  const size_t bytes = ((pout ? 12 : 0) + (vout ? 12 : 0)) * N;
+  const bool split = n_steps > 0 && bytes >= kSplitBytes;
+  cudaStream_t out = s;
+  if (split) {
+    if (!b->copy) {
+      AQB_CUDA(cudaStreamCreateWithFlags(&b->copy, cudaStreamNonBlocking));
+      AQB_CUDA(cudaEventCreateWithFlags(&b->sorted, cudaEventDisableTiming));
+      AQB_CUDA(cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming));
     }
+    if (n_steps > 1) AQB_TRY(aq_batch_step(b, n_steps - 1));
+    if (!b->exec_sort) AQB_TRY(b->capture_step(true, false, &b->exec_sort));
+    if (!b->exec_rest) AQB_TRY(b->capture_step(false, true, &b->exec_rest));
+    AQB_CUDA(cudaGraphLaunch(b->exec_sort, s));
+    AQB_CUDA(cudaEventRecord(b->sorted, s));
+    AQB_CUDA(cudaGraphLaunch(b->exec_rest, s));
+    for (int k = 0; k < b->ns; ++k) b->time[k] += (double)b->cfgs[k].timestep;
+    AQB_CUDA(cudaStreamWaitEvent(b->copy, b->sorted, 0));
+    out = b->copy;
+  } else {
+    AQB_TRY(aq_batch_step(b, n_steps));
   }
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 3 && N && e == cudaSuccess; ++k) {
+    if (pout) e = cudaMemcpyAsync(pout + k * N, dp[k], 4 * N, cudaMemcpyDeviceToHost, out);
+    if (vout && e == cudaSuccess) e = cudaMemcpyAsync(vout + k * N, dv[k], 4 * N, cudaMemcpyDeviceToHost, out);
+  }
+  if (split) {  // whatever follows on the batch's stream finds the copies done
+    const cudaError_t r = cudaEventRecord(b->copied, b->copy);
+    const cudaError_t w = cudaStreamWaitEvent(s, b->copied, 0);
+    if (e == cudaSuccess) e = r != cudaSuccess ? r : w;
+  }
+  AQB_CUDA(e);
   AQB_CUDA(cudaStreamSynchronize(s));
   return AQ_OK;
 }

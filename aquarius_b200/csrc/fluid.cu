@@ -614,9 +614,12 @@ aq_status aq_fluid::run_stage(int stage) {
   }
 }
 
-aq_status aq_fluid::enq_pre_solve() {
+aq_status aq_fluid::enq_sort() {
   nv_cur = 2;
-  AQ_TRY(enq_particles(true));
+  return enq_particles(true);
+}
+
+aq_status aq_fluid::enq_pre_solve() {
   AQ_TRY(enq_p2g(true));
   AQ_TRY(enq_divergence());
   if (cfg.pressure_init == AQ_PRESSURE_LEARNED) AQ_TRY(enq_learned_start());
@@ -689,8 +692,7 @@ static aq_status leaves_of(cudaGraph_t g, std::vector<cudaGraphNode_t>& out) {
 // The whole step as one CUDA graph.  RESIDUAL mode puts the sweeps in a
 // conditional WHILE node whose body ends with the residual check that sets
 // the loop condition, so a step needs no host round trip.
-aq_status aq_fluid::build_graph() {
-  invalidate_graph();
+aq_status aq_fluid::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   AQ_CUDA(cudaGraphCreate(&g, 0));
   int launches = 0;
@@ -703,11 +705,17 @@ aq_status aq_fluid::build_graph() {
     if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
     return AQ_OK;
   };
+  auto before_solve = [&]() -> aq_status {
+    if (sort) AQ_TRY(enq_sort());
+    return rest ? enq_pre_solve() : AQ_OK;
+  };
   aq_status st = AQ_OK;
   launches += (n > 0 ? 6 : 3) + 2 + 2;  // particles (+3 scan kernels), p2g, slayer, divergence, b2
-  if (cfg.solve_mode == AQ_SOLVE_RESIDUAL && whole_solve(plan)) {
+  if (!rest) {
+    st = capture(g, nullptr, 0, before_solve);
+  } else if (cfg.solve_mode == AQ_SOLVE_RESIDUAL && whole_solve(plan)) {
     st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = enq_pre_solve();
+      aq_status s2 = before_solve();
       if (s2 != AQ_OK) return s2;
       s2 = enqueue_whole(this, 0);
       if (s2 != AQ_OK) return s2;
@@ -716,7 +724,7 @@ aq_status aq_fluid::build_graph() {
     launches += count_jacobi_launches(0);
     body_launches = 0;
   } else if (cfg.solve_mode == AQ_SOLVE_RESIDUAL) {
-    st = capture(g, nullptr, 0, [&]() { return enq_pre_solve(); });
+    st = capture(g, nullptr, 0, before_solve);
     if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
     std::vector<cudaGraphNode_t> leaves;
     st = leaves_of(g, leaves);
@@ -742,7 +750,7 @@ aq_status aq_fluid::build_graph() {
     st = capture(g, &cnode, 1, [&]() { return enq_post_solve(); });
   } else {
     st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = enq_pre_solve();
+      aq_status s2 = before_solve();
       if (s2 != AQ_OK) return s2;
       s2 = enq_solve_fixed(cfg.pressure_iterations - solve_sweeps_done());
       if (s2 != AQ_OK) return s2;
@@ -757,16 +765,37 @@ aq_status aq_fluid::build_graph() {
     launches += kUNetForwardLaunches +
                 2 * (plan.by == 5 ? 1 : jacobi_launches(plan.by == 4 ? JacobiPlan{1, 3, 1} : plan, kWarmSweeps) - 1) + 2;
   launches += 1 + 3 + (multiphase ? cfg.diffusion_iterations : 0) + (ink_on && n_ink > 0 ? 1 : 0);
-  graph_launches = launches;
-  cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+  if (sort && rest) graph_launches = launches;
+  cudaError_t e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
-  if (e != cudaSuccess) { exec = nullptr; return fail(AQ_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e)); }
+  if (e != cudaSuccess) { *out = nullptr; return fail(AQ_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e)); }
+  return AQ_OK;
+}
+
+aq_status aq_fluid::build_graph() {
+  invalidate_graph();
+  return capture_step(true, true, &exec);
+}
+
+// One step as two graph launches, with the event `sorted` between them.
+aq_status aq_fluid::step_split() {
+  if (!exec_sort) AQ_TRY(capture_step(true, false, &exec_sort));
+  if (!exec_rest) {
+    nv_cur = 2;
+    AQ_TRY(capture_step(false, true, &exec_rest));
+  }
+  AQ_CUDA(cudaGraphLaunch(exec_sort, stream));
+  AQ_CUDA(cudaEventRecord(sorted, stream));
+  AQ_CUDA(cudaGraphLaunch(exec_rest, stream));
+  time += (double)cfg.timestep;
+  nv_cur = has_cur = 2;
   return AQ_OK;
 }
 
 aq_status aq_fluid::step(int nsteps) {
   if (!use_graph) {
     for (int i = 0; i < nsteps; ++i) {
+      AQ_TRY(enq_sort());
       AQ_TRY(enq_pre_solve());
       if (cfg.solve_mode == AQ_SOLVE_RESIDUAL) AQ_TRY(enq_solve_residual_eager());
       else AQ_TRY(enq_solve_fixed(cfg.pressure_iterations - solve_sweeps_done()));
@@ -1307,19 +1336,38 @@ aq_status aq_fluid_step_host(aq_fluid* f, int32_t n_steps, const float* pin, con
       AQ_CUDA(cudaMemcpyAsync(f->cur.vz, vin + 2 * N, 4 * N, cudaMemcpyHostToDevice, s));
     }
   }
-  AQ_TRY(f->step(n_steps));
-  if (N) {
-    if (pout) {
-      AQ_CUDA(cudaMemcpyAsync(pout, f->cur.px, 4 * N, cudaMemcpyDeviceToHost, s));
-      AQ_CUDA(cudaMemcpyAsync(pout + N, f->cur.py, 4 * N, cudaMemcpyDeviceToHost, s));
-      AQ_CUDA(cudaMemcpyAsync(pout + 2 * N, f->cur.pz, 4 * N, cudaMemcpyDeviceToHost, s));
+  // The particles of a step are final once they are sorted: copies of more
+  // than kSplitBytes go out beside the rest of the last step (below that the
+  // second graph launch and the stream's wait cost more than the copy).
+  const size_t bytes = ((pout ? 12 : 0) + (vout ? 12 : 0)) * N;
+  const bool split = f->use_graph && n_steps > 0 && bytes >= kSplitBytes;
+  cudaStream_t out = s;
+  if (split) {
+    if (!f->copy) {
+      AQ_CUDA(cudaStreamCreateWithFlags(&f->copy, cudaStreamNonBlocking));
+      AQ_CUDA(cudaEventCreateWithFlags(&f->sorted, cudaEventDisableTiming));
+      AQ_CUDA(cudaEventCreateWithFlags(&f->copied, cudaEventDisableTiming));
     }
-    if (vout) {
-      AQ_CUDA(cudaMemcpyAsync(vout, f->cur.vx, 4 * N, cudaMemcpyDeviceToHost, s));
-      AQ_CUDA(cudaMemcpyAsync(vout + N, f->cur.vy, 4 * N, cudaMemcpyDeviceToHost, s));
-      AQ_CUDA(cudaMemcpyAsync(vout + 2 * N, f->cur.vz, 4 * N, cudaMemcpyDeviceToHost, s));
-    }
+    if (n_steps > 1) AQ_TRY(f->step(n_steps - 1));
+    AQ_TRY(f->step_split());
+    AQ_CUDA(cudaStreamWaitEvent(f->copy, f->sorted, 0));
+    out = f->copy;
+  } else {
+    AQ_TRY(f->step(n_steps));
   }
+  const float* dp[3] = {f->cur.px, f->cur.py, f->cur.pz};
+  const float* dv[3] = {f->cur.vx, f->cur.vy, f->cur.vz};
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 3 && N && e == cudaSuccess; ++k) {
+    if (pout) e = cudaMemcpyAsync(pout + k * N, dp[k], 4 * N, cudaMemcpyDeviceToHost, out);
+    if (vout && e == cudaSuccess) e = cudaMemcpyAsync(vout + k * N, dv[k], 4 * N, cudaMemcpyDeviceToHost, out);
+  }
+  if (split) {  // whatever follows on the fluid's stream finds the copies done
+    const cudaError_t r = cudaEventRecord(f->copied, f->copy);
+    const cudaError_t w = cudaStreamWaitEvent(s, f->copied, 0);
+    if (e == cudaSuccess) e = r != cudaSuccess ? r : w;
+  }
+  AQ_CUDA(e);
   return f->health();
 }
 

@@ -13,6 +13,9 @@
 #include "aq_kernels.cuh"
 
 namespace aqb {
+// Host steps copy out this much or more beside their last step's solve.
+constexpr size_t kSplitBytes = 1u << 20;
+
 inline aq_status fail(aq_status st, const std::string& msg) { return set_last_error(st, msg); }
 struct UActs;
 struct MeshState;                  // surface mesher buffers (mesh.cu)
@@ -116,6 +119,11 @@ struct aq_fluid {
   bool ink_on = false;
   aqb::MeshState* mesher = nullptr;  // made by the first aq_fluid_mesh call
   cudaGraphExec_t exec = nullptr;
+  // The step in two graphs, split behind the sort: aq_fluid_step_host copies
+  // the particles out (on `copy`) while the rest of its last step runs.
+  cudaGraphExec_t exec_sort = nullptr, exec_rest = nullptr;
+  cudaStream_t copy = nullptr;
+  cudaEvent_t sorted = nullptr, copied = nullptr;
   bool use_graph = true;
   int graph_launches = 0;  // launches outside the residual loop
   int body_launches = 0;   // launches per residual-loop iteration
@@ -128,7 +136,11 @@ struct aq_fluid {
   ~aq_fluid() {
     if (device >= 0) cudaSetDevice(device);
     if (stream) cudaStreamSynchronize(stream);
-    if (exec) cudaGraphExecDestroy(exec);
+    invalidate_graph();
+    if (copy) cudaStreamSynchronize(copy);
+    if (copy) cudaStreamDestroy(copy);
+    if (sorted) cudaEventDestroy(sorted);
+    if (copied) cudaEventDestroy(copied);
     if (mesher) aqb::mesh_release(mesher);
     for (void* p : allocs) cudaFree(p);
     if (ss_host) cudaFreeHost(ss_host);
@@ -175,10 +187,15 @@ struct aq_fluid {
   aq_status enq_ink();     // advance the ink (no-op without ink)
   aq_status enable_ink();  // seed and allocate the ink once
   aq_status run_stage(int stage);
-  aq_status enq_pre_solve();
+  aq_status enq_sort();       // the step's particle stage
+  aq_status enq_pre_solve();  // the rest up to the solve
   aq_status enq_post_solve();
+  // The step as one graph (split: as two, behind the sort); `sort` and `rest`
+  // choose the parts captured into *out.
+  aq_status capture_step(bool sort, bool rest, cudaGraphExec_t* out);
   aq_status build_graph();
   aq_status step(int nsteps);
+  aq_status step_split();
   aq_status upload(const aq_host_state* s);
   aq_status health();  // synchronises; AQ_ERR_TIMEOUT / AQ_ERR_NONFINITE from the device's records
   aq_status download(aq_host_state* s);
@@ -186,9 +203,9 @@ struct aq_fluid {
                               const std::vector<float>& dens);
   int count_jacobi_launches(int sweeps) const;
   void invalidate_graph() {
-    if (exec) {
-      cudaGraphExecDestroy(exec);
-      exec = nullptr;
+    for (cudaGraphExec_t* e : {&exec, &exec_sort, &exec_rest}) {
+      if (*e) cudaGraphExecDestroy(*e);
+      *e = nullptr;
     }
   }
 };
