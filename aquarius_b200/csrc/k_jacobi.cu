@@ -190,29 +190,41 @@ __host__ __device__ __forceinline__ int resid_flat_parts_dev(const Dims& d) {
   return ((d.sz / 4 + 31) / 32) * ((d.sy + 7) / 8) * d.sx;
 }
 
+// RN(s / 6) for four sums: the corrected reciprocal product (see
+// k_resident.cu's div6_fast) where it is exact, else the divide.  One check
+// for the four instead of a branch in each divide: a sweep of the 128^3
+// workload's rows takes 2.65 us instead of 3.00.
+__device__ __forceinline__ float4 sixth4(const float4& s) {
+  auto key = [](float v) { return 2u * __float_as_uint(v) - 1u; };  // orders magnitudes, 0 above all
+  const unsigned least = min(min(key(s.x), key(s.y)), min(key(s.z), key(s.w)));
+  const float total = (s.x + s.y) + (s.z + s.w);  // finite only if all four are
+  if (least >= 0x07ffffffu && fabsf(total) <= 3.402823466e38f) {  // 2 bits(2^-123) - 1
+    const float r = 0x1.555556p-3f;
+    auto q = [r](float v) {
+      const float q0 = __fmul_rn(v, r);
+      return __fmaf_rn(__fmaf_rn(-q0, 6.0f, v), r, q0);
+    };
+    return make_float4(q(s.x), q(s.y), q(s.z), q(s.w));
+  }
+  return make_float4(__fdiv_rn(s.x, 6.f), __fdiv_rn(s.y, 6.f), __fdiv_rn(s.z, 6.f), __fdiv_rn(s.w, 6.f));
+}
+
 // One Jacobi update of 4 consecutive z cells: p' = (x+1, x-1, y+1, y-1, z+1,
 // z-1 summed in that order, + rhs) / 6 on fluid cells, 0 elsewhere.  Every
 // sweep kernel uses this function, so they agree bit for bit.
 __device__ __forceinline__ float4 jacobi_quad(const float4& xm, const float4& xp, const float4& ym, const float4& yp,
                                               const float4& pc, float zlo, float zhi, const float4& b,
                                               const char4& t) {
-  float4 o;
-  {
-    float s = xp.x + xm.x; s += yp.x; s += ym.x; s += pc.y; s += zlo; s += b.x;
-    o.x = t.x == kFluid ? __fdiv_rn(s, 6.f) : 0.f;
-  }
-  {
-    float s = xp.y + xm.y; s += yp.y; s += ym.y; s += pc.z; s += pc.x; s += b.y;
-    o.y = t.y == kFluid ? __fdiv_rn(s, 6.f) : 0.f;
-  }
-  {
-    float s = xp.z + xm.z; s += yp.z; s += ym.z; s += pc.w; s += pc.y; s += b.z;
-    o.z = t.z == kFluid ? __fdiv_rn(s, 6.f) : 0.f;
-  }
-  {
-    float s = xp.w + xm.w; s += yp.w; s += ym.w; s += zhi; s += pc.z; s += b.w;
-    o.w = t.w == kFluid ? __fdiv_rn(s, 6.f) : 0.f;
-  }
+  float4 s;
+  s.x = xp.x + xm.x; s.x += yp.x; s.x += ym.x; s.x += pc.y; s.x += zlo;  s.x += b.x;
+  s.y = xp.y + xm.y; s.y += yp.y; s.y += ym.y; s.y += pc.z; s.y += pc.x; s.y += b.y;
+  s.z = xp.z + xm.z; s.z += yp.z; s.z += ym.z; s.z += pc.w; s.z += pc.y; s.z += b.z;
+  s.w = xp.w + xm.w; s.w += yp.w; s.w += ym.w; s.w += zhi;  s.w += pc.z; s.w += b.w;
+  float4 o = sixth4(s);
+  if (t.x != kFluid) o.x = 0.f;
+  if (t.y != kFluid) o.y = 0.f;
+  if (t.z != kFluid) o.z = 0.f;
+  if (t.w != kFluid) o.w = 0.f;
   return o;
 }
 
@@ -341,8 +353,10 @@ __global__ void __launch_bounds__(256, 6) k_jacobi_list(Dims d, const float* __r
       pre = true;
     }
   }
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // the next sweep may start its own early part now; it waits for this one
+  // where it reads the iterate
   asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (!early) n = *n_items;
   if (pre) {
     jacobi_row_pre(d, pin, pout, x0, y0, zb0, b0, t0);
@@ -356,46 +370,55 @@ __global__ void __launch_bounds__(256, 6) k_jacobi_list(Dims d, const float* __r
 }
 
 // Ordered list of the active warp rows: id = (x * sy + y) * gz + zb for every
-// row whose 8^3 bricks (x/8, y/8, 16 z bricks of block zb) hold fluid.
+// row whose 8^3 bricks (x/8, y/8, 16 z bricks of block zb) hold fluid.  One
+// CTA: the activity of every (x brick, y brick, zb) is gathered into shared
+// memory first (grids of more than kColumns of them read it from global
+// memory), and a thread lists a run of consecutive ids, so one scan places
+// them all (reading 16 bricks a row and scanning 1024 rows at a time the list
+// of a 128^3 grid took 36 us, 8 us now).
+constexpr int kColumns = 40000;
 __global__ void __launch_bounds__(1024) k_row_items(Dims d, const uint8_t* __restrict__ bact, int* __restrict__ items,
                                                    int* __restrict__ n_items) {
-  __shared__ int s_cnt[32], s_pre[32];
-  __shared__ int s_tot, s_base;
+  __shared__ uint8_t s_col[kColumns];
+  __shared__ int s_cnt[32];
   const int gz = (d.sz / 4 + 31) / 32;
-  const int total = d.sx * d.sy * gz;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  if (threadIdx.x == 0) s_base = 0;
-  __syncthreads();
-  for (int base = 0; base < total; base += 1024) {
-    const int id = base + threadIdx.x;
+  const int cols = d.bx * d.by * gz, total = d.sx * d.sy * gz;
+  auto column = [&](int bx, int by, int zb) -> bool {
+    const uint8_t* p = bact + (bx * d.by + by) * d.bz + zb * 16;
+    const int m = min(16, d.bz - zb * 16);
     int a = 0;
-    if (id < total) {
-      const int zb = id % gz, t = id / gz, y = t % d.sy, x = t / d.sy;
-      for (int k = 0; k < 16 && zb * 16 + k < d.bz && !a; ++k)
-        a = bact[((x / kBrick) * d.by + y / kBrick) * d.bz + zb * 16 + k] ? 1 : 0;
+    for (int k = 0; k < m; ++k) a |= p[k];
+    return a != 0;
+  };
+  const bool cached = cols <= kColumns;
+  if (cached)
+    for (int i = threadIdx.x; i < cols; i += 1024) {
+      const int zb = i % gz, q = i / gz;
+      s_col[i] = column(q / d.by, q % d.by, zb) ? 1 : 0;
     }
-    const unsigned m = __ballot_sync(0xffffffffu, a);
-    const int pre = __popc(m & ((1u << lane) - 1u));
-    if (lane == 0) s_cnt[w] = __popc(m);
-    __syncthreads();
-    if (w == 0) {
-      const int v = s_cnt[lane];
-      int incl = v;
+  __syncthreads();
+  auto active = [&](int id) -> bool {
+    const int zb = id % gz, q = id / gz, y = q % d.sy, x = q / d.sy;
+    const int bx = x / kBrick, by = y / kBrick;
+    return cached ? s_col[(bx * d.by + by) * gz + zb] != 0 : column(bx, by, zb);
+  };
+  const int per = (total + 1023) / 1024, first = threadIdx.x * per, last = min(first + per, total);
+  int n = 0;
+  for (int id = first; id < last; ++id) n += active(id) ? 1 : 0;
+  int incl = n;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int tt = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += tt;
-      }
-      s_pre[lane] = incl - v;
-      if (lane == 31) s_tot = incl;
-    }
-    __syncthreads();
-    if (a) items[s_base + s_pre[w] + pre] = id;
-    __syncthreads();
-    if (threadIdx.x == 0) s_base += s_tot;
-    __syncthreads();
+  for (int o = 1; o < 32; o <<= 1) {
+    const int t = __shfl_up_sync(0xffffffffu, incl, o);
+    if (lane >= o) incl += t;
   }
-  if (threadIdx.x == 0) *n_items = s_base;
+  if (lane == 31) s_cnt[w] = incl;
+  __syncthreads();
+  const int v = s_cnt[lane];
+  int at = __reduce_add_sync(0xffffffffu, lane < w ? v : 0) + incl - n;
+  for (int id = first; id < last; ++id)
+    if (active(id)) items[at++] = id;
+  if (threadIdx.x == 1023) *n_items = at;
 }
 
 // Programmatic dependent launch: the activity bricks were written two or more
@@ -1710,11 +1733,13 @@ cudaError_t launch_row_items(cudaStream_t st, const Dims& d, const uint8_t* bric
 cudaError_t launch_jacobi_list(cudaStream_t st, const Dims& d, const float* pin, float* pout, const float* rhs,
                                const int8_t* type, const int* items, const int* n_items, bool early) {
   if (d.sz % 4 != 0) return cudaErrorInvalidValue;
-  // 8 warps per CTA, one resident wave (4 to 32 warps per CTA and fewer,
-  // fatter waves measured the same or slower at 128^3); the kernel is held
-  // to 40 registers so 6 CTAs fit per SM (888 CTAs, 7104 warps): every warp
-  // of a 128^3 pool's ~6300 rows then has at most one row, and none waits
-  // on a second row's loads after the first (3.02 against 3.29 us a sweep)
+  // 8 warps per CTA, one resident wave; the kernel is held to 40 registers so
+  // 6 CTAs fit per SM (888 CTAs, 7104 warps): every warp of a 128^3 pool's
+  // ~6300 rows then has at most one row.  A row's chain of loads takes about
+  // 1.4 us, so warps with a second row, or fewer warps with four rows' loads
+  // in flight each, lose more than their smaller launch gains (us a sweep:
+  // 888 CTAs of 8 warps 2.62, 444 of 16 2.74, 296 of 22 2.68, 148 of 22 3.3;
+  // 148 CTAs of 12 warps with 4 x 4 row blocks 4.9)
   const int wy = 8;
   const int need = (row_items_capacity(d) + wy - 1) / wy;
   cudaLaunchConfig_t lc = {};
