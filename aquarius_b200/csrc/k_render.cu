@@ -25,6 +25,7 @@
 // The shading is the arithmetic of resources/Shaders/RayTraceEnvironment.glsl,
 // Container_face_fs.glsl, FluidMeshRenderer_fs.glsl, PointSprites_*.glsl.
 #include <algorithm>
+#include <climits>
 #include <cstdint>
 
 #include "aq_kernels.cuh"
@@ -596,6 +597,119 @@ __global__ void __launch_bounds__(64) k_phase(RenderParams P, const int2* __rest
   if (i < P.W && j < P.H) phase[(size_t)j * P.W + i] = acc;
 }
 
+// The same pass where every fraction is 0 or 1 (no two phases have mixed): a
+// pixel's sums are then counts, exact in any order below 2^24, so the sprites
+// need no per-tile lists, no sort and no serial walk.  A CTA takes kSplat
+// consecutive points, counts the pixels that their discs cover in shared
+// memory over the points' common bounding box (neighbours in cell order are
+// close on the screen; a box too large is counted in global memory) and adds
+// the box to the texture.  The tests are k_phase's, pixel for pixel.  A CTA
+// that meets another fraction sets *mixed; the texture is then void.
+// 5.2M sprites in a 1728x864 window: 342 us, against 1.3 ms of k_phase and
+// the 0.5 ms of the lists and their sort.
+constexpr int kSplat = 512, kSplatBox = 5120;  // pixels; two words each
+__global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const float* __restrict__ pts, int n,
+                                                       float* __restrict__ phase,
+                                                       unsigned long long* __restrict__ mixed) {
+  __shared__ unsigned s_cnt[2][kSplatBox];  // phases 0, 1 and 2, 3 in 16-bit halves
+  __shared__ int s_box[4];
+  if (__ldcg(mixed)) return;
+  const int tid = threadIdx.x, i = blockIdx.x * kSplat + tid;
+  if (tid == 0) {
+    s_box[0] = s_box[2] = INT_MAX;
+    s_box[1] = s_box[3] = -1;
+  }
+  float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+  int i0 = 0, i1 = -1, j0 = 0, j1 = -1;
+  unsigned add01 = 0, add23 = 0;
+  bool bad = false;
+  if (i < n) {
+    const float* p = pts + (size_t)i * 7;
+    if (sprite_setup(P, p, s) && sprite_pixels(s, P.W, P.H, i0, i1, j0, j1)) {
+      unsigned f[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const float v = p[3 + k];
+        bad |= !(v == 0.0f || v == 1.0f);
+        f[k] = v == 1.0f ? 1u : 0u;
+      }
+      add01 = f[0] | (f[1] << 16);
+      add23 = f[2] | (f[3] << 16);
+    } else {
+      i1 = j1 = -1;
+    }
+  }
+  if (__syncthreads_or(bad)) {
+    if (tid == 0) atomicExch(mixed, 1ull);
+    return;
+  }
+  const bool draws = (add01 | add23) != 0;
+  // the CTA's box
+  const unsigned all = 0xffffffffu;
+  const int bi0 = __reduce_min_sync(all, draws ? i0 : INT_MAX), bi1 = __reduce_max_sync(all, draws ? i1 : -1);
+  const int bj0 = __reduce_min_sync(all, draws ? j0 : INT_MAX), bj1 = __reduce_max_sync(all, draws ? j1 : -1);
+  if ((tid & 31) == 0) {
+    atomicMin(&s_box[0], bi0);
+    atomicMax(&s_box[1], bi1);
+    atomicMin(&s_box[2], bj0);
+    atomicMax(&s_box[3], bj1);
+  }
+  const int second = __syncthreads_or(add23 != 0);
+  const int ox = s_box[0], oy = s_box[2], w = s_box[1] - ox + 1, h = s_box[3] - oy + 1;
+  if (s_box[1] < 0) return;  // nothing to draw
+  const bool local = (long long)w * h <= kSplatBox;
+  if (local) {
+    for (int k = tid; k < w * h; k += kSplat) {
+      s_cnt[0][k] = 0u;
+      if (second) s_cnt[1][k] = 0u;
+    }
+  }
+  __syncthreads();
+  if (draws) {
+    const float hs = fm(s.z, 0.5f), R2 = fm(hs, hs), in2 = fm(R2, 0.99998f), out2 = fm(R2, 1.00002f);
+    const float lx = fs(s.x, hs), hx = fa(s.x, hs), ly = fs(s.y, hs), hy = fa(s.y, hs);
+    for (int j = j0; j <= j1; ++j) {
+      const float py = fa((float)j, 0.5f);
+      if (!(py >= ly && py < hy)) continue;
+      const float dy = fs(py, s.y), dy2 = fm(dy, dy);
+      for (int q = i0; q <= i1; ++q) {
+        const float px = fa((float)q, 0.5f);
+        if (!(px >= lx && px < hx)) continue;
+        const float dx = fs(px, s.x);
+        const float r2 = fa(fm(dx, dx), dy2);
+        if (r2 > out2) continue;
+        if (!(r2 < in2)) {  // the band: the exact gl_PointCoord arithmetic
+          const float a = fa(fd(dx, s.z), 0.5f), b = fa(fd(dy, s.z), 0.5f);
+          const float x = fs(fm(a, 2.0f), 1.0f), y = fs(fm(b, 2.0f), 1.0f);
+          if (!(fsq(fa(fm(x, x), fm(y, y))) < 1.0f)) continue;
+        }
+        if (local) {
+          const int k = (j - oy) * w + (q - ox);
+          if (add01) atomicAdd(&s_cnt[0][k], add01);
+          if (add23) atomicAdd(&s_cnt[1][k], add23);
+        } else {
+          float* t = phase + ((size_t)j * P.W + q) * 4;
+          if (add01 & 0xffffu) atomicAdd(t, 1.0f);
+          if (add01 >> 16) atomicAdd(t + 1, 1.0f);
+          if (add23 & 0xffffu) atomicAdd(t + 2, 1.0f);
+          if (add23 >> 16) atomicAdd(t + 3, 1.0f);
+        }
+      }
+    }
+  }
+  if (!local) return;
+  __syncthreads();
+  for (int k = tid; k < w * h; k += kSplat) {
+    const int y = k / w, x = k - y * w;
+    float* t = phase + ((size_t)(oy + y) * P.W + (ox + x)) * 4;
+    const unsigned c0 = s_cnt[0][k], c1 = second ? s_cnt[1][k] : 0u;
+    if (c0 & 0xffffu) atomicAdd(t, (float)(c0 & 0xffffu));
+    if (c0 >> 16) atomicAdd(t + 1, (float)(c0 >> 16));
+    if (c1 & 0xffffu) atomicAdd(t + 2, (float)(c1 & 0xffffu));
+    if (c1 >> 16) atomicAdd(t + 3, (float)(c1 >> 16));
+  }
+}
+
 // Sprite-tile list lengths (sort keys for the longest-first order) and tile ids.
 __global__ void __launch_bounds__(256) k_tile_load(const int2* __restrict__ range, int n, unsigned* __restrict__ load,
                                                    int* __restrict__ ids) {
@@ -647,10 +761,28 @@ __global__ void __launch_bounds__(kT * kT) k_frame(RenderParams P, const RenderT
         color = blend(color, trace_env(P, cam, dir));
       }
     if (P.mode <= AQ_RENDER_PHASE1_MESH) {
+      // the warp walks its tile's triangles, 32 at a time, visiting those whose
+      // bounds reach its block, lowest index first (the bounds test per lane
+      // instead of the edge functions of every triangle per pixel)
       const int2 r = trange[tile];
-      if (inside)
-        for (int k = r.x; k < r.y; ++k) {
-          const RenderTri& tr = tris[__ldg(tvals + k)];
+      const int x0 = bx * 256 + 128, x1 = x0 + 7 * 256, y0 = by * 256 + 128, y1 = y0 + 3 * 256;
+      for (int b = r.x; b < r.y; b += 32) {
+        const int kk = b + lane;
+        int id = 0;
+        bool hit = false;
+        if (kk < r.y) {
+          id = __ldg(tvals + kk);
+          const RenderTri& tr = tris[id];
+          const int X0 = tr.X[0], X1 = tr.X[1], X2 = tr.X[2], Y0 = tr.Y[0], Y1 = tr.Y[1], Y2 = tr.Y[2];
+          hit = min(X0, min(X1, X2)) <= x1 && max(X0, max(X1, X2)) >= x0 && min(Y0, min(Y1, Y2)) <= y1 &&
+                max(Y0, max(Y1, Y2)) >= y0;
+        }
+        unsigned mask = __ballot_sync(0xffffffffu, hit);
+        while (mask) {
+          const int q = __ffs(mask) - 1;
+          mask &= mask - 1;
+          const RenderTri& tr = tris[__shfl_sync(0xffffffffu, id, q)];
+          if (!inside) continue;
           float z, a[8];
           if (!tri_fragment(tr, i, j, z, a, false)) continue;
           const uint32_t d = depth24(z);
@@ -669,6 +801,7 @@ __global__ void __launch_bounds__(kT * kT) k_frame(RenderParams P, const RenderT
           }
           color = blend(color, shade_mesh(P, mk3(a[0], a[1], a[2]), mk3(a[5], a[6], a[7]), tex));
         }
+      }
     } else if (P.mode == AQ_RENDER_PARTICLES) {
       // the warp walks its sprite tile's list, 32 sprites at a time, visiting
       // those that reach its block lowest index first
@@ -717,14 +850,24 @@ __global__ void __launch_bounds__(kT * kT) k_frame(RenderParams P, const RenderT
     rgba[(size_t)j * P.W + i] = make_uchar4(color & 0xffu, (color >> 8) & 0xffu, (color >> 16) & 0xffu, color >> 24);
 }
 
+// Staged in shared memory: a thread's seven floats are 28 bytes apart from the
+// next one's, so stored one by one every store of a warp touches 28 sectors
+// (5.2M points: 104 us, 37 us now).
 __global__ void __launch_bounds__(256) k_points_vbo(Particles cur, int n, int phase, float* __restrict__ vbo) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  float* o = vbo + (size_t)i * 7;
-  o[0] = cur.px[i]; o[1] = cur.py[i]; o[2] = cur.pz[i];
-  float4 f = make_float4(phase == 0 ? 1.f : 0.f, phase == 1 ? 1.f : 0.f, phase == 2 ? 1.f : 0.f, phase == 3 ? 1.f : 0.f);
-  if (cur.frac) f = cur.frac[i];
-  o[3] = f.x; o[4] = f.y; o[5] = f.z; o[6] = f.w;
+  __shared__ float s[256 * 7];
+  const int first = blockIdx.x * 256, i = first + threadIdx.x;
+  if (i < n) {
+    float* o = s + threadIdx.x * 7;
+    o[0] = cur.px[i]; o[1] = cur.py[i]; o[2] = cur.pz[i];
+    float4 f = make_float4(phase == 0 ? 1.f : 0.f, phase == 1 ? 1.f : 0.f, phase == 2 ? 1.f : 0.f,
+                           phase == 3 ? 1.f : 0.f);
+    if (phase < 0) f = cur.frac[i];
+    o[3] = f.x; o[4] = f.y; o[5] = f.z; o[6] = f.w;
+  }
+  __syncthreads();
+  const int m = min(256, n - first) * 7;
+  float* out = vbo + (size_t)first * 7;
+  for (int k = threadIdx.x; k < m; k += 256) out[k] = s[k];
 }
 
 }  // namespace
@@ -771,6 +914,13 @@ cudaError_t launch_tile_ranges(cudaStream_t st, const unsigned* keys, int n, int
 cudaError_t launch_phase(cudaStream_t st, const RenderParams& P, const int2* range, const int* order,
                          const int* vals, const float4* spr, const float4* frac, float4* phase) {
   k_phase<<<P.stiles_x * P.stiles_y, 64, 0, st>>>(P, range, order, vals, spr, frac, phase);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_phase_splat(cudaStream_t st, const RenderParams& P, const float* pts, int n, float4* phase,
+                               unsigned long long* mixed) {
+  if (n <= 0) return cudaSuccess;
+  k_phase_splat<<<(n + kSplat - 1) / kSplat, kSplat, 0, st>>>(P, pts, n, reinterpret_cast<float*>(phase), mixed);
   return cudaGetLastError();
 }
 

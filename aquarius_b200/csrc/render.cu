@@ -237,7 +237,7 @@ aq_status aq_renderer_create(int32_t device, void* stream, aq_renderer** out) {
     }
     r->own_stream = true;
   }
-  if (cudaMallocHost(&r->totals_host, 2 * sizeof(unsigned long long)) != cudaSuccess) {
+  if (cudaMallocHost(&r->totals_host, 3 * sizeof(unsigned long long)) != cudaSuccess) {
     delete r;
     return fail(AQ_ERR_OUT_OF_MEMORY, "aq_renderer_create: pinned memory");
   }
@@ -356,11 +356,18 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
   AQR_TRY(r->trange.ensure((size_t)ntiles));
   AQR_TRY(r->ctris.ensure(12));
   AQR_TRY(r->clive.ensure(12));
-  AQR_TRY(r->totals.ensure(2));
-  AQR_CUDA(cudaMemsetAsync(r->totals.p, 0, 2 * sizeof(unsigned long long), st));
+  AQR_TRY(r->totals.ensure(3));  // sprite-tile pairs, triangle-tile pairs, mixed fractions
+  AQR_CUDA(cudaMemsetAsync(r->totals.p, 0, 3 * sizeof(unsigned long long), st));
   AQR_CUDA(cudaMemsetAsync(r->srange.p, 0, sizeof(int2) * nstiles, st));
   AQR_CUDA(cudaMemsetAsync(r->trange.p, 0, sizeof(int2) * ntiles, st));
-  if (need_spr) {
+  // the phase thickness by counting, unless phases have mixed
+  bool splat = P.use_phase && n_points <= kSplatPoints;
+  if (splat) {
+    AQR_CUDA(cudaMemsetAsync(r->phase.p, 0, sizeof(float4) * npx, st));
+    AQR_CUDA(launch_phase_splat(st, P, points, n_points, r->phase.p, r->totals.p + 2));
+    ++r->launches;
+  }
+  auto sprites = [&]() -> aq_status {
     const size_t n = (size_t)n_points;
     AQR_TRY(r->spr.ensure(n));
     AQR_TRY(r->frac.ensure(n));
@@ -371,7 +378,14 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
     AQR_CUDA(launch_sprite_setup(st, P, points, n_points, r->spr.p, r->frac.p, r->scnt.p, r->totals.p));
     AQR_CUDA(launch_cell_scan(st, n_points, r->scnt.p, r->soff.p, r->sscan.p));
     r->launches += 4;
-  }
+    return AQ_OK;
+  };
+  auto read_totals = [&]() -> aq_status {
+    AQR_CUDA(cudaMemcpyAsync(r->totals_host, r->totals.p, 3 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
+    AQR_CUDA(cudaStreamSynchronize(st));
+    return AQ_OK;
+  };
+  if (need_spr && !splat) AQR_TRY(sprites());
   if (need_tri) {
     const size_t n = (size_t)ntri;
     AQR_TRY(r->tris.ensure(n));
@@ -390,12 +404,16 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
     AQR_CUDA(cudaMemsetAsync(r->clive.p, 0, sizeof(int) * 12, st));
   }
   if (need_spr || need_tri) {
-    AQR_CUDA(cudaMemcpyAsync(r->totals_host, r->totals.p, 2 * sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    AQR_CUDA(cudaStreamSynchronize(st));
+    AQR_TRY(read_totals());
+    if (splat && r->totals_host[2]) {
+      splat = false;
+      AQR_TRY(sprites());
+      AQR_TRY(read_totals());
+    }
     if (r->totals_host[0] > (unsigned long long)INT_MAX || r->totals_host[1] > (unsigned long long)INT_MAX)
       return fail(AQ_ERR_INVALID_ARGUMENT, "aq_renderer_draw: more than 2^31 primitive-tile pairs");
   }
-  if (need_spr && r->totals_host[0] > 0) {
+  if (need_spr && !splat && r->totals_host[0] > 0) {
     const int np = (int)r->totals_host[0];
     AQR_TRY(r->skeys.ensure(np)); AQR_TRY(r->skeys2.ensure(np));
     AQR_TRY(r->svals.ensure(np)); AQR_TRY(r->svals2.ensure(np));
@@ -411,7 +429,7 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
     ++r->launches;
     AQR_TRY(r->sort_pairs(r->tkeys, r->tkeys2, r->tvals, r->tvals2, np, ntiles, r->trange));
   }
-  if (P.use_phase) {
+  if (P.use_phase && !splat) {
     // sprite tiles longest list first, so the heaviest start in the first wave
     AQR_TRY(r->tload.ensure(nstiles)); AQR_TRY(r->tload2.ensure(nstiles));
     AQR_TRY(r->tids.ensure(nstiles)); AQR_TRY(r->torder.ensure(nstiles));
@@ -420,7 +438,7 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
     AQR_CUDA(radix_sort_pairs(st, r->tload.p, r->tids.p, r->tload2.p, r->torder.p, nstiles, 32, true, r->sort_tmp.p));
     AQR_CUDA(launch_phase(st, P, r->srange.p, r->torder.p, r->svals2.p, r->spr.p, r->frac.p, r->phase.p));
     r->launches += 2;
-  } else {
+  } else if (!splat) {
     AQR_CUDA(cudaMemsetAsync(r->phase.p, 0, sizeof(float4) * npx, st));
   }
   AQR_TRY(r->ctris.ensure(12));

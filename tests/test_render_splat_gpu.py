@@ -1,0 +1,62 @@
+"""The phase thickness by counting (fractions all 0 or 1) against the oracle's
+sums in submission order: bit for bit, for points in cell order and shuffled
+(a CTA's box too large for shared memory), one and several phases, sprites of
+one pixel to most of the window, numbers of points around a CTA's share, and
+with a fraction that is neither 0 nor 1, which takes the ordered lists."""
+import numpy as np
+import pytest
+
+import aquarius_b200 as aq
+from aquarius_b200 import _abi
+from oracle_binding import RenderOracle
+from test_render_gpu import _draw
+
+pytestmark = pytest.mark.gpu
+
+
+def _points(n, seed, phases, shuffled):
+    rng = np.random.default_rng(seed)
+    side = int(np.ceil(n ** (1 / 3)))
+    grid = np.stack(np.meshgrid(*(np.arange(side),) * 3, indexing="ij"), -1).reshape(-1, 3)[:n]
+    p = np.zeros((n, 7), np.float32)
+    p[:, :3] = (grid + rng.random((n, 3))) * (10.0 / side)
+    f = np.eye(4, dtype=np.float32)[rng.integers(0, phases, n)] if phases else np.zeros((n, 4), np.float32)
+    if phases > 1:
+        f[::7] = 1.0  # several at once, and none
+        f[::11] = 0.0
+    p[:, 3:] = f
+    return np.ascontiguousarray(p[rng.permutation(n)] if shuffled else p)
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("n,phases,shuffled,radius,window", [
+    (1, 1, False, 0.2, (64, 32)),
+    (511, 1, False, 0.2, (333, 197)),
+    (512, 4, False, 0.1, (128, 64)),
+    (513, 2, True, 0.4, (200, 100)),
+    (20000, 1, False, 0.05, (640, 320)),
+    (20000, 4, True, 0.1, (1728, 864)),
+    (700, 2, False, 20.0, (160, 120)),   # sprites over most of the window
+    (3000, 0, False, 0.1, (160, 120)),   # no fraction at all
+])
+def test_counted_thickness_equals_the_ordered_sums(n, phases, shuffled, radius, window, mixed):
+    pts = _points(n, n, phases, shuffled)
+    if mixed:
+        pts[n // 2, 3:] = (0.25, 0.75, 0.0, 0.0)
+    dc = aq.draw_command_default(*window, 10.0, 32)
+    dc.render_mode = _abi.RENDER_MULTIPHASE_MESH
+    dc.point_radius = radius
+    r = aq.Renderer(0)
+    img, got = _draw(r, dc, pts, None)
+    want_img, want = RenderOracle().frame(dc, pts, None)
+    np.testing.assert_array_equal(got, want)
+    np.testing.assert_array_equal(img, want_img)
+    assert phases == 0 or n < 100 or got.any()
+    # the same renderer again, the other way round
+    pts2 = _points(n, n + 1, max(phases, 1), shuffled)
+    if not mixed:
+        pts2[0, 3] = 0.5
+    _, got2 = _draw(r, dc, pts2, None)
+    _, want2 = RenderOracle().frame(dc, pts2, None)
+    np.testing.assert_array_equal(got2, want2)
+    r.close()
