@@ -107,6 +107,64 @@ __device__ __forceinline__ int find_scene(const int* __restrict__ pre, int ns, i
   return lo;
 }
 
+// Two floats in a 64-bit register, and the packed FP32 operations on them (one
+// instruction for both, each rounded as its scalar form).
+using u64 = unsigned long long;
+__device__ __forceinline__ u64 pack2(float a, float b) {
+  u64 r;
+  asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(u64 v) {
+  float2 r;
+  asm("mov.b64 {%0,%1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ u64 add2(u64 a, u64 b) {
+  u64 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
+  u64 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
+  u64 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
+// a * b as its own rounding.  The assembler contracts mul.rn.f32x2 and a
+// following add.rn.f32x2 into one rounding (it leaves the scalar forms alone);
+// a product with -0 added has the same bits and stays apart, if the -0 comes
+// from where the assembler cannot see it (a kernel parameter).
+__device__ __forceinline__ u64 product2(u64 a, u64 b, u64 minus_zero) { return fma2(a, b, minus_zero); }
+
+// Division by a divisor used many times (a constant of the kernels, a
+// distance, a rest density): with y the correctly rounded reciprocal of b, two
+// residual corrections of a * y round as the IEEE division does (Markstein's
+// theorem: the first makes the quotient faithful, the second correct), where
+// nothing over- or underflows: |a| and |b| within 2^-60 .. 2^60, or a = 0.
+// Five FMAs and a check shared by up to three quotients, against a dozen
+// instructions and a branch each.
+struct Divisor {
+  float b, y;
+  bool ok;
+};
+__device__ __forceinline__ Divisor divisor(float b, float y) {
+  return {b, y, fabsf(b) >= 0x1p-60f && fabsf(b) <= 0x1p60f};
+}
+__device__ __forceinline__ float dvd_fast(float a, const Divisor& d) {
+  const float q0 = __fmul_rn(a, d.y);
+  const float q1 = __fmaf_rn(__fmaf_rn(-q0, d.b, a), d.y, q0);
+  return __fmaf_rn(__fmaf_rn(-q1, d.b, a), d.y, q1);
+}
+// 2 bits - 1 orders magnitudes, with 0 above all of them
+__device__ __forceinline__ unsigned mag_key(float a) { return 2u * __float_as_uint(a) - 1u; }
+constexpr unsigned kLeastKey = 0x42ffffffu;  // of 2^-60
+
 // Device-side record of the pressure solve; read back on demand.
 // ||b - A p|| / ||b|| from the squared norms; 0 for an empty system, NaN
 // when either norm is not finite (a NaN or Inf in the right-hand side).

@@ -59,8 +59,6 @@ constexpr int kScanBits = 32;              // scan passes a thread remembers as 
 constexpr int kSmallUnits = 1024;          // grids up to this many units (fluid or not) take one CTA
 static_assert(kCap <= kT * kU && kCap < kZero && kCap % 32 == 0, "a CTA's share must fit its threads");
 
-using u64 = unsigned long long;
-
 struct ClusterScene {
   Dims d;
   float *pa, *pb;
@@ -115,37 +113,11 @@ __device__ __forceinline__ unsigned mapa(unsigned addr, unsigned rank) {
 struct Quad {
   u64 lo, hi;
 };
-__device__ __forceinline__ u64 pack2(float a, float b) {
-  u64 r;
-  asm("mov.b64 %0, {%1,%2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float2 unpack2(u64 v) {
-  float2 r;
-  asm("mov.b64 {%0,%1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
-  return r;
-}
 __device__ __forceinline__ Quad pack4(const float4& v) { return {pack2(v.x, v.y), pack2(v.z, v.w)}; }
 __device__ __forceinline__ float4 unpack4(const Quad& q) {
   const float2 a = unpack2(q.lo), b = unpack2(q.hi);
   return make_float4(a.x, a.y, b.x, b.y);
 }
-__device__ __forceinline__ u64 add2(u64 a, u64 b) {
-  u64 r;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ u64 mul2(u64 a, u64 b) {
-  u64 r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ u64 fma2(u64 a, u64 b, u64 c) {
-  u64 r;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-  return r;
-}
-
 // Loads and stores at an address of buffer 0, OFF bytes on.  They are
 // volatile, so they keep their place between the barriers; no other access
 // touches the buffers.

