@@ -5,6 +5,9 @@
 // Reference: Fluid/Fluid_3D_FLIP.cu:8-186 (P2G, divide, fractions, counts),
 // Fluid/Fluid_3D_kernels.cu:4-98 (gravity, fixBoundary), :118-207 (pressure
 // update), :210-422 (extrapolation), :426-458 (divergence), :520-556 (diffusion).
+#include <algorithm>
+#include <type_traits>
+
 #include "aq_kernels.cuh"
 
 namespace aqb {
@@ -24,31 +27,6 @@ __device__ __forceinline__ void p2g_particle(int DX, int DY, int DZ, float qx, f
   const float bx = hat1(__fsub_rn(qx, fxh)), by = hat1(__fsub_rn(qy, fyh)), bz = hat1(__fsub_rn(qz, fzh));
   if (DX < 1) {  // a cell at dx = +1 cannot touch the u face (weight exactly 0)
     const float w = __fmul_rn(__fmul_rn(hat1(__fsub_rn(qx, fx)), by), bz);
-    su = __fmaf_rn(w, vx, su);
-    wu = __fadd_rn(wu, w);
-  }
-  if (DY < 1) {
-    const float w = __fmul_rn(__fmul_rn(bx, hat1(__fsub_rn(qy, fy))), bz);
-    sv = __fmaf_rn(w, vy, sv);
-    wv = __fadd_rn(wv, w);
-  }
-  if (DZ < 1) {
-    const float w = __fmul_rn(__fmul_rn(bx, by), hat1(__fsub_rn(qz, fz)));
-    sw = __fmaf_rn(w, vz, sw);
-    ww = __fadd_rn(ww, w);
-  }
-  bxyz = __fmul_rn(__fmul_rn(bx, by), bz);
-}
-
-// p2g_particle with the x factors already evaluated: ax = hat1(qx - fx) and
-// bx = hat1(qx - fxh), the same values (a staged plane shares the node x).
-__device__ __forceinline__ void p2g_particle_x(int DX, int DY, int DZ, float ax, float bx, float qy, float qz,
-                                               float vx, float vy, float vz, float fy, float fz, float fyh,
-                                               float fzh, float& su, float& sv, float& sw, float& wu, float& wv,
-                                               float& ww, float& bxyz) {
-  const float by = hat1(__fsub_rn(qy, fyh)), bz = hat1(__fsub_rn(qz, fzh));
-  if (DX < 1) {
-    const float w = __fmul_rn(__fmul_rn(ax, by), bz);
     su = __fmaf_rn(w, vx, su);
     wu = __fadd_rn(wu, w);
   }
@@ -214,126 +192,231 @@ __global__ void __launch_bounds__(256) k_p2g(Dims d, StepParams sp, Particles cu
 }
 
 // ------------------------------------------------------- shared-memory P2G
-// The gather of p2g_body (same arithmetic, same (dx, dy, dz, j) order, same
-// epilogue) with the particles staged in shared memory.  A CTA owns the
-// nodes of one x plane, 8 y rows and 32 z columns, one per thread.  For each
-// dx it stages, once and coalesced, the particles of the cells it reads in
-// plane x + dx (10 rows of 34 cells: its own rows and columns and a one-cell
-// rim), into cell-major slots: slot k of cell c sits at k * kP2gCells + c.
-// A slot holds the particle's two x hat factors (the CTA's nodes share one
-// x, so they are the particle's for the whole plane), its y and z in cell
-// units and its velocity.  The 32 lanes of a warp read the k-th
-// particle of 32 consecutive cells, i.e. 32 consecutive words and 32
-// distinct banks, where the one-thread-per-node kernel's lanes gathered from
-// scattered addresses through L1.  A cell holding more than kP2gSlots
-// particles reads the rest from global memory.
-constexpr int kP2gCols = 34, kP2gRows = 10, kP2gCells = kP2gCols * kP2gRows;
-constexpr int p2g_smem(int slots) { return 7 * slots * kP2gCells * (int)sizeof(float); }
+// The gather of p2g_body (same sums in the same (dx, dy, dz, j) order, same
+// epilogue) marching along x with the particles staged in shared memory.  A
+// CTA owns 4 y rows and 32 z columns of nodes, one (y, z) column per thread,
+// over `planes` x planes.  It stages each plane of cells once (6 rows of 34:
+// its own and a one-cell rim) and adds the plane's particles to the three
+// nodes of the column they touch: x - 1 (as dx = +1), x (dx = 0) and x + 1
+// (dx = -1), so a node collects its planes in the reference's order, and the
+// loads and the y and z hat factors serve three nodes.
+// A row of cells is one contiguous run of the sorted particles, so a warp
+// reads it coalesced and scatters it to cell-major slots: slot k of cell c at
+// k * kP2gCells + c, where the 32 lanes of a warp find the k-th particles of
+// 32 consecutive cells in 32 distinct banks.  A cell holding more than
+// kP2gSlots particles reads the rest from global memory.
+// Bound by FP32 issue (about 60 instructions per particle, cell of the column
+// and three nodes; 62% of the issue slots at 4 CTAs an SM).  One plane per
+// CTA, each staging all three planes cell by cell, took 484 us for 5.2M
+// particles on 128^3 (267 now), 268 for 2.6M on 96^3 multiphase (172) and 57
+// for 214k on 50^3 (50).  A thread for each of u, v and w took 390 at 128^3 and
+// nodes x and x + 1 in packed halves the same time as scalar.
+constexpr int kP2gY = 4, kP2gCols = 34, kP2gRows = kP2gY + 2, kP2gCells = kP2gCols * kP2gRows;
+constexpr int kP2gThreads = kP2gY * 32;
+constexpr int p2g_smem(int slots) { return 6 * slots * kP2gCells * (int)sizeof(float); }
+
+// hat1 with the lower clamp as the subtraction's saturation (1 - |r| <= 1)
+__device__ __forceinline__ float hat1s(float r) { return __saturatef(__fsub_rn(1.f, fabsf(r))); }
+
+// One particle's terms of one node from its hat factors (p2g_particle's
+// products and sums); U, V, W: the components its cell can touch.
+template <bool U, bool V, bool W>
+__device__ __forceinline__ void p2g_node(float ax, float bx, float ay, float by, float az, float bz, float vx, float vy,
+                                         float vz, float& su, float& sv, float& sw, float& wu, float& wv, float& ww) {
+  if (U) {
+    const float w = __fmul_rn(__fmul_rn(ax, by), bz);
+    su = __fmaf_rn(w, vx, su);
+    wu = __fadd_rn(wu, w);
+  }
+  if (V) {
+    const float w = __fmul_rn(__fmul_rn(bx, ay), bz);
+    sv = __fmaf_rn(w, vy, sv);
+    wv = __fadd_rn(wv, w);
+  }
+  if (W) {
+    const float w = __fmul_rn(__fmul_rn(bx, by), az);
+    sw = __fmaf_rn(w, vz, sw);
+    ww = __fadd_rn(ww, w);
+  }
+}
 
 template <bool FORCES, bool MULTI, int kP2gSlots>
-__global__ void __launch_bounds__(256, kP2gSlots <= 7 ? 3 : (kP2gSlots <= 11 ? 2 : 1)) k_p2g_tiled(Dims d, StepParams sp, Particles cur, const int* __restrict__ off,
-                                                     float* __restrict__ u0, float* __restrict__ v0,
-                                                     float* __restrict__ w0, float* __restrict__ un,
-                                                     float* __restrict__ vn, float* __restrict__ wn,
-                                                     int8_t* __restrict__ type, float* __restrict__ density,
-                                                     float4* __restrict__ vf, float4* __restrict__ nvf) {
-  // hat1(qx - fx), hat1(qx - fxh), qy, qz, vx, vy, vz: [kP2gSlots][kP2gCells] each (the x
-  // factors are per particle: the CTA's nodes share one x)
+__global__ void __launch_bounds__(kP2gThreads, kP2gSlots <= 7 ? 6 : (kP2gSlots <= 11 ? 4 : 2))
+    k_p2g_march(Dims d, StepParams sp, Particles cur, const int* __restrict__ off, float* __restrict__ u0,
+                float* __restrict__ v0, float* __restrict__ w0, float* __restrict__ un, float* __restrict__ vn,
+                float* __restrict__ wn, int8_t* __restrict__ type, float* __restrict__ density,
+                float4* __restrict__ vf, float4* __restrict__ nvf, int planes) {
+  // px, py, pz in cell units, vx, vy, vz: [kP2gSlots][kP2gCells] each
   extern __shared__ float p2g_sm[];
   __shared__ int s_beg[kP2gCells], s_cnt[kP2gCells];
   constexpr int A = kP2gSlots * kP2gCells;
-  float* const sax = p2g_sm;
-  float* const sbx = sax + A;
-  float* const sqy = sbx + A;
-  float* const sqz = sqy + A;
-  float* const svx = sqz + A;
-  float* const svy = svx + A;
-  float* const svz = svy + A;
   const int lane = threadIdx.x, wy = threadIdx.y, tid = wy * 32 + lane;
-  const int z0 = blockIdx.x * 32, y0 = blockIdx.y * 8, x = blockIdx.z;
+  const int z0 = blockIdx.x * 32, y0 = blockIdx.y * kP2gY, x0 = blockIdx.z * planes;
+  const int x1 = min(x0 + planes, d.sx);
   const int z = z0 + lane, y = y0 + wy;
   const bool node = z < d.sz && y < d.sy;
-  const float fx = (float)x, fy = (float)y, fz = (float)z;
-  const float fxh = fx + 0.5f, fyh = fy + 0.5f, fzh = fz + 0.5f;
+  const float fy = (float)y, fz = (float)z;
+  const float fyh = fy + 0.5f, fzh = fz + 0.5f;
   const float inv_h = d.inv_h;
-  float su = 0.f, sv = 0.f, sw = 0.f, wu = 0.f, wv = 0.f, ww = 0.f;
-  float4 fs = make_float4(0.f, 0.f, 0.f, 0.f);
-  float fw = 0.f;
-  int own = 0, left = 0, down = 0, back = 0;
+
+  // this thread's cells of a plane: first particle and count
+  constexpr int NC = (kP2gCells + kP2gThreads - 1) / kP2gThreads;
+  int pb[NC], pn[NC];
+  auto offsets = [&](int X) {
 #pragma unroll
-  for (int dx = -1; dx <= 1; ++dx) {
-    const int X = x + dx;
-    if (X < 0 || X >= d.sx) continue;  // the same for the whole CTA
-    __syncthreads();                   // the previous plane's slots are consumed
-    for (int lc = tid; lc < kP2gCells; lc += 256) {
+    for (int q = 0; q < NC; ++q) {
+      const int lc = tid + q * kP2gThreads;
+      pb[q] = 0;
+      pn[q] = 0;
       const int Y = y0 - 1 + lc / kP2gCols, Z = z0 - 1 + lc % kP2gCols;
-      int b = 0, n = 0;
-      if (Y >= 0 && Y < d.sy && Z >= 0 && Z < d.sz) {
-        const int c = (X * d.sy + Y) * d.sz + Z;
-        b = __ldg(off + c);
-        n = __ldg(off + c + 1) - b;
-      }
-      s_beg[lc] = b;
-      s_cnt[lc] = n;
-      const int m = min(n, kP2gSlots);
-      for (int k = 0; k < m; ++k) {
-        const int j = b + k, sl = k * kP2gCells + lc;
-        const float qx = __fmul_rn(__ldg(cur.px + j), inv_h);
-        sax[sl] = hat1(__fsub_rn(qx, fx));
-        sbx[sl] = hat1(__fsub_rn(qx, fxh));
-        sqy[sl] = __fmul_rn(__ldg(cur.py + j), inv_h);
-        sqz[sl] = __fmul_rn(__ldg(cur.pz + j), inv_h);
-        svx[sl] = __ldg(cur.vx + j);
-        svy[sl] = __ldg(cur.vy + j);
-        svz[sl] = __ldg(cur.vz + j);
+      if (lc < kP2gCells && X >= 0 && X < d.sx && Y >= 0 && Y < d.sy) {
+        const int* row = off + (X * d.sy + Y) * d.sz;
+        pb[q] = __ldg(row + min(max(Z, 0), d.sz));  // outside in z: empty, at the row's end
+        if (Z >= 0 && Z < d.sz) pn[q] = __ldg(row + Z + 1) - pb[q];
       }
     }
-    __syncthreads();
-    if (!node) continue;
-    // dy and dz stay loops (the branches on them are uniform across the
-    // warp): 27 unrolled copies of the particle loop overflow the
-    // instruction cache
-#pragma unroll 1
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int Y = y + dy;
-      if (Y < 0 || Y >= d.sy) continue;
-#pragma unroll 1
-      for (int dz = -1; dz <= 1; ++dz) {
-        const int Z = z + dz;
-        if (Z < 0 || Z >= d.sz) continue;
-        const int lc = (wy + 1 + dy) * kP2gCols + lane + 1 + dz;
-        const int b = s_beg[lc], n = s_cnt[lc];
-        if (dx == 0 && dy == 0 && dz == 0) own = n;
-        if (dx == -1 && dy == 0 && dz == 0) left = n;
-        if (dx == 0 && dy == -1 && dz == 0) down = n;
-        if (dx == 0 && dy == 0 && dz == -1) back = n;
-        const int m = min(n, kP2gSlots);
-        for (int k = 0; k < m; ++k) {  // the staged slots
-          const int sl = k * kP2gCells + lc;
-          float bxyz;
-          p2g_particle_x(dx, dy, dz, sax[sl], sbx[sl], sqy[sl], sqz[sl], dx < 1 ? svx[sl] : 0.f,
-                         dy < 1 ? svy[sl] : 0.f, dz < 1 ? svz[sl] : 0.f, fy, fz, fyh, fzh, su, sv, sw, wu, wv, ww,
-                         bxyz);
-          if (MULTI && dx == 0 && dy == 0 && dz == 0) p2g_fractions(bxyz, cur.frac[b + k], fs, fw);
-        }
-        for (int k = m; k < n; ++k) {  // a crowded cell's particles beyond the slots
-          const int j = b + k;
-          float bxyz;
-          p2g_particle(dx, dy, dz, __fmul_rn(__ldg(cur.px + j), inv_h), __fmul_rn(__ldg(cur.py + j), inv_h),
-                       __fmul_rn(__ldg(cur.pz + j), inv_h), dx < 1 ? __ldg(cur.vx + j) : 0.f,
-                       dy < 1 ? __ldg(cur.vy + j) : 0.f, dz < 1 ? __ldg(cur.vz + j) : 0.f, fx, fy, fz, fxh, fyh, fzh,
-                       su, sv, sw, wu, wv, ww, bxyz);
-          if (MULTI && dx == 0 && dy == 0 && dz == 0) p2g_fractions(bxyz, cur.frac[j], fs, fw);
-        }
+  };
+
+  P2gAcc a{}, c{};
+  P2gAcc b{};
+  int left1 = 0;  // node x + 1's
+
+  offsets(x0 - 1);
+  for (int X = x0 - 1; X <= x1; ++X) {
+    __syncthreads();  // the previous plane's slots are consumed
+    int any = 0;
+#pragma unroll
+    for (int q = 0; q < NC; ++q) {
+      const int lc = tid + q * kP2gThreads;
+      if (lc < kP2gCells) {
+        s_beg[lc] = pb[q];
+        s_cnt[lc] = pn[q];
+        any |= pn[q];
       }
     }
+    any = __syncthreads_or(any);
+    if (X < x1) offsets(X + 1);
+    float4 fs = make_float4(0.f, 0.f, 0.f, 0.f);
+    float fw = 0.f;
+    int own = 0, down = 0, back = 0;
+    if (any) {
+      // a warp reads its own row and half of row 4 or 5, 4 + 2 particles a lane
+      // in flight
+      const int r1 = kP2gY + (wy >> 1);
+      auto row_end = [&](int r) { return s_beg[r * kP2gCols + kP2gCols - 1] + s_cnt[r * kP2gCols + kP2gCols - 1]; };
+      const int je0 = row_end(wy), je1 = row_end(r1);
+      int j0 = s_beg[wy * kP2gCols] + lane, j1 = s_beg[r1 * kP2gCols] + (wy & 1) * 32 + lane;
+#pragma unroll 1
+      for (; j0 < je0 || j1 < je1; j0 += 128, j1 += 128) {
+        float v[6][6];
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+          const int j = q < 4 ? j0 + q * 32 : j1 + (q - 4) * 64;
+          if (j < (q < 4 ? je0 : je1)) {
+            v[q][0] = __ldg(cur.px + j); v[q][1] = __ldg(cur.py + j); v[q][2] = __ldg(cur.pz + j);
+            v[q][3] = __ldg(cur.vx + j); v[q][4] = __ldg(cur.vy + j); v[q][5] = __ldg(cur.vz + j);
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+          const int j = q < 4 ? j0 + q * 32 : j1 + (q - 4) * 64;
+          if (j < (q < 4 ? je0 : je1)) {
+            const int row = (q < 4 ? wy : r1) * kP2gCols;
+            const float qz = __fmul_rn(v[q][2], inv_h);
+            // the cell whose run holds j: the position's, but for its rounding
+            int lc = row + min(max((int)qz - (z0 - 1), 0), kP2gCols - 1);
+            int k = j - s_beg[lc];
+            if (k < 0 || k >= s_cnt[lc]) {
+              lc = row;
+              while (j >= s_beg[lc] + s_cnt[lc]) ++lc;  // j is below the row's end
+              k = j - s_beg[lc];
+            }
+            if (k < kP2gSlots) {
+              float* const sl = p2g_sm + k * kP2gCells + lc;
+              sl[0] = __fmul_rn(v[q][0], inv_h);
+              sl[A] = __fmul_rn(v[q][1], inv_h);
+              sl[2 * A] = qz;
+              sl[3 * A] = v[q][3];
+              sl[4 * A] = v[q][4];
+              sl[5 * A] = v[q][5];
+            }
+          }
+        }
+      }
+      __syncthreads();
+      if (node) {
+        const float fx = (float)X, fx1 = (float)(X + 1);
+        const float fxh0 = (float)(X - 1) + 0.5f, fxh = fx + 0.5f, fxh1 = fx1 + 0.5f;
+        // the particles of cell (X, y + DY, z + DZ); WHICH = 0: the plane before
+        // the CTA's own, for node x + 1 alone; 1: for all three; 2: the plane
+        // after, for node x - 1 alone; 3: a CTA's single plane, for node x alone
+        auto cell = [&](auto which, auto dyc, auto dzc) {
+          constexpr int WHICH = decltype(which)::value, DY = decltype(dyc)::value, DZ = decltype(dzc)::value;
+          if (WHICH == 2 && DY == 1 && DZ == 1) return;
+          const int lc = (wy + 1 + DY) * kP2gCols + lane + 1 + DZ;
+          const int n = s_cnt[lc];
+          if (DY == 0 && DZ == 0) own = n;
+          if (DY == -1 && DZ == 0) down = n;
+          if (DY == 0 && DZ == -1) back = n;
+          const float* sl = p2g_sm + lc;
+          constexpr int kUnroll = WHICH == 1 ? 1 : 2;
+#pragma unroll kUnroll
+          for (int k = 0; k < n; ++k, sl += kP2gCells) {
+            float qx, qy, qz, vx, vy, vz;
+            if (k < kP2gSlots) {
+              qx = sl[0]; qy = sl[A]; qz = sl[2 * A];
+              vx = sl[3 * A]; vy = sl[4 * A]; vz = sl[5 * A];
+            } else {  // a crowded cell's particles beyond the slots
+              const int j = s_beg[lc] + k;
+              qx = __fmul_rn(__ldg(cur.px + j), inv_h);
+              qy = __fmul_rn(__ldg(cur.py + j), inv_h);
+              qz = __fmul_rn(__ldg(cur.pz + j), inv_h);
+              vx = __ldg(cur.vx + j); vy = __ldg(cur.vy + j); vz = __ldg(cur.vz + j);
+            }
+            const float by = hat1s(__fsub_rn(qy, fyh)), bz = hat1s(__fsub_rn(qz, fzh));
+            const float ay = hat1s(__fsub_rn(qy, fy)), az = hat1s(__fsub_rn(qz, fz));
+            if (WHICH == 0) {
+              const float b1 = hat1s(__fsub_rn(qx, fxh1)), a1 = hat1s(__fsub_rn(qx, fx1));
+              p2g_node<true, DY < 1, DZ < 1>(a1, b1, ay, by, az, bz, vx, vy, vz, c.su, c.sv, c.sw, c.wu, c.wv, c.ww);
+            }
+            if (WHICH == 1 || WHICH == 3) {
+              const float b0 = hat1s(__fsub_rn(qx, fxh)), b1 = hat1s(__fsub_rn(qx, fxh1));
+              const float a0 = hat1s(__fsub_rn(qx, fx)), a1 = hat1s(__fsub_rn(qx, fx1));
+              p2g_node<true, DY < 1, DZ < 1>(a0, b0, ay, by, az, bz, vx, vy, vz, b.su, b.sv, b.sw, b.wu, b.wv, b.ww);
+              if (WHICH == 1)
+                p2g_node<true, DY < 1, DZ < 1>(a1, b1, ay, by, az, bz, vx, vy, vz, c.su, c.sv, c.sw, c.wu, c.wv, c.ww);
+              if (MULTI && DY == 0 && DZ == 0)
+                p2g_fractions(__fmul_rn(__fmul_rn(b0, by), bz), cur.frac[s_beg[lc] + k], fs, fw);
+            }
+            if (WHICH == 1 || WHICH == 2)
+              p2g_node<false, DY < 1, DZ < 1>(0.f, hat1s(__fsub_rn(qx, fxh0)), ay, by, az, bz, vx, vy, vz, a.su, a.sv,
+                                              a.sw, a.wu, a.wv, a.ww);
+          }
+        };
+        auto plane = [&](auto which) {
+          using M1 = std::integral_constant<int, -1>;
+          using C0 = std::integral_constant<int, 0>;
+          using P1 = std::integral_constant<int, 1>;
+          cell(which, M1(), M1()); cell(which, M1(), C0()); cell(which, M1(), P1());
+          cell(which, C0(), M1()); cell(which, C0(), C0()); cell(which, C0(), P1());
+          cell(which, P1(), M1()); cell(which, P1(), C0()); cell(which, P1(), P1());
+        };
+        if (X < x0) plane(std::integral_constant<int, 0>());
+        else if (X == x1) plane(std::integral_constant<int, 2>());
+        else if (planes == 1) plane(std::integral_constant<int, 3>());
+        else plane(std::integral_constant<int, 1>());
+      }
+    }
+    if (node && X > x0)
+      p2g_finish<FORCES, MULTI>(d, sp, X - 1, y, z, a, u0, v0, w0, un, vn, wn, type, density, vf, nvf);
+    // on to the next plane: node x becomes x - 1, x + 1 becomes x
+    a = b;
+    b = c;
+    c = P2gAcc{};
+    a.fs = fs; a.fw = fw;
+    a.own = own; a.left = left1; a.down = down; a.back = back;
+    left1 = own;
   }
-  if (!node) return;
-  P2gAcc a;
-  a.su = su; a.sv = sv; a.sw = sw; a.wu = wu; a.wv = wv; a.ww = ww;
-  a.fs = fs; a.fw = fw;
-  a.own = own; a.left = left; a.down = down; a.back = back;
-  p2g_finish<FORCES, MULTI>(d, sp, x, y, z, a, u0, v0, w0, un, vn, wn, type, density, vf, nvf);
 }
 
 // node-grid virtual block -> (z block, y block, x plane) of one scene
@@ -798,21 +881,35 @@ cudaError_t launch_batch_extrapolate(cudaStream_t st, const BatchIndex& bi, int 
 }
 
 // 0: one thread per node through L1; 1, 2, 3: shared-memory staged with
-// 11, 7 or 16 slots per cell (2, 3 or 1 CTAs per SM; with fewer slots more
+// 11, 7 or 16 slots per cell (4, 6 or 2 CTAs per SM; with fewer slots more
 // crowded cells read partly from global memory)
 static int g_p2g_variant = 1;
 void set_p2g_variant(int v) { g_p2g_variant = v; }
 int p2g_variant() { return g_p2g_variant; }
+
+// x planes per CTA: a chunk of L planes stages L + 2, so longer chunks do less
+// work, as long as there are CTAs enough (4 fit on an SM and a grid's CTAs
+// over its air finish at once).  1400 CTAs or more are kept, at most 5 planes.
+// P2G in us at 1, 2, 3, 5 planes: 50^3 (1300 columns x planes) 50, 62, 65, 84;
+// 90 x 61 x 75 (4320) 130, 112, 93, 115; multiphase 96^3 (6912) 248, 201, 183,
+// 172; 128^3 (16384) 515, 334, 291, 267 and no better with more.
+static int p2g_planes(const Dims& d) {
+  const long long ctas = (long long)((d.sz + 31) / 32) * ((d.sy + kP2gY - 1) / kP2gY) * d.sx;
+  return (int)std::min(std::max((ctas + 700) / 1400, 1LL), 5LL);
+}
 
 template <bool F, bool M, int SLOTS>
 static cudaError_t launch_p2g_slots(cudaStream_t st, const Dims& d, const StepParams& sp, Particles cur,
                                     const int* off, float* u0, float* v0, float* w0, float* un, float* vn,
                                     float* wn, int8_t* type, float* density, float4* vf, float4* nvf) {
   constexpr int smem = p2g_smem(SLOTS);
-  cudaError_t e = cudaFuncSetAttribute(k_p2g_tiled<F, M, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cudaFuncSetAttribute(k_p2g_march<F, M, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  k_p2g_tiled<F, M, SLOTS><<<node_grid(d), dim3(32, 8), smem, st>>>(d, sp, cur, off, u0, v0, w0, un, vn, wn, type,
-                                                                     density, vf, nvf);
+  const int tiles = ((d.sz + 31) / 32) * ((d.sy + kP2gY - 1) / kP2gY);
+  const int planes = p2g_planes(d);
+  const dim3 grid((d.sz + 31) / 32, (d.sy + kP2gY - 1) / kP2gY, (d.sx + planes - 1) / planes);
+  k_p2g_march<F, M, SLOTS><<<grid, dim3(32, kP2gY), smem, st>>>(d, sp, cur, off, u0, v0, w0, un, vn, wn, type, density,
+                                                               vf, nvf, planes);
   return cudaGetLastError();
 }
 

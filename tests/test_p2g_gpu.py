@@ -11,7 +11,7 @@ import pytest
 import aquarius_b200 as aq
 from aquarius_b200 import _abi
 from oracle_binding import Oracle
-from scenes import SCENES, rel_l2
+from scenes import SCENES, ball_drop, rel_l2
 
 pytestmark = pytest.mark.gpu
 
@@ -91,3 +91,22 @@ def test_staged_p2g_overflowing_cells_and_init_transfer():
     np.testing.assert_array_equal(b["content"], want["content"])
     o.close()
     assert n > 200
+
+
+@pytest.mark.parametrize("size,multi", [((48, 64, 70), False), ((67, 83, 65), False), ((67, 83, 65), True),
+                                        ((33, 130, 129), False), ((81, 95, 97), True)])
+def test_staged_p2g_chunks_of_planes(size, multi):
+    """Grids large enough for 2, 3, 4 and 5 x planes to a CTA, with ragged last
+    chunks, rows and columns."""
+    cfg = ball_drop(size, pool=0.25, center=(0.5, 0.7, 0.5), radius=0.12, dt=0.005, phase_ball=1 if multi else 0,
+                    pressure_iterations=20)
+    st = _state(cfg, 1)
+    try:
+        _variant(0)
+        a = _p2g(cfg, st)
+        _variant(1)
+        b = _p2g(cfg, st)
+    finally:
+        _variant(1)
+    for k in P2G_FIELDS:
+        np.testing.assert_array_equal(b[k], a[k], err_msg=k)
