@@ -133,9 +133,12 @@ cudaError_t launch_project(cudaStream_t st, const Dims& d, const int8_t* type, c
 cudaError_t launch_extrapolate(cudaStream_t st, const Dims& d, const float* ui, const float* vi,
                                const float* wi, const uint8_t* hi, float* uo, float* vo, float* wo,
                                uint8_t* ho);
-// One diffusionJacobi sweep of the phase fractions (multiphase only).
+// Sweep `sweep` of diffusionJacobi of the phase fractions (multiphase only); the
+// first one lists the tiles that hold fluid for the others.
 cudaError_t launch_diffuse(cudaStream_t st, const Dims& d, const int8_t* type, float lambda,
-                           const float4* fin, float4* fout);
+                           const float4* fin, float4* fout, int* items, int sweep);
+// Ints of the sweeps' tile list, without its count (one more).
+size_t diffuse_items(const Dims& d);
 
 // ---- pressure (k_jacobi.cu) -------------------------------------------------
 struct JacobiPlan {

@@ -257,6 +257,7 @@ aq_status aq_fluid::allocate() {
   AQ_TRY(alloc(&type, C)); AQ_TRY(alloc(&density, C)); AQ_TRY(alloc(&div, C)); AQ_TRY(alloc(&rhs, C));
   AQ_TRY(alloc(&pa, C)); AQ_TRY(alloc(&pb, C)); AQ_TRY(alloc(&pcount, C));
   AQ_TRY(alloc(&vf, C)); AQ_TRY(alloc(&nvf, C)); AQ_TRY(alloc(&nvf2, C));
+  AQ_TRY(alloc(&diffuse_list, diffuse_items(d) + 1));
   nbricks = d.bx * d.by * d.bz;
   AQ_TRY(alloc(&bact, (size_t)nbricks)); AQ_TRY(alloc(&part_b2, (size_t)nbricks));
   AQ_TRY(alloc(&part_nf, (size_t)nbricks));
@@ -573,7 +574,7 @@ aq_status aq_fluid::enq_diffuse() {
   float4* a = nvf;
   float4* b = nvf2;
   for (int i = 0; i < cfg.diffusion_iterations; ++i) {
-    AQ_CUDA(launch_diffuse(stream, d, type, lambda, a, b));
+    AQ_CUDA(launch_diffuse(stream, d, type, lambda, a, b, diffuse_list, i));
     std::swap(a, b);
   }
   if (a != nvf) AQ_CUDA(cudaMemcpyAsync(nvf, a, sizeof(float4) * d.C, cudaMemcpyDeviceToDevice, stream));

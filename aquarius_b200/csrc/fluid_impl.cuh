@@ -78,6 +78,7 @@ struct aq_fluid {
   float *density = nullptr, *div = nullptr, *rhs = nullptr, *pa = nullptr, *pb = nullptr;
   int* pcount = nullptr;
   float4 *vf = nullptr, *nvf = nullptr, *nvf2 = nullptr;
+  int* diffuse_list = nullptr;  // tiles that hold fluid, and their count
   uint8_t* bact = nullptr;
   double* part_b2 = nullptr;
   int* part_nf = nullptr;
