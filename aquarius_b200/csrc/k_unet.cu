@@ -357,133 +357,199 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
-__host__ __device__ constexpr int tmem_cols(int n) { return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : 256; }
+__host__ __device__ constexpr int tmem_cols(int n) {
+  return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512;
+}
 
-// Output block of the tcgen05 kernel: 2 (x) x 16 (y) x 8 (z) voxels, two
-// M = 128 tiles (one per x plane, row m = 8 y + z).  Its input halo
-// (4 x 18 x 10 voxels) is stored per 8-channel chunk as z columns of 10 rows
-// of 16 B: the A operand of any tap is then a descriptor into the halo
-// itself — rows of a core matrix are 8 consecutive z (16 B apart), the 16
-// core matrices along M are the y columns (SBO = 160 B), the two along K the
-// chunk planes (LBO) — so no per-tap copy and no per-tap barrier: the CTA
-// loads the halo and all 27 taps' weights, one thread issues every MMA and
-// commits once.  On B200 the 128^3 network's inference takes 1.55 ms this
-// way against 1.64 ms with k_conv3_fwd_tile; per layer it is ahead where
-// COUT is 32 and behind at 128^3 with COUT = 16, whose N = 16 MMAs are too
-// narrow to keep the tensor pipe busy.
-constexpr int kUX = 2, kUY = 16, kUZ = 8;
-constexpr int kUHX = kUX + 2, kUHY = kUY + 2, kUHZ = kUZ + 2;
-constexpr int kUPlane = kUHX * kUHY * kUHZ * 16;  // bytes of one 8-channel chunk of the halo
+// The tcgen05 kernel: a CTA owns a column of 16 (y) x 8 (z) voxels, an M = 128
+// tile per x plane (row m = 8 y + z), and marches over `planes` of them.  A
+// halo plane (18 x 10 voxels) is stored per 8-channel chunk as z columns of 10
+// rows of 16 B: the A operand of any (dy, dz) is then a descriptor into the
+// plane itself - rows of a core matrix are 8 consecutive z (16 B apart), the
+// 16 core matrices along M are the y columns (SBO = 160 B), the two along K the
+// chunks (LBO) - so no per-tap copy.  Halo plane h feeds the output planes
+// h - 2, h - 1 and h, whose accumulators are neighbours in TMEM: one MMA with
+// N = 3 COUT takes the three dx of a (dy, dz), as reading A (128 rows for every
+// MMA, 32 cycles) bounds the narrow layers.  An accumulator still takes its taps
+// in the order dx, dy, dz, the same bits as one MMA a tap.  Four planes are in
+// shared memory: two being loaded, two whose MMAs run; finished output planes
+// are written meanwhile.  The weights are loaded once a CTA.
+// 128^3 in us, against a CTA that loaded a 2-plane halo and all weights, issued
+// an MMA a tap and stored: 48 -> 16 channels 427 -> 231 (400 with the wide MMAs
+// alone), 16 -> 16 148 -> 98, 64^3 32 -> 32 82 -> 56; the network's inference
+// 1.23 -> 0.84 ms.
+constexpr int kUY = 16, kUZ = 8;
+constexpr int kUHY = kUY + 2, kUHZ = kUZ + 2;
+constexpr int kUChunk = kUHY * kUHZ * 16;  // bytes of one 8-channel chunk of a halo plane
+constexpr int kUSlots = 4;                 // halo planes in shared memory
 
 template <int CIN, int COUT>
 __host__ __device__ constexpr size_t fwd_umma_smem() {
-  return (size_t)(CIN / 8) * kUPlane + (size_t)27 * COUT * CIN * 2 + 1024;
+  return (size_t)kUSlots * (CIN / 8) * kUChunk + (size_t)27 * COUT * CIN * 2 + 1024;
+}
+
+// CTAs an SM holds (shared memory, and 4 by registers) and the output planes
+// that its share of the 512 TMEM columns holds.
+template <int CIN, int COUT>
+__host__ __device__ constexpr int umma_ctas() {
+  const size_t s = fwd_umma_smem<CIN, COUT>() + 1024;
+  return s * 4 <= 227 * 1024 && COUT <= 16 ? 4 : s * 2 <= 227 * 1024 ? 2 : 1;
+}
+template <int CIN, int COUT>
+__host__ __device__ constexpr int umma_planes() {
+  return 512 / umma_ctas<CIN, COUT>() / COUT;
 }
 
 // The pairs the tcgen05 kernel takes: cout a multiple of 16 (UMMA N), the
 // halo and all weights resident.
 template <int CIN, int COUT>
 __host__ __device__ constexpr bool umma_fits() {
-  return COUT % 16 == 0 && COUT <= 128 && fwd_umma_smem<CIN, COUT>() <= 200 * 1024;
+  return COUT % 16 == 0 && COUT <= 80 && fwd_umma_smem<CIN, COUT>() <= 200 * 1024;
 }
 
 template <int CIN, int COUT, bool RELU, bool BIAS>
 __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__ in, const bf16* __restrict__ w,
                                                        const float* __restrict__ bias, bf16* __restrict__ out,
-                                                       int sx, int sy, int sz) {
-  static_assert(umma_fits<CIN, COUT>(), "UMMA shapes: M = 128, N = COUT, operands resident");
+                                                       int sx, int sy, int sz, int planes) {
+  static_assert(umma_fits<CIN, COUT>(), "UMMA shapes: M = 128, N = COUT .. 3 COUT, operands resident");
   constexpr int CH = CIN / 8, KS = CIN / 16;
+  constexpr int SLOT = CH * kUChunk;
   constexpr int TAPB = COUT * CIN * 2;  // one tap's weights
-  constexpr int COLS = tmem_cols(2 * COUT);
-  constexpr uint32_t IDESC = umma_idesc(128, COUT);
+  constexpr int COLS = tmem_cols(umma_planes<CIN, COUT>() * COUT);
   extern __shared__ __align__(1024) unsigned char um_smem[];
-  unsigned char* sH = um_smem;                // [CH][kUHX][kUHY][kUHZ][16 B]
-  unsigned char* sB = um_smem + CH * kUPlane;  // [27][canonical COUT x CIN]
-  __shared__ __align__(8) uint64_t s_mbar;
+  unsigned char* sH = um_smem;                  // [kUSlots][CH][kUHY][kUHZ][16 B]
+  unsigned char* sB = um_smem + kUSlots * SLOT;  // [9 (dy, dz)][canonical 3 COUT x CIN]
+  __shared__ __align__(8) uint64_t s_mbar[kUSlots];
   __shared__ uint32_t s_tmem;
   const int tid = threadIdx.x, warp = tid >> 5;
-  const int z0 = blockIdx.x * kUZ, y0 = blockIdx.y * kUY, x0 = blockIdx.z * kUX;
+  const int z0 = blockIdx.x * kUZ, y0 = blockIdx.y * kUY, x0 = blockIdx.z * planes;
+  const int n = min(planes, sx - x0);  // output planes; halo planes 0 .. n + 1
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smem_u32(&s_tmem)),
                  "r"(COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&s_mbar)), "r"(1));
+    for (int i = 0; i < kUSlots; ++i)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(smem_u32(&s_mbar[i])), "r"(1));
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
-  // the halo: chunk c of voxel (hx, hy, hz), zero outside the grid
-  for (int i = tid; i < kUHX * kUHY * kUHZ * CH; i += 256) {
-    const int c = i % CH, h = i / CH;
-    const int hz = h % kUHZ, t = h / kUHZ, hy = t % kUHY, hx = t / kUHY;
-    const int gx = x0 + hx - 1, gy = y0 + hy - 1, gz = z0 + hz - 1;
-    const bool ok = gx >= 0 && gx < sx && gy >= 0 && gy < sy && gz >= 0 && gz < sz;
-    cp_async16(sH + c * kUPlane + h * 16, ok ? in + ((size_t)((gx * sy + gy) * sz + gz) * CIN + c * 8) : in, ok);
-  }
-  // all weights: tap t, row n, chunk c in the canonical K-major layout
+  // halo plane h, zero outside the grid, as one copy group (an empty one past the last)
+  auto load = [&](int h) {
+    if (h < n + 2) {
+      const int gx = x0 + h - 1;
+      unsigned char* const slot = sH + (h % kUSlots) * SLOT;
+      for (int i = tid; i < kUHY * kUHZ * CH; i += 256) {
+        const int c = i % CH, t = i / CH, gy = y0 + t / kUHZ - 1, gz = z0 + t % kUHZ - 1;
+        const bool ok = gx >= 0 && gx < sx && gy >= 0 && gy < sy && gz >= 0 && gz < sz;
+        cp_async16(slot + c * kUChunk + t * 16, ok ? in + ((size_t)((gx * sy + gy) * sz + gz) * CIN + c * 8) : in, ok);
+      }
+    }
+    cp_async_commit();
+  };
+  // all weights: of (dy, dz) the rows of dx = +1, 0, -1, in the canonical
+  // K-major layout (with plane 0's copy group)
   for (int i = tid; i < 27 * COUT * CH; i += 256) {
-    const int c = i % CH, n = (i / CH) % COUT, t = i / (CH * COUT);
-    cp_async16(sB + t * TAPB + (c >> 1) * (COUT * 32) + (n >> 3) * 256 + (c & 1) * 128 + (n & 7) * 16,
-               w + ((size_t)(t * COUT + n) * CIN + c * 8), true);
+    const int c = i % CH, r = (i / CH) % COUT, t = i / (CH * COUT);
+    const int row = (2 - t / 9) * COUT + r;
+    cp_async16(sB + (t % 9) * (3 * TAPB) + (c >> 1) * (3 * COUT * 32) + (row >> 3) * 256 + (c & 1) * 128 + (row & 7) * 16,
+               w + ((size_t)(t * COUT + r) * CIN + c * 8), true);
   }
-  cp_async_commit();
-  cp_async_wait<0>();
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  const uint32_t tmem = s_tmem;
-  if (tid == 0 && !g_umma_test_skip) {
-    const uint32_t h0 = smem_u32(sH), b0 = smem_u32(sB);
-    for (int tap = 0; tap < 27; ++tap) {
-      int dx, dy, dz;
-      tap_offset(tap, dx, dy, dz);
+  load(0);
+  load(1);
+  const uint32_t h0 = smem_u32(sH), b0 = smem_u32(sB);
+  // warp w reads TMEM lanes 32 (w % 4) .., channels 16 (w / 4) and on in steps
+  // of 32 (of every other plane where COUT is 16): row m -> (y, z)
+  const int m = (warp & 3) * 32 + (tid & 31);
+  const int gy = y0 + (m >> 3), gz = z0 + (m & 7);
+  uint32_t tmem = 0;
+  auto store_plane = [&](int q) {
+    const bool store = gy < sy && gz < sz;
+    const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(q * COUT);
+    bf16* dst = out + (size_t)(((x0 + q) * sy + gy) * sz + gz) * COUT;
+    if (COUT == 16 && (q & 1) != (warp >> 2)) return;
 #pragma unroll
-      for (int j = 0; j < kUX; ++j) {
-        // tile j: output x plane j reads halo plane j + dx + 1, columns from dy + 1, rows from dz + 1
-        const uint32_t a0 = h0 + (uint32_t)((((j + dx + 1) * kUHY + (dy + 1)) * kUHZ + (dz + 1)) * 16);
+    for (int cb = 0; cb < COUT; cb += 32) {
+      const int c0 = COUT == 16 ? 0 : cb + (warp >> 2) * 16;
+      if (c0 < COUT) {
+        float v[16];
+        tmem_ld16(trow + (uint32_t)c0, v);
+        if (store) {
+          __align__(16) __nv_bfloat162 pk[8];
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            float a = v[2 * q] + (BIAS ? bias[c0 + 2 * q] : 0.f), b = v[2 * q + 1] + (BIAS ? bias[c0 + 2 * q + 1] : 0.f);
+            if (RELU) {
+              a = fmaxf(a, 0.f);
+              b = fmaxf(b, 0.f);
+            }
+            pk[q] = __floats2bfloat162_rn(a, b);
+          }
+          uint4* d4 = reinterpret_cast<uint4*>(dst + c0);
+          d4[0] = reinterpret_cast<const uint4*>(pk)[0];
+          d4[1] = reinterpret_cast<const uint4*>(pk)[1];
+        }
+      }
+    }
+  };
+  // wait until the products of halo plane h are done (the last wait of a slot's
+  // barrier before its next use, so the parity tells them apart)
+  auto wait_plane = [&](int h) {
+    const bool ok = mbar_wait(&s_mbar[h % kUSlots], (uint32_t)((h / kUSlots) & 1));
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    return ok;
+  };
+  bool ok = true;
+  for (int h = 0; h < n + 2; ++h) {
+    // the slot of plane h - 2 is free once its products are done, which also
+    // completes output plane h - 4
+    if (h >= 2) ok = wait_plane(h - 2);
+    load(h + 2);
+    if (ok && h >= 4) store_plane(h - 4);
+    cp_async_wait<2>();
+    asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+    ok = __syncthreads_and(ok);
+    asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    if (!ok) break;  // a wait ran out (flagged); the same for every thread
+    tmem = s_tmem;
+    if (tid == 0 && !g_umma_test_skip) {
+      // halo plane h feeds the output planes lo .. hi, whose accumulators are
+      // neighbours; plane h itself for the first time
+      const int lo = max(h - 2, 0), hi = min(h, n - 1), old = h < n ? h - lo : hi - lo + 1;
+      const uint32_t idesc_all = umma_idesc(128, (hi - lo + 1) * COUT), idesc_old = umma_idesc(128, old * COUT);
+      const uint32_t d_lo = tmem + (uint32_t)(lo * COUT), b_lo = (uint32_t)((lo - h + 2) * (COUT * 32));
+      const uint32_t ah = h0 + (uint32_t)((h % kUSlots) * SLOT);
+#pragma unroll 1
+      for (int g = 0; g < 9; ++g) {
+        const uint32_t a0 = ah + (uint32_t)(((g / 3) * kUHZ + g % 3) * 16);
+        const uint32_t bg = b0 + (uint32_t)(g * (3 * TAPB));
 #pragma unroll
         for (int ks = 0; ks < KS; ++ks) {
-          const uint64_t ad = umma_desc(a0 + (uint32_t)(2 * ks * kUPlane), kUPlane, kUHZ * 16);
-          const uint64_t bd = umma_desc(b0 + (uint32_t)(tap * TAPB + ks * (COUT * 32)), 128, 256);
-          umma_f16(tmem + (uint32_t)(j * COUT), ad, bd, IDESC, (tap > 0 || ks > 0) ? 1u : 0u);
+          const uint64_t ad = umma_desc(a0 + (uint32_t)(2 * ks * kUChunk), kUChunk, kUHZ * 16);
+          const uint32_t bk = bg + (uint32_t)(ks * (3 * COUT * 32));
+          if (h < n && g == 0 && ks == 0) {
+            if (old > 0) umma_f16(d_lo, ad, umma_desc(bk + b_lo, 128, 256), idesc_old, 1u);
+            umma_f16(tmem + (uint32_t)(h * COUT), ad, umma_desc(bk + (uint32_t)(2 * COUT * 32), 128, 256),
+                     umma_idesc(128, COUT), 0u);
+          } else {
+            umma_f16(d_lo, ad, umma_desc(bk + b_lo, 128, 256), idesc_all, 1u);
+          }
         }
       }
-    }
-    umma_commit(&s_mbar);
-  }
-  const bool ok_wait = mbar_wait(&s_mbar, 0u);
-  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-  // warp w reads TMEM lanes 32 (w % 4) .. of tile w / 4: its row m -> (y, z)
-  const int j = warp >> 2, m = (warp & 3) * 32 + (tid & 31);
-  const int gx = x0 + j, gy = y0 + (m >> 3), gz = z0 + (m & 7);
-  const bool store = ok_wait && gx < sx && gy < sy && gz < sz;
-  const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(j * COUT);
-  bf16* dst = out + (size_t)((gx * sy + gy) * sz + gz) * COUT;
-#pragma unroll
-  for (int c0 = 0; c0 < COUT; c0 += 16) {
-    float v[16];
-    tmem_ld16(trow + (uint32_t)c0, v);
-    if (store) {
-      __align__(16) __nv_bfloat162 pk[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) {
-        float a = v[2 * q] + (BIAS ? bias[c0 + 2 * q] : 0.f), b = v[2 * q + 1] + (BIAS ? bias[c0 + 2 * q + 1] : 0.f);
-        if (RELU) {
-          a = fmaxf(a, 0.f);
-          b = fmaxf(b, 0.f);
-        }
-        pk[q] = __floats2bfloat162_rn(a, b);
-      }
-      uint4* d4 = reinterpret_cast<uint4*>(dst + c0);
-      d4[0] = reinterpret_cast<const uint4*>(pk)[0];
-      d4[1] = reinterpret_cast<const uint4*>(pk)[1];
+      umma_commit(&s_mbar[h % kUSlots]);
     }
   }
+  cp_async_wait<0>();
+  if (ok) ok = wait_plane(n);
+  if (ok && n >= 2) store_plane(n - 2);
+  if (ok) ok = wait_plane(n + 1);
+  if (ok) store_plane(n - 1);
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+    tmem = s_tmem;
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(COLS));
   }
 }
@@ -630,6 +696,14 @@ __global__ void k_flip_transpose(const bf16* __restrict__ w, bf16* __restrict__ 
   }
 }
 
+// Output planes of a CTA: as many as TMEM holds (a chunk of n loads n + 2), but
+// chunks enough to give every resident CTA one: a 64^3 layer of 32 columns
+// would otherwise leave half of the SMs idle.
+int umma_chunk_planes(int sx, int sy, int sz, int most, int ctas) {
+  const long long columns = (long long)((sz + kUZ - 1) / kUZ) * ((sy + kUY - 1) / kUY);
+  return (int)std::max(2LL, std::min((long long)most, columns * sx / (148LL * ctas)));
+}
+
 template <int CIN, int COUT, bool RELU, bool BIAS>
 cudaError_t fwd_launch(cudaStream_t st, const bf16* in, const bf16* w, const float* b, bf16* out, int sx, int sy,
                        int sz) {
@@ -639,8 +713,9 @@ cudaError_t fwd_launch(cudaStream_t st, const bf16* in, const bf16* w, const flo
       static const cudaError_t attr = cudaFuncSetAttribute(
           k_conv3_fwd_umma<CIN, COUT, RELU, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (attr != cudaSuccess) return attr;
-      const dim3 grid((sz + kUZ - 1) / kUZ, (sy + kUY - 1) / kUY, (sx + kUX - 1) / kUX);
-      k_conv3_fwd_umma<CIN, COUT, RELU, BIAS><<<grid, 256, smem, st>>>(in, w, b, out, sx, sy, sz);
+      const int planes = umma_chunk_planes(sx, sy, sz, umma_planes<CIN, COUT>(), umma_ctas<CIN, COUT>());
+      const dim3 grid((sz + kUZ - 1) / kUZ, (sy + kUY - 1) / kUY, (sx + planes - 1) / planes);
+      k_conv3_fwd_umma<CIN, COUT, RELU, BIAS><<<grid, 256, smem, st>>>(in, w, b, out, sx, sy, sz, planes);
       return cudaGetLastError();
     }
   }

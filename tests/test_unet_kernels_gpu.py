@@ -166,3 +166,38 @@ def test_umma_and_mma_sync_networks_agree():
     _no_umma_timeouts(lib)
     assert _rel(outs[1], outs[0]) < 1e-3
     net.close()
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (48, 16), (16, 32), (32, 32), (32, 64), (64, 32), (16, 48)])
+@pytest.mark.parametrize("shape", [(67, 40, 72), (71, 130, 82), (1, 200, 100)])
+def test_conv3_forward_chunks_of_planes(cin, cout, shape):
+    """Grids whose tcgen05 CTAs march over 3 to 16 planes, with a ragged last
+    chunk, and a single plane: one accumulator sums its taps in the order of
+    the one-plane launches, so a few planes cut out (with their neighbours)
+    give the same bits; and the whole is close to PyTorch's FP32 result (a BF16
+    rounding, 2^-9, of every output)."""
+    torch = _torch()
+    lib = _lib()
+    assert lib.aq_conv3_set_tiled(2) == 0
+    sx, sy, sz = shape
+    g = torch.Generator(device="cuda").manual_seed(cin * 100 + cout)
+    x = torch.randn(sx * sy * sz, cin, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(27, cout, cin, device="cuda", generator=g) / (27 * cin) ** 0.5).bfloat16()
+    b = torch.randn(cout, device="cuda", generator=g)
+
+    def run(xs, n):
+        y = torch.empty(n * sy * sz, cout, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        assert lib.aq_conv3_forward(cin, cout, 0, xs.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), n, sy, sz,
+                                    None) == 0
+        torch.cuda.synchronize()
+        return y.reshape(n, sy * sz, cout)
+
+    y = run(x, sx)
+    _no_umma_timeouts(lib)
+    want = torch.nn.functional.conv3d(_to_ncdhw(x, shape), _w_torch(w, cin, cout), b, padding=1)
+    assert _rel(_to_ncdhw(y, shape), want) <= 2.0 ** -9
+    plane = sy * sz
+    for q in [q for q in (1, 9, 16, 33, sx - 2) if 0 < q < sx - 1]:
+        cut = run(x[(q - 1) * plane:(q + 2) * plane].contiguous(), 3)
+        assert torch.equal(cut[1], y[q]), q
