@@ -332,6 +332,10 @@ cudaError_t launch_batch_solve_condition(cudaStream_t st, const int* live, int n
 // (cin, cout) must be one of the instantiated pairs (else cudaErrorInvalidValue).
 cudaError_t launch_conv3_fwd(cudaStream_t st, int cin, int cout, bool relu, const void* in, const void* w,
                              const float* bias, void* out, int sx, int sy, int sz);
+// The network's last 48 -> 16 layer, ReLU, on [coarse (32, half resolution), skip (16)];
+// cat is scratch for that concatenation, written only by the variants that need it.
+cudaError_t launch_upcat_conv3_fwd(cudaStream_t st, const void* coarse, const void* skip, void* cat, const void* w,
+                                   const float* bias, void* out, int sx, int sy, int sz);
 // dw[t][co][ci] (f32) from x (cin) and dy (cout); part: conv3_wgrad_part_floats scratch.
 cudaError_t launch_conv3_wgrad(cudaStream_t st, int cin, int cout, const void* x, const void* dy, float* part,
                                float* dw, int sx, int sy, int sz);

@@ -407,10 +407,13 @@ __host__ __device__ constexpr bool umma_fits() {
   return COUT % 16 == 0 && COUT <= 80 && fwd_umma_smem<CIN, COUT>() <= 200 * 1024;
 }
 
-template <int CIN, int COUT, bool RELU, bool BIAS>
-__global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__ in, const bf16* __restrict__ w,
-                                                       const float* __restrict__ bias, bf16* __restrict__ out,
-                                                       int sx, int sy, int sz, int planes) {
+// SKIP > 0: the input's last SKIP channels are read from `skip`, the others from
+// `in` at half the resolution (the concatenation that k_upcat writes, without
+// writing it: 128^3, 32 + 16 channels, 260 us against 67 + 231).
+template <int CIN, int COUT, bool RELU, bool BIAS, int SKIP = 0>
+__global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__ in, const bf16* __restrict__ skip,
+                                                       const bf16* __restrict__ w, const float* __restrict__ bias,
+                                                       bf16* __restrict__ out, int sx, int sy, int sz, int planes) {
   static_assert(umma_fits<CIN, COUT>(), "UMMA shapes: M = 128, N = COUT .. 3 COUT, operands resident");
   constexpr int CH = CIN / 8, KS = CIN / 16;
   constexpr int SLOT = CH * kUChunk;
@@ -442,7 +445,15 @@ __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__
       for (int i = tid; i < kUHY * kUHZ * CH; i += 256) {
         const int c = i % CH, t = i / CH, gy = y0 + t / kUHZ - 1, gz = z0 + t % kUHZ - 1;
         const bool ok = gx >= 0 && gx < sx && gy >= 0 && gy < sy && gz >= 0 && gz < sz;
-        cp_async16(slot + c * kUChunk + t * 16, ok ? in + ((size_t)((gx * sy + gy) * sz + gz) * CIN + c * 8) : in, ok);
+        const bf16* src = in;
+        if (ok) {
+          constexpr int CU = CIN - SKIP;
+          const size_t v = (size_t)(gx * sy + gy) * sz + gz;
+          if (SKIP == 0) src = in + v * CIN + c * 8;
+          else if (c * 8 < CU) src = in + ((size_t)((gx >> 1) * (sy >> 1) + (gy >> 1)) * (sz >> 1) + (gz >> 1)) * CU + c * 8;
+          else src = skip + v * SKIP + (c * 8 - CU);
+        }
+        cp_async16(slot + c * kUChunk + t * 16, src, ok);
       }
     }
     cp_async_commit();
@@ -704,20 +715,24 @@ int umma_chunk_planes(int sx, int sy, int sz, int most, int ctas) {
   return (int)std::max(2LL, std::min((long long)most, columns * sx / (148LL * ctas)));
 }
 
+template <int CIN, int COUT, bool RELU, bool BIAS, int SKIP>
+cudaError_t umma_launch(cudaStream_t st, const bf16* in, const bf16* skip, const bf16* w, const float* b, bf16* out,
+                        int sx, int sy, int sz) {
+  constexpr size_t smem = fwd_umma_smem<CIN, COUT>();
+  static const cudaError_t attr = cudaFuncSetAttribute(k_conv3_fwd_umma<CIN, COUT, RELU, BIAS, SKIP>,
+                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (attr != cudaSuccess) return attr;
+  const int planes = umma_chunk_planes(sx, sy, sz, umma_planes<CIN, COUT>(), umma_ctas<CIN, COUT>());
+  const dim3 grid((sz + kUZ - 1) / kUZ, (sy + kUY - 1) / kUY, (sx + planes - 1) / planes);
+  k_conv3_fwd_umma<CIN, COUT, RELU, BIAS, SKIP><<<grid, 256, smem, st>>>(in, skip, w, b, out, sx, sy, sz, planes);
+  return cudaGetLastError();
+}
+
 template <int CIN, int COUT, bool RELU, bool BIAS>
 cudaError_t fwd_launch(cudaStream_t st, const bf16* in, const bf16* w, const float* b, bf16* out, int sx, int sy,
                        int sz) {
   if constexpr (umma_fits<CIN, COUT>()) {
-    if (g_conv_impl == 2) {
-      constexpr size_t smem = fwd_umma_smem<CIN, COUT>();
-      static const cudaError_t attr = cudaFuncSetAttribute(
-          k_conv3_fwd_umma<CIN, COUT, RELU, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (attr != cudaSuccess) return attr;
-      const int planes = umma_chunk_planes(sx, sy, sz, umma_planes<CIN, COUT>(), umma_ctas<CIN, COUT>());
-      const dim3 grid((sz + kUZ - 1) / kUZ, (sy + kUY - 1) / kUY, (sx + planes - 1) / planes);
-      k_conv3_fwd_umma<CIN, COUT, RELU, BIAS><<<grid, 256, smem, st>>>(in, w, b, out, sx, sy, sz, planes);
-      return cudaGetLastError();
-    }
+    if (g_conv_impl == 2) return umma_launch<CIN, COUT, RELU, BIAS, 0>(st, in, nullptr, w, b, out, sx, sy, sz);
   }
   if (g_conv_impl >= 1) {
     constexpr size_t smem = fwd_tile_smem<CIN, COUT>();
@@ -1225,6 +1240,16 @@ cudaError_t launch_conv3_fwd(cudaStream_t st, int cin, int cout, bool relu, cons
   AQ_CONV_PAIRS(X)
 #undef X
   return cudaErrorInvalidValue;
+}
+
+// The tcgen05 convolution reads the concatenation's parts itself.
+cudaError_t launch_upcat_conv3_fwd(cudaStream_t st, const void* coarse, const void* skip, void* cat, const void* w,
+                                   const float* bias, void* out, int sx, int sy, int sz) {
+  if (g_conv_impl == 2)
+    return umma_launch<48, 16, true, true, 16>(st, (const bf16*)coarse, (const bf16*)skip, (const bf16*)w, bias,
+                                               (bf16*)out, sx, sy, sz);
+  const cudaError_t e = launch_upcat(st, coarse, skip, cat, sx, sy, sz, 32, 16);
+  return e != cudaSuccess ? e : launch_conv3_fwd(st, 48, 16, true, cat, w, bias, out, sx, sy, sz);
 }
 
 cudaError_t launch_conv3_wgrad(cudaStream_t st, int cin, int cout, const void* x, const void* dy, float* part,

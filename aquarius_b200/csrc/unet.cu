@@ -160,8 +160,12 @@ aq_status forward(aq_unet* net, cudaStream_t st, UActs* a) {
   UN_CUDA(launch_upcat(st, a->b2, a->e2, a->u2, hx, hy, hz, 64, 32));
   UN_TRY(conv(net, st, 6, a->u2, a->d2a, hx, hy, hz));
   UN_TRY(conv(net, st, 7, a->d2a, a->d2, hx, hy, hz));
-  UN_CUDA(launch_upcat(st, a->d2, a->e1, a->u1, sx, sy, sz, 32, 16));
-  UN_TRY(conv(net, st, 8, a->u1, a->d1a, sx, sy, sz));
+  if (a->grads) {  // training: the weight gradient reads u1
+    UN_CUDA(launch_upcat(st, a->d2, a->e1, a->u1, sx, sy, sz, 32, 16));
+    UN_TRY(conv(net, st, 8, a->u1, a->d1a, sx, sy, sz));
+  } else {
+    UN_CUDA(launch_upcat_conv3_fwd(st, a->d2, a->e1, a->u1, net->L[8].wb, net->L[8].b, a->d1a, sx, sy, sz));
+  }
   UN_TRY(conv(net, st, 9, a->d1a, a->d1, sx, sy, sz));
   UN_CUDA(launch_head_fwd(st, a->d1, net->hp, net->hp + 16, a->out, sx * sy * sz));
   return AQ_OK;

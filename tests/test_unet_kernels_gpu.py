@@ -201,3 +201,29 @@ def test_conv3_forward_chunks_of_planes(cin, cout, shape):
     for q in [q for q in (1, 9, 16, 33, sx - 2) if 0 < q < sx - 1]:
         cut = run(x[(q - 1) * plane:(q + 2) * plane].contiguous(), 3)
         assert torch.equal(cut[1], y[q]), q
+
+
+@pytest.mark.parametrize("size", [(36, 20, 44), (100, 48, 72)])
+def test_umma_and_mma_sync_networks_agree_on_ragged_grids(size):
+    """The inference's last concatenation is read by its convolution without
+    being written; the mma.sync variant writes it (the same
+    products, f32 sums in the tensor core's order)."""
+    torch = _torch()
+    lib = _lib()
+    import pathlib
+    net = aq.UNet(weights=pathlib.Path(aq.__file__).resolve().parent / "weights" / "unet_64.bin")
+    V = size[0] * size[1] * size[2]
+    g = torch.Generator(device="cuda").manual_seed(11)
+    typ = (torch.rand(V, device="cuda", generator=g) < 0.5).to(torch.int8)
+    rhs = torch.randn(V, device="cuda", generator=g)
+    outs = []
+    for impl in (1, 2):
+        lib.aq_conv3_set_tiled(impl)
+        o = torch.zeros(V, device="cuda")
+        net.predict(size, rhs.data_ptr(), typ.data_ptr(), o.data_ptr())
+        torch.cuda.synchronize()
+        outs.append(o)
+    lib.aq_conv3_set_tiled(2)
+    _no_umma_timeouts(lib)
+    assert _rel(outs[1], outs[0]) < 1e-3
+    net.close()
