@@ -156,6 +156,8 @@ def jacobi_kernel_name_of(plan) -> str:
         return f"k_jacobi_flat<{xplanes}> (1 sweep/launch, float4 z-quads)"
     if rows == 3:
         return "k_jacobi_list (1 sweep/launch over the listed active warp rows, one resident wave)"
+    if rows == 5:
+        return f"k_cluster_solve<{xplanes} CTAs> (whole solve in one thread-block cluster)"
     if rows == 4:
         shapes = ["8x40x24", "16x24x24", "8x32x24", "16x16x24", "8x16x24", "24x16x24", "8x48x24"]
         return (f"k_resident_solve<tiles {shapes[xplanes]}, halo {levels}> (whole solve in one cooperative launch, "
@@ -765,7 +767,9 @@ def run_batch(args, rank: int, world: int, dist):
     s1 = [b.solve_stats(i) for i in range(b.scene_count)]
     # the solve loop runs until its slowest scene stops: loop blocks = max over scenes
     loop_blocks = max(x["total_blocks"] - y["total_blocks"] for x, y in zip(s1, s0))
-    launches = args.steps * per_step + loop_blocks * per_block
+    # the step's launches outside the solve loop: a lower bound, as the loop's own
+    # depend on whether the scenes are solved by rows or in clusters
+    launches = args.steps * per_step
     value = weak_scaling_value(args.steps, world, ms_max)
     sweeps = [x["total_sweeps"] - y["total_sweeps"] for x, y in zip(s1, s0)]
     conv = sum(1 for x in s1 if x["converged"])
