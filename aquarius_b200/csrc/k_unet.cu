@@ -376,8 +376,8 @@ __host__ __device__ constexpr int tmem_cols(int n) {
 // are written meanwhile.  The weights are loaded once a CTA.
 // 128^3 in us, against a CTA that loaded a 2-plane halo and all weights, issued
 // an MMA a tap and stored: 48 -> 16 channels 427 -> 231 (400 with the wide MMAs
-// alone), 16 -> 16 148 -> 98, 64^3 32 -> 32 82 -> 56; the network's inference
-// 1.23 -> 0.84 ms.
+// alone), 16 -> 16 148 -> 98, 64^3 32 -> 32 82 -> 41; the network's inference
+// 1.23 -> 0.80 ms.
 constexpr int kUY = 16, kUZ = 8;
 constexpr int kUHY = kUY + 2, kUHZ = kUZ + 2;
 constexpr int kUChunk = kUHY * kUHZ * 16;  // bytes of one 8-channel chunk of a halo plane
@@ -409,7 +409,7 @@ __host__ __device__ constexpr bool umma_fits() {
 
 // SKIP > 0: the input's last SKIP channels are read from `skip`, the others from
 // `in` at half the resolution (the concatenation that k_upcat writes, without
-// writing it: 128^3, 32 + 16 channels, 260 us against 67 + 231).
+// writing it: 128^3, 32 + 16 channels, 245 us against 67 + 231).
 template <int CIN, int COUT, bool RELU, bool BIAS, int SKIP = 0>
 __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__ in, const bf16* __restrict__ skip,
                                                        const bf16* __restrict__ w, const float* __restrict__ bias,
@@ -707,12 +707,24 @@ __global__ void k_flip_transpose(const bf16* __restrict__ w, bf16* __restrict__ 
   }
 }
 
-// Output planes of a CTA: as many as TMEM holds (a chunk of n loads n + 2), but
-// chunks enough to give every resident CTA one: a 64^3 layer of 32 columns
-// would otherwise leave half of the SMs idle.
+// Output planes of a CTA, at most as many as TMEM holds: the number whose waves
+// of resident CTAs take the fewest plane steps (a chunk of n planes loads
+// n + 2 and starts and ends in about one more).  A 64^3 layer of 32 columns in
+// chunks of 8 fills one wave of 296; in chunks of 6, as many as give every
+// resident CTA one, a second wave of 56 CTAs followed (16 -> 32 channels 41 us
+// against 29, 32 -> 32 55 against 41).
 int umma_chunk_planes(int sx, int sy, int sz, int most, int ctas) {
-  const long long columns = (long long)((sz + kUZ - 1) / kUZ) * ((sy + kUY - 1) / kUY);
-  return (int)std::max(2LL, std::min((long long)most, columns * sx / (148LL * ctas)));
+  const long long columns = (long long)((sz + kUZ - 1) / kUZ) * ((sy + kUY - 1) / kUY), resident = 148LL * ctas;
+  int best = 2;
+  long long least = 0;
+  for (int p = 2; p <= most; ++p) {
+    const long long waves = (columns * ((sx + p - 1) / p) + resident - 1) / resident, cost = waves * (p + 3);
+    if (p == 2 || cost < least) {
+      best = p;
+      least = cost;
+    }
+  }
+  return best;
 }
 
 template <int CIN, int COUT, bool RELU, bool BIAS, int SKIP>
