@@ -330,8 +330,9 @@ __global__ void __launch_bounds__(256, 6) k_jacobi_list(Dims d, const float* __r
   int it = blockIdx.x * W + threadIdx.y;
   int n = 0;
   // early (every sweep of a block but the first): the list, rhs and types
-  // were written before the previous sweep was launched, so the warp's first
-  // row is decoded and its rhs and types loaded before waiting for that sweep
+  // were complete before this sweep could be launched (see the trigger below),
+  // so the warp's first row is decoded and its rhs and types loaded before
+  // waiting for the previous sweep
   bool pre = false;
   int x0 = 0, y0 = 0, zb0 = 0;
   float4 b0 = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -353,11 +354,16 @@ __global__ void __launch_bounds__(256, 6) k_jacobi_list(Dims d, const float* __r
       pre = true;
     }
   }
-  // the next sweep may start its own early part now; it waits for this one
-  // where it reads the iterate
+  // A block's first sweep follows the kernel that writes the list: it lets the
+  // next one start only after its own wait, so that no early part runs before
+  // the list is there.  From then on the next sweep may start its early part
+  // at once; it waits for this one where it reads the iterate.
+  if (!early) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    n = *n_items;
+  }
   asm volatile("griddepcontrol.launch_dependents;");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (!early) n = *n_items;
+  if (early) asm volatile("griddepcontrol.wait;" ::: "memory");
   if (pre) {
     jacobi_row_pre(d, pin, pout, x0, y0, zb0, b0, t0);
     it += gridDim.x * W;

@@ -1,0 +1,43 @@
+"""Orders that the kernels' sources have to keep and that no run shows reliably:
+each rule is read off the text of the kernels it is about."""
+import pathlib
+import re
+
+import pytest
+
+CSRC = pathlib.Path(__file__).resolve().parent.parent / "aquarius_b200" / "csrc"
+SOURCES = {p.name: p.read_text() for p in sorted(CSRC.glob("*.cu*"))}
+
+
+def _code(text):
+    return re.sub(r"//[^\n]*", "", text)
+
+
+def _kernels(text):
+    """(name, body) of every __global__ function definition."""
+    out = []
+    for m in re.finditer(r"__global__\s+void[^;{]*?\b(k\w+)\s*\(", text):
+        at = text.index(")", m.end())
+        brace, semi = text.find("{", at), text.find(";", at)
+        if brace < 0 or 0 <= semi < brace:
+            continue  # a declaration
+        depth, i = 0, brace
+        while True:
+            depth += (text[i] == "{") - (text[i] == "}")
+            i += 1
+            if depth == 0:
+                break
+        out.append((m.group(1), text[brace:i]))
+    return out
+
+
+KERNELS = {f"{f}:{name}": body for f, text in SOURCES.items() for name, body in _kernels(_code(text))}
+
+
+@pytest.mark.parametrize("kernel", [k for k, b in KERNELS.items() if "griddepcontrol.launch_dependents" in b])
+def test_a_first_launch_waits_before_it_triggers(kernel):
+    """A kernel that triggers its dependents has a path, ahead of the trigger,
+    that has waited for its own predecessor: the first launch of a chain takes
+    it, so what later launches read early was complete before they started."""
+    body = KERNELS[kernel]
+    assert 0 <= body.find("griddepcontrol.wait") < body.find("griddepcontrol.launch_dependents")
