@@ -572,7 +572,7 @@ __device__ __noinline__ void solve_global(const ClusterScene& S, const SolveArgs
       [&](int todo) {
         for (int k = 0; k < todo; ++k) {
           for (int i = begin + tid; i < v.n; i += stride) {
-            const UnitPos p = unit_pos(d, nq, __ldg(S.list + i));
+            const UnitPos p = unit_pos(d, nq, __ldcg(S.list + i));
             const unsigned f = unit_fluid(d, S.type, p, vec);
             UnitIn u = gload_unit(d, bufs[cur], p);
             const Quad r0 = load_cells(S.rhs, p.cell, p.len);
@@ -589,7 +589,7 @@ __device__ __noinline__ void solve_global(const ClusterScene& S, const SolveArgs
         for (int i0 = begin + warp * 32; i0 < v.n; i0 += stride) {
           double acc = 0.0;
           if (i0 + lane < v.n) {
-            const UnitPos p = unit_pos(d, nq, __ldg(S.list + i0 + lane));
+            const UnitPos p = unit_pos(d, nq, __ldcg(S.list + i0 + lane));
             const Quad r0 = load_cells(S.rhs, p.cell, p.len);
             acc = resid_unit(gload_unit(d, bufs[cur], p), r0,
                              p.two ? load_cells(S.rhs, p.cell + plane, p.len) : r0, unit_fluid(d, S.type, p, vec));
@@ -600,7 +600,7 @@ __device__ __noinline__ void solve_global(const ClusterScene& S, const SolveArgs
       });
   if (cur) {
     for (int i = begin + tid; i < v.n; i += stride) {
-      const UnitPos p = unit_pos(d, nq, __ldg(S.list + i));
+      const UnitPos p = unit_pos(d, nq, __ldcg(S.list + i));
       store_cells(S.pa, p.cell, p.len, load_cells(S.pb, p.cell, p.len));
       if (p.two) store_cells(S.pa, p.cell + plane, p.len, load_cells(S.pb, p.cell + plane, p.len));
     }

@@ -41,3 +41,12 @@ def test_a_first_launch_waits_before_it_triggers(kernel):
     it, so what later launches read early was complete before they started."""
     body = KERNELS[kernel]
     assert 0 <= body.find("griddepcontrol.wait") < body.find("griddepcontrol.launch_dependents")
+
+
+@pytest.mark.parametrize("array", ["umap", "list", "part", "pa", "pb"])
+def test_cluster_solve_reads_what_it_writes_through_l2(array):
+    """The cluster solve's CTAs exchange these arrays within one launch: the
+    read-only path (__ldg) is for data that stays constant for a kernel's life."""
+    code = _code(SOURCES["k_cluster.cu"])
+    assert re.search(rf"\bS\.{array}\b", code)
+    assert not re.search(rf"__ldg\(\s*S\.{array}\b", code)
