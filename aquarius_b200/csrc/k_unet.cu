@@ -504,9 +504,10 @@ __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__
     }
   };
   // wait until the products of halo plane h are done (the last wait of a slot's
-  // barrier before its next use, so the parity tells them apart)
+  // barrier before its next use, so the parity tells them apart).  The warp's
+  // lanes decide together: what follows reads TMEM, which takes whole warps.
   auto wait_plane = [&](int h) {
-    const bool ok = mbar_wait(&s_mbar[h % kUSlots], (uint32_t)((h / kUSlots) & 1));
+    const bool ok = __all_sync(0xffffffffu, mbar_wait(&s_mbar[h % kUSlots], (uint32_t)((h / kUSlots) & 1)));
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     return ok;
   };

@@ -50,3 +50,11 @@ def test_cluster_solve_reads_what_it_writes_through_l2(array):
     code = _code(SOURCES["k_cluster.cu"])
     assert re.search(rf"\bS\.{array}\b", code)
     assert not re.search(rf"__ldg\(\s*S\.{array}\b", code)
+
+
+@pytest.mark.parametrize("kernel", [k for k, b in KERNELS.items() if "mbar_wait(" in b])
+def test_bounded_waits_are_decided_by_whole_warps(kernel):
+    """A wait that may run out for some lanes alone must not steer a warp around
+    tcgen05.ld, which all of its lanes execute together."""
+    body = KERNELS[kernel]
+    assert "mbar_wait(" not in re.sub(r"__all_sync\(0xffffffffu, mbar_wait\(", "", body)
