@@ -357,6 +357,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 16 columns of this thread's TMEM lane set to 0 (tcgen05.wait::st follows).
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(taddr),
+      "r"(0u)
+      : "memory");
+}
+
 __host__ __device__ constexpr int tmem_cols(int n) {
   return n <= 32 ? 32 : n <= 64 ? 64 : n <= 128 ? 128 : n <= 256 ? 256 : 512;
 }
@@ -371,9 +379,13 @@ __host__ __device__ constexpr int tmem_cols(int n) {
 // h - 2, h - 1 and h, whose accumulators are neighbours in TMEM: one MMA with
 // N = 3 COUT takes the three dx of a (dy, dz), as reading A (128 rows for every
 // MMA, 32 cycles) bounds the narrow layers.  An accumulator still takes its taps
-// in the order dx, dy, dz, the same bits as one MMA a tap.  Four planes are in
-// shared memory: two being loaded, two whose MMAs run; finished output planes
-// are written meanwhile.  The weights are loaded once a CTA.
+// in the order dx, dy, dz, the same bits as one MMA a tap.  MMAs are ordered
+// among themselves only where they share accumulator and shape, so the
+// accumulators are cleared first (every MMA of a halo plane then has that
+// plane's window of columns and its N), and a plane's MMAs are issued when the
+// plane before, whose window overlaps, has completed.  Four planes are in
+// shared memory: two being loaded, one whose MMAs run, one that waits; finished
+// output planes are written meanwhile.  The weights are loaded once a CTA.
 // 128^3 in us, against a CTA that loaded a 2-plane halo and all weights, issued
 // an MMA a tap and stored: 48 -> 16 channels 427 -> 231 (400 with the wide MMAs
 // alone), 16 -> 16 148 -> 98, 64^3 32 -> 32 82 -> 41; the network's inference
@@ -473,7 +485,14 @@ __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__
   // of 32 (of every other plane where COUT is 16): row m -> (y, z)
   const int m = (warp & 3) * 32 + (tid & 31);
   const int gy = y0 + (m >> 3), gz = z0 + (m & 7);
-  uint32_t tmem = 0;
+  // the accumulators start at zero, so that every MMA adds
+  asm volatile("tcgen05.fence::before_thread_sync;\n" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
+  const uint32_t tmem = s_tmem;
+  for (int c0 = (warp >> 2) * 16; c0 < n * COUT; c0 += 32)
+    tmem_zero16(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0);
+  asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
   auto store_plane = [&](int q) {
     const bool store = gy < sy && gz < sz;
     const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(q * COUT);
@@ -524,30 +543,22 @@ __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__
     ok = __syncthreads_and(ok);
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
     if (!ok) break;  // a wait ran out (flagged); the same for every thread
-    tmem = s_tmem;
-    if (tid == 0 && !g_umma_test_skip) {
-      // halo plane h feeds the output planes lo .. hi, whose accumulators are
-      // neighbours; plane h itself for the first time
-      const int lo = max(h - 2, 0), hi = min(h, n - 1), old = h < n ? h - lo : hi - lo + 1;
-      const uint32_t idesc_all = umma_idesc(128, (hi - lo + 1) * COUT), idesc_old = umma_idesc(128, old * COUT);
-      const uint32_t d_lo = tmem + (uint32_t)(lo * COUT), b_lo = (uint32_t)((lo - h + 2) * (COUT * 32));
+    // the products of plane h - 1 first: the accumulators' window moves on
+    const bool go = warp == 0 && (h == 0 || wait_plane(h - 1));
+    if (tid == 0 && go && !g_umma_test_skip) {
+      // halo plane h feeds the output planes lo .. hi, whose accumulators are neighbours
+      const int lo = max(h - 2, 0), hi = min(h, n - 1);
+      const uint32_t idesc = umma_idesc(128, (hi - lo + 1) * COUT);
+      const uint32_t d_lo = tmem + (uint32_t)(lo * COUT), b_lo = b0 + (uint32_t)((lo - h + 2) * (COUT * 32));
       const uint32_t ah = h0 + (uint32_t)((h % kUSlots) * SLOT);
 #pragma unroll 1
       for (int g = 0; g < 9; ++g) {
         const uint32_t a0 = ah + (uint32_t)(((g / 3) * kUHZ + g % 3) * 16);
-        const uint32_t bg = b0 + (uint32_t)(g * (3 * TAPB));
+        const uint32_t bg = b_lo + (uint32_t)(g * (3 * TAPB));
 #pragma unroll
-        for (int ks = 0; ks < KS; ++ks) {
-          const uint64_t ad = umma_desc(a0 + (uint32_t)(2 * ks * kUChunk), kUChunk, kUHZ * 16);
-          const uint32_t bk = bg + (uint32_t)(ks * (3 * COUT * 32));
-          if (h < n && g == 0 && ks == 0) {
-            if (old > 0) umma_f16(d_lo, ad, umma_desc(bk + b_lo, 128, 256), idesc_old, 1u);
-            umma_f16(tmem + (uint32_t)(h * COUT), ad, umma_desc(bk + (uint32_t)(2 * COUT * 32), 128, 256),
-                     umma_idesc(128, COUT), 0u);
-          } else {
-            umma_f16(d_lo, ad, umma_desc(bk + b_lo, 128, 256), idesc_all, 1u);
-          }
-        }
+        for (int ks = 0; ks < KS; ++ks)
+          umma_f16(d_lo, umma_desc(a0 + (uint32_t)(2 * ks * kUChunk), kUChunk, kUHZ * 16),
+                   umma_desc(bg + (uint32_t)(ks * (3 * COUT * 32)), 128, 256), idesc, 1u);
       }
       umma_commit(&s_mbar[h % kUSlots]);
     }
@@ -561,7 +572,6 @@ __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__
   __syncthreads();
   if (warp == 0) {
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::: "memory");
-    tmem = s_tmem;
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(COLS));
   }
 }

@@ -58,3 +58,13 @@ def test_bounded_waits_are_decided_by_whole_warps(kernel):
     tcgen05.ld, which all of its lanes execute together."""
     body = KERNELS[kernel]
     assert "mbar_wait(" not in re.sub(r"__all_sync\(0xffffffffu, mbar_wait\(", "", body)
+
+
+def test_dependent_mmas_share_accumulator_and_shape():
+    """tcgen05.mma instructions are ordered among themselves only with the same
+    accumulator and shape.  The convolution issues one form of it per halo
+    plane, and a plane's after those of the plane before have completed."""
+    body = KERNELS["k_unet.cu:k_conv3_fwd_umma"]
+    assert body.count("umma_f16(") == 1
+    issue = body.index("umma_f16(")
+    assert body.rfind("wait_plane(h - 1)", 0, issue) > body.rfind("__syncthreads_and", 0, issue) > 0

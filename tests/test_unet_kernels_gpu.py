@@ -227,3 +227,27 @@ def test_umma_and_mma_sync_networks_agree_on_ragged_grids(size):
     _no_umma_timeouts(lib)
     assert _rel(outs[1], outs[0]) < 1e-3
     net.close()
+
+
+@pytest.mark.parametrize("cin,cout", [(16, 16), (48, 16), (16, 32), (32, 32), (32, 64), (64, 32), (16, 48)])
+def test_conv3_forward_repeats_bit_for_bit(cin, cout):
+    """Accumulators are summed by MMAs whose windows overlap from plane to plane:
+    many launches, many CTAs to an SM, always the same bits."""
+    torch = _torch()
+    lib = _lib()
+    assert lib.aq_conv3_set_tiled(2) == 0
+    sx, sy, sz = shape = (65, 96, 80)
+    g = torch.Generator(device="cuda").manual_seed(cin + cout)
+    x = torch.randn(sx * sy * sz, cin, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(27, cout, cin, device="cuda", generator=g) / (27 * cin) ** 0.5).bfloat16()
+    b = torch.randn(cout, device="cuda", generator=g)
+    ys = [torch.empty(sx * sy * sz, cout, device="cuda", dtype=torch.bfloat16) for _ in range(30)]
+    torch.cuda.synchronize()
+    for y in ys:
+        assert lib.aq_conv3_forward(cin, cout, 0, x.data_ptr(), w.data_ptr(), b.data_ptr(), y.data_ptr(), *shape,
+                                    None) == 0
+    torch.cuda.synchronize()
+    _no_umma_timeouts(lib)
+    want = torch.nn.functional.conv3d(_to_ncdhw(x, shape), _w_torch(w, cin, cout), b, padding=1)
+    assert _rel(_to_ncdhw(ys[0], shape), want) <= 2.0 ** -9
+    assert all(torch.equal(y, ys[0]) for y in ys[1:])
