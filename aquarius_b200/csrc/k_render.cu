@@ -613,12 +613,13 @@ __global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const fl
                                                        unsigned long long* __restrict__ mixed) {
   __shared__ unsigned s_cnt[2][kSplatBox];  // phases 0, 1 and 2, 3 in 16-bit halves
   __shared__ int s_box[4];
-  if (__ldcg(mixed)) return;
   const int tid = threadIdx.x, i = blockIdx.x * kSplat + tid;
   if (tid == 0) {
     s_box[0] = s_box[2] = INT_MAX;
     s_box[1] = s_box[3] = -1;
   }
+  // another CTA may set the flag at any time: one thread's look decides for all
+  if (__syncthreads_or(tid == 0 && __ldcg(mixed) != 0)) return;
   float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
   int i0 = 0, i1 = -1, j0 = 0, j1 = -1;
   unsigned add01 = 0, add23 = 0;

@@ -68,3 +68,12 @@ def test_dependent_mmas_share_accumulator_and_shape():
     assert body.count("umma_f16(") == 1
     issue = body.index("umma_f16(")
     assert body.rfind("wait_plane(h - 1)", 0, issue) > body.rfind("__syncthreads_and", 0, issue) > 0
+
+
+def test_splat_leaves_by_a_vote():
+    """Other CTAs set the flag that ends the counting: its value may differ from
+    thread to thread, so the CTA leaves on one thread's reading, together."""
+    body = KERNELS["k_render.cu:k_phase_splat"]
+    assert "return" not in body[:body.index("__syncthreads")]
+    for m in re.finditer(r"__ldcg\(mixed\)", body):
+        assert re.search(r"__syncthreads_or\(tid == 0 && $", body[:m.start()])
