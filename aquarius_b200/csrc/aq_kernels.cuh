@@ -4,12 +4,34 @@
 
 #include <cuda_bf16.h>
 
+#include <atomic>
+#include <cstdint>
 #include <string>
 
 #include "../../include/aquarius_b200.h"
 #include "aq_common.cuh"
 
 namespace aqb {
+
+// A kernel's attributes (shared memory, cluster size) hold on one device: runs
+// `set` on the first use of each device, on every use beyond 64 of them.
+class PerDevice {
+ public:
+  template <class F>
+  cudaError_t operator()(F&& set) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const uint64_t bit = dev < 64 ? uint64_t{1} << dev : 0;
+    if (done_.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    e = set();
+    if (e == cudaSuccess) done_.fetch_or(bit, std::memory_order_release);
+    return e;
+  }
+
+ private:
+  std::atomic<uint64_t> done_{0};
+};
 
 // Records the message aq_last_error() returns on this thread; returns st.
 aq_status set_last_error(aq_status st, const std::string& msg);
@@ -186,6 +208,7 @@ long long cluster_solve_units(const Dims& d);  // units of 2 x 1 x 4 cells: entr
 int cluster_solve_width(const Dims& d);   // CTAs of the default plan
 bool cluster_solve_takes(const Dims& d, int width);               // the launch's limits
 bool cluster_solve_fits(const Dims& d, long long particles);      // the default plan's rule
+bool cluster_solve_runs(int width);  // the current device holds such a cluster, alone and in a batch
 // fixed_sweeps > 0: that many sweeps then one residual; else residual mode.
 // part: one double per 32 units.  Starts from pa, result in pa.  r2_only (may
 // be null): the squared residual goes there and *ss is only read.

@@ -231,6 +231,8 @@ aq_status aq_batch::plan_clusters() {
     units += u;
     parts += u / 32 + 1;
   }
+  for (int k = 0; k < kWidths; ++k)
+    if (!by[k].empty() && !cluster_solve_runs(1 << k)) return AQ_OK;
   std::vector<int> order;
   for (int k = 0; k < kWidths; ++k) {
     std::stable_sort(by[k].begin(), by[k].end(), [&](int a, int b) { return scenes[a].n > scenes[b].n; });

@@ -306,7 +306,7 @@ aq_status aq_fluid::allocate() {
   }
   memset(ss_host, 0, sizeof(SolveState));
   // small grids: the whole solve in one thread-block cluster
-  if (cluster_solve_fits(d, n)) {
+  if (cluster_solve_fits(d, n) && cluster_solve_runs(cluster_solve_width(d))) {
     AQ_TRY(alloc_cluster());
     plan = JacobiPlan{1, 5, cluster_solve_width(d)};
   }

@@ -741,6 +741,14 @@ cudaError_t allow_cluster(K kernel) {
   const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   return e != cudaSuccess ? e : cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 }
+cudaError_t allow_solve() {
+  static PerDevice once;
+  return once([] { return allow_cluster(k_cluster_solve); });
+}
+cudaError_t allow_batch_solve() {
+  static PerDevice once;
+  return once([] { return allow_cluster(kb_cluster_solve); });
+}
 
 }  // namespace
 
@@ -765,11 +773,21 @@ bool cluster_solve_fits(const Dims& d, long long particles) {
   return particles / 64 <= (long long)w * kCap * 7 / 10;
 }
 
+bool cluster_solve_runs(int width) {
+  ClusterLaunch l(nullptr, 1, width);
+  int alone = 0, batch = 0;
+  cudaError_t e = allow_solve();
+  if (e == cudaSuccess) e = allow_batch_solve();
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&alone, k_cluster_solve, &l.lc);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&batch, kb_cluster_solve, &l.lc);
+  if (e != cudaSuccess) cudaGetLastError();
+  return e == cudaSuccess && alone > 0 && batch > 0;
+}
+
 cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, float* pb, const float* rhs,
                                  const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
                                  int fixed_sweeps, int check, int max_iters, double tol, double* r2_only) {
-  static const cudaError_t prep = allow_cluster(k_cluster_solve);
-  if (prep != cudaSuccess) return prep;
+  if (const cudaError_t e = allow_solve()) return e;
   ClusterLaunch l(st, 1, width);
   const ClusterScene S{d, pa, pb, rhs, type, umap, list, part, ss};
   return cudaLaunchKernelEx(&l.lc, k_cluster_solve, S, SolveArgs{fixed_sweeps, check, max_iters, tol, r2_only});
@@ -791,8 +809,7 @@ cudaError_t launch_batch_cluster_solve(cudaStream_t st, const BatchIndex& bi, in
                                        const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
                                        int fixed_sweeps, int check, int max_iters, double tol) {
   if (scenes <= 0) return cudaSuccess;
-  static const cudaError_t prep = allow_cluster(kb_cluster_solve);
-  if (prep != cudaSuccess) return prep;
+  if (const cudaError_t e = allow_batch_solve()) return e;
   ClusterLaunch l(st, scenes, width);
   return cudaLaunchKernelEx(&l.lc, kb_cluster_solve, bi, order, scratch, pa, pb, rhs, type, umap, list, part, ss,
                             SolveArgs{fixed_sweeps, check, max_iters, tol, nullptr});

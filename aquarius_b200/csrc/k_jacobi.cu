@@ -631,8 +631,10 @@ cudaError_t launch_cube(cudaStream_t st, const Dims& d, const float* pin, float*
                         const int8_t* type, const uint8_t* bact) {
   using S = CubeShape<L, TX>;
   constexpr size_t smem = (size_t)2 * S::ROWS * 32 * sizeof(float);
-  static const cudaError_t attr = cudaFuncSetAttribute(
-      k_jacobi_cube<L, TX, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static PerDevice once;
+  const cudaError_t attr = once([] {
+    return cudaFuncSetAttribute(k_jacobi_cube<L, TX, WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
   if (attr != cudaSuccess) return attr;
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3((d.sz + S::TZ - 1) / S::TZ, (d.sy + TX - 1) / TX, (d.sx + TX - 1) / TX);

@@ -742,8 +742,11 @@ template <int CIN, int COUT, bool RELU, bool BIAS, int SKIP>
 cudaError_t umma_launch(cudaStream_t st, const bf16* in, const bf16* skip, const bf16* w, const float* b, bf16* out,
                         int sx, int sy, int sz) {
   constexpr size_t smem = fwd_umma_smem<CIN, COUT>();
-  static const cudaError_t attr = cudaFuncSetAttribute(k_conv3_fwd_umma<CIN, COUT, RELU, BIAS, SKIP>,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  static PerDevice once;
+  const cudaError_t attr = once([] {
+    return cudaFuncSetAttribute(k_conv3_fwd_umma<CIN, COUT, RELU, BIAS, SKIP>,
+                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  });
   if (attr != cudaSuccess) return attr;
   const int planes = umma_chunk_planes(sx, sy, sz, umma_planes<CIN, COUT>(), umma_ctas<CIN, COUT>());
   const dim3 grid((sz + kUZ - 1) / kUZ, (sy + kUY - 1) / kUY, (sx + planes - 1) / planes);
@@ -759,9 +762,11 @@ cudaError_t fwd_launch(cudaStream_t st, const bf16* in, const bf16* w, const flo
   }
   if (g_conv_impl >= 1) {
     constexpr size_t smem = fwd_tile_smem<CIN, COUT>();
-    static const cudaError_t attr =
-        cudaFuncSetAttribute(k_conv3_fwd_tile<CIN, COUT, RELU, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem);
+    static PerDevice once;
+    const cudaError_t attr = once([] {
+      return cudaFuncSetAttribute(k_conv3_fwd_tile<CIN, COUT, RELU, BIAS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)smem);
+    });
     if (attr != cudaSuccess) return attr;
     const dim3 grid((sz + kTZ - 1) / kTZ, (sy + kTY - 1) / kTY, (sx + kTX - 1) / kTX);
     k_conv3_fwd_tile<CIN, COUT, RELU, BIAS><<<grid, 256, smem, st>>>(in, w, b, out, sx, sy, sz);
@@ -1284,8 +1289,11 @@ cudaError_t launch_conv3_wgrad(cudaStream_t st, int cin, int cout, const void* x
   bool done = false;
 #define X(A, B)                                                                                   \
   if (!done && cin == A && cout == B) {                                                           \
-    static const cudaError_t attr = cudaFuncSetAttribute(                                         \
-        k_conv3_wgrad<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)wgrad_smem<A, B>()); \
+    static PerDevice once;                                                                        \
+    const cudaError_t attr = once([] {                                                            \
+      return cudaFuncSetAttribute(k_conv3_wgrad<A, B>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+                                  (int)wgrad_smem<A, B>());                                       \
+    });                                                                                           \
     if (attr != cudaSuccess) return attr;                                                         \
     k_conv3_wgrad<A, B><<<grid, 128, wgrad_smem<A, B>(), st>>>((const bf16*)x, (const bf16*)dy, part, sx, sy, \
                                                              sz, cv);                             \

@@ -77,3 +77,10 @@ def test_splat_leaves_by_a_vote():
     assert "return" not in body[:body.index("__syncthreads")]
     for m in re.finditer(r"__ldcg\(mixed\)", body):
         assert re.search(r"__syncthreads_or\(tid == 0 && $", body[:m.start()])
+
+
+@pytest.mark.parametrize("source", [f for f, t in SOURCES.items() if "cudaFuncSetAttribute" in t])
+def test_kernel_attributes_are_set_on_every_device(source):
+    """cudaFuncSetAttribute acts on the current device: its result is not kept in
+    a static of the process."""
+    assert not re.search(r"static\s+(const\s+)?cudaError_t\s+\w+\s*=", _code(SOURCES[source]))
