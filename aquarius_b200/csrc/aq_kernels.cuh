@@ -208,20 +208,26 @@ long long cluster_solve_units(const Dims& d);  // units of 2 x 1 x 4 cells: entr
 int cluster_solve_width(const Dims& d);   // CTAs of the default plan
 bool cluster_solve_takes(const Dims& d, int width);               // the launch's limits
 bool cluster_solve_fits(const Dims& d, long long particles);      // the default plan's rule
+bool cluster_solve_holds(const Dims& d, int width);               // whatever the fluid does
 bool cluster_solve_runs(int width);  // the current device holds such a cluster, alone and in a batch
 // fixed_sweeps > 0: that many sweeps then one residual; else residual mode.
 // part: one double per 32 units.  Starts from pa, result in pa.  r2_only (may
-// be null): the squared residual goes there and *ss is only read.
-cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, float* pb, const float* rhs,
+// be null): the squared residual goes there and *ss is only read.  spill: the
+// graph condition that a fluid of too many units sets, whose solve is then
+// still to be done (0 only where cluster_solve_holds).
+cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, const float* rhs,
                                  const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
-                                 int fixed_sweeps, int check, int max_iters, double tol, double* r2_only);
-// The same for scenes order[0 .. scenes) of a batch, one cluster each;
-// scratch[s]: scene s's first entry in umap and list, and in part.
+                                 int fixed_sweeps, int check, int max_iters, double tol, double* r2_only,
+                                 unsigned long long spill);
+// The same for the live scenes of order[0 .. scenes) of a batch, one cluster
+// each; a solved scene is no longer live.  scratch[s]: scene s's first entry in
+// umap and list, and in part.
 int batch_cluster_width(const Dims& d, long long particles);  // 0: the scene does not fit a cluster
 cudaError_t launch_batch_cluster_solve(cudaStream_t st, const BatchIndex& bi, int scenes, int width, const int* order,
-                                       const int2* scratch, float* pa, float* pb, const float* rhs,
+                                       const int2* scratch, int* live, float* pa, const float* rhs,
                                        const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
-                                       int fixed_sweeps, int check, int max_iters, double tol);
+                                       int fixed_sweeps, int check, int max_iters, double tol,
+                                       unsigned long long spill);
 // ---- resident solve (k_resident.cu) ------------------------------------------
 // Plan rows = 4: the whole solve in one cooperative launch, one CTA per SM;
 // a CTA keeps a tile (plan.xc selects the TX x TY x TZ shape) plus a K-cell

@@ -77,9 +77,12 @@ struct aq_batch {
   int row_list_cap = 0;
 
   // Cluster solve (when every scene fits one): scenes by cluster width, largest
-  // first; each width is a launch on a stream of its own inside the step.
+  // first; each width is a launch on a stream of its own inside the step.  A
+  // fluid that has outgrown its cluster stays live and is solved behind them
+  // in a cluster of 16 CTAs, or else by the row sweeps (cl_spill, cl_spill16:
+  // some scene can come to that).
   static constexpr int kWidths = 5;  // 1, 2, 4, 8, 16 CTAs
-  bool clusters = false;
+  bool clusters = false, cl_spill = false, cl_spill16 = false;
   int cl_first[kWidths + 1] = {0};
   int* cl_order = nullptr;
   int2* cl_scratch = nullptr;
@@ -154,12 +157,13 @@ struct aq_batch {
 
   aq_status allocate();
   aq_status plan_clusters();
-  aq_status enq_clusters();
+  aq_status enq_clusters(unsigned long long spill);
+  aq_status enq_wide_clusters(unsigned long long spill);
   aq_status add_scene(int s, aq_fluid* f);
   aq_status enq_sort();       // the step's particle stage
   aq_status enq_pre_solve();  // the rest up to the solve
   aq_status enq_sweeps(int sweeps);
-  aq_status enq_solve_fixed();
+  aq_status enq_solve_fixed();  // by row sweeps, of the live scenes
   aq_status enq_solve_body(unsigned long long handle);
   aq_status enq_post_solve();
   aq_status capture_step(bool sort, bool rest, cudaGraphExec_t* out);
@@ -226,13 +230,15 @@ aq_status aq_batch::plan_clusters() {
     int k = 0;
     while ((1 << k) < w) ++k;
     by[k].push_back(s);
+    cl_spill |= !cluster_solve_holds(S.d, w);
+    cl_spill16 |= !cluster_solve_holds(S.d, 16);
     scratch[s] = make_int2((int)units, (int)parts);
     const long long u = cluster_solve_units(S.d);
     units += u;
     parts += u / 32 + 1;
   }
   for (int k = 0; k < kWidths; ++k)
-    if (!by[k].empty() && !cluster_solve_runs(1 << k)) return AQ_OK;
+    if ((!by[k].empty() || (cl_spill && k == kWidths - 1)) && !cluster_solve_runs(1 << k)) return AQ_OK;
   std::vector<int> order;
   for (int k = 0; k < kWidths; ++k) {
     std::stable_sort(by[k].begin(), by[k].end(), [&](int a, int b) { return scenes[a].n > scenes[b].n; });
@@ -255,19 +261,29 @@ aq_status aq_batch::plan_clusters() {
 }
 
 // The solves of all scenes; widest clusters first.
-aq_status aq_batch::enq_clusters() {
+aq_status aq_batch::enq_clusters(unsigned long long spill) {
   const int fixed = solver.solve_mode == AQ_SOLVE_RESIDUAL ? 0 : solver.pressure_iterations;
   AQB_CUDA(cudaEventRecord(cl_event[kWidths], stream));
   for (int k = kWidths - 1; k >= 0; --k) {
     const int n = cl_first[k + 1] - cl_first[k];
     if (n == 0) continue;
     AQB_CUDA(cudaStreamWaitEvent(cl_stream[k], cl_event[kWidths], 0));
-    AQB_CUDA(launch_batch_cluster_solve(cl_stream[k], bi, n, 1 << k, cl_order + cl_first[k], cl_scratch, pa, pb, rhs,
+    AQB_CUDA(launch_batch_cluster_solve(cl_stream[k], bi, n, 1 << k, cl_order + cl_first[k], cl_scratch, live, pa, rhs,
                                         type, cl_map, cl_list, cl_part, ss, fixed, solver.check_interval,
-                                        solver.max_iterations, (double)solver.rel_residual));
+                                        solver.max_iterations, (double)solver.rel_residual, spill));
     AQB_CUDA(cudaEventRecord(cl_event[k], cl_stream[k]));
     AQB_CUDA(cudaStreamWaitEvent(stream, cl_event[k], 0));
   }
+  return AQ_OK;
+}
+
+// The scenes still live, a cluster of 16 CTAs each.
+aq_status aq_batch::enq_wide_clusters(unsigned long long spill) {
+  AQB_CUDA(launch_batch_cluster_solve(stream, bi, ns, 1 << (kWidths - 1), cl_order, cl_scratch, live, pa, rhs, type,
+                                      cl_map, cl_list, cl_part, ss,
+                                      solver.solve_mode == AQ_SOLVE_RESIDUAL ? 0 : solver.pressure_iterations,
+                                      solver.check_interval, solver.max_iterations, (double)solver.rel_residual,
+                                      spill));
   return AQ_OK;
 }
 
@@ -360,13 +376,17 @@ aq_status aq_batch::enq_sweeps(int sweeps) {
 aq_status aq_batch::enq_solve_fixed() {
   const int K = solver.pressure_iterations;
   if (K <= 0) return AQ_OK;
-  if (clusters) return enq_clusters();
-  AQB_TRY(enq_sweeps(K));
-  AQB_CUDA(launch_batch_resid_flat(stream, bi, pre_f[ns], grid(), live, K % 2 ? pb : pa, rhs, type, bact, rpart));
+  // an odd count sweeps from a copy in pb, so that it ends in pa, where the
+  // scenes that are not live keep theirs
   if (K % 2) {
-    kb_copy_f<<<cdiv(C, 256), 256, 0, stream>>>(pb, pa, C);
+    kb_copy_f<<<cdiv(C, 256), 256, 0, stream>>>(pa, pb, C);
     AQB_CUDA(cudaGetLastError());
+    std::swap(pa, pb);
   }
+  const aq_status st = enq_sweeps(K);
+  if (K % 2) std::swap(pa, pb);
+  AQB_TRY(st);
+  AQB_CUDA(launch_batch_resid_flat(stream, bi, pre_f[ns], grid(), live, pa, rhs, type, bact, rpart));
   AQB_CUDA(launch_batch_resid_finalize(stream, bi, rpart, ss, live, K, 0.0, 0));
   return AQ_OK;
 }
@@ -399,79 +419,60 @@ aq_status aq_batch::build_graph() {
 aq_status aq_batch::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   AQB_CUDA(cudaGraphCreate(&g, 0));
-  auto capture = [&](cudaGraph_t into, const cudaGraphNode_t* deps, size_t nd, auto&& body) -> aq_status {
-    AQB_CUDA(cudaStreamBeginCaptureToGraph(stream, into, deps, nullptr, nd, cudaStreamCaptureModeThreadLocal));
-    aq_status st = body();
-    cudaGraph_t got = nullptr;
-    cudaError_t e = cudaStreamEndCapture(stream, &got);
-    if (st != AQ_OK) return st;
-    if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    return AQ_OK;
-  };
   // counted as the row sweeps run; the cluster solve does a step's blocks in
   // one launch per cluster width instead
   const int pre_launches = (N > 0 ? 6 : 3) + 5;  // sort; p2g, s-layer, divergence, b2, row list
   const int post_launches = 4;
+  const bool residual = solver.solve_mode == AQ_SOLVE_RESIDUAL;
+  const int K = residual ? 0 : std::max(0, solver.pressure_iterations);
   auto before_solve = [&]() -> aq_status {
     if (sort) AQB_TRY(enq_sort());
     return rest ? enq_pre_solve() : AQ_OK;
   };
-  aq_status st;
-  if (!rest) {
-    st = capture(g, nullptr, 0, before_solve);
-  } else if (solver.solve_mode == AQ_SOLVE_RESIDUAL && clusters) {
-    st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = before_solve();
-      if (s2 != AQ_OK) return s2;
-      s2 = enq_clusters();
-      if (s2 != AQ_OK) return s2;
-      return enq_post_solve();
-    });
-    body_launches = solver.check_interval + 3;
-    graph_launches = pre_launches + post_launches;
-  } else if (solver.solve_mode == AQ_SOLVE_RESIDUAL) {
-    st = capture(g, nullptr, 0, before_solve);
-    if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
-    size_t nn = 0;
-    cudaGraphGetNodes(g, nullptr, &nn);
-    std::vector<cudaGraphNode_t> nodes(nn), leaves;
-    cudaGraphGetNodes(g, nodes.data(), &nn);
-    for (cudaGraphNode_t nd : nodes) {
-      size_t k = 0;
-      cudaGraphNodeGetDependentNodes(nd, nullptr, &k);
-      if (k == 0) leaves.push_back(nd);
-    }
-    cudaGraphConditionalHandle handle;
-    cudaError_t e = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) { cudaGraphDestroy(g); return fail(AQ_ERR_CUDA, cudaGetErrorString(e)); }
-    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-    cp.conditional.handle = handle;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    e = cudaGraphAddNode(&cnode, g, leaves.data(), leaves.size(), &cp);
-    if (e != cudaSuccess) {
-      cudaGraphDestroy(g);
-      return fail(AQ_ERR_CUDA, std::string("conditional node: ") + cudaGetErrorString(e));
-    }
-    st = capture(cp.conditional.phGraph_out[0], nullptr, 0,
-                 [&]() { return enq_solve_body((unsigned long long)handle); });
-    if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
-    st = capture(g, &cnode, 1, [&]() { return enq_post_solve(); });
-    body_launches = solver.check_interval + 3;
-    graph_launches = pre_launches + post_launches;
-  } else {
-    st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = before_solve();
-      if (s2 != AQ_OK) return s2;
-      s2 = enq_solve_fixed();
-      if (s2 != AQ_OK) return s2;
-      return enq_post_solve();
-    });
-    const int K = solver.pressure_iterations;
-    body_launches = 0;
+  auto build = [&]() -> aq_status {
+    if (!rest) return capture_into(stream, g, nullptr, 0, before_solve);
+    body_launches = residual ? solver.check_interval + 3 : 0;
     graph_launches = pre_launches + post_launches + (K > 0 ? K + 2 + (K % 2) : 0);
-  }
+    cudaGraphConditionalHandle spill = 0, rows = 0;
+    cudaGraphNode_t node;
+    cudaGraph_t body;
+    const bool solve = residual || K > 0;
+    if (solve && clusters && !cl_spill) {
+      return capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
+        AQB_TRY(before_solve());
+        AQB_TRY(enq_clusters(0));
+        return enq_post_solve();
+      });
+    }
+    if (!residual && !(solve && clusters)) {
+      return capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
+        AQB_TRY(before_solve());
+        AQB_TRY(enq_solve_fixed());
+        return enq_post_solve();
+      });
+    }
+    // conditional nodes, one behind the other: the scenes that spill go to
+    // clusters of 16 CTAs, those that do not fit them to the row sweeps
+    if (clusters) AQB_TRY(make_condition(g, 0, &spill));
+    if (!clusters || cl_spill16) AQB_TRY(make_condition(g, clusters ? 0 : 1, &rows));
+    AQB_TRY(capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
+      AQB_TRY(before_solve());
+      return clusters ? enq_clusters(spill) : AQ_OK;
+    }));
+    if (clusters) {
+      AQB_TRY(add_conditional(g, spill, false, &node, &body));
+      AQB_TRY(capture_into(stream, body, nullptr, 0, [&]() { return enq_wide_clusters(rows); }));
+    }
+    if (rows) {
+      AQB_TRY(add_conditional(g, rows, residual, &node, &body));
+      AQB_TRY(capture_into(stream, body, nullptr, 0, [&]() -> aq_status {
+        if (clusters) AQB_TRY(enq_row_list());
+        return residual ? enq_solve_body(rows) : enq_solve_fixed();
+      }));
+    }
+    return capture_into(stream, g, &node, 1, [&]() { return enq_post_solve(); });
+  };
+  const aq_status st = build();
   if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
   cudaError_t e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);

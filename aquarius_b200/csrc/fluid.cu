@@ -291,7 +291,7 @@ aq_status aq_fluid::allocate() {
   // default Jacobi plan: one vectorised sweep per launch over the listed
   // active warp rows where z allows it, otherwise the tiled kernel with two
   // sweeps per launch
-  plan = d.sz % 4 == 0 ? JacobiPlan{1, 3, 1} : JacobiPlan{2, 16, 16};
+  plan = wide = d.sz % 4 == 0 ? JacobiPlan{1, 3, 1} : JacobiPlan{2, 16, 16};
   // room for the default plan's residual partials: the flat pass, or the
   // fused residual level of every launch size split_sweeps can produce
   int need = d.sz % 4 == 0 ? resid_flat_parts(d) : 0;
@@ -407,10 +407,6 @@ static aq_status enqueue_sweeps_on(aq_fluid* f, const JacobiPlan& plan, float* a
   return AQ_OK;
 }
 
-static aq_status enqueue_sweeps(aq_fluid* f, int sweeps, bool with_residual = true) {
-  return enqueue_sweeps_on(f, f->plan, f->pa, f->pb, sweeps, with_residual, f->jpart);
-}
-
 static int last_parts_of(const aq_fluid* f, const JacobiPlan& plan, int sweeps) {
   const std::vector<int> parts = split_sweeps(sweeps, plan.levels);
   if (parts.empty()) return 0;
@@ -419,8 +415,6 @@ static int last_parts_of(const aq_fluid* f, const JacobiPlan& plan, int sweeps) 
   p.levels = parts.back();
   return jacobi_parts(f->d, p, true);
 }
-
-static int last_parts(const aq_fluid* f, int sweeps) { return last_parts_of(f, f->plan, sweeps); }
 
 aq_status aq_fluid::enq_row_items() {
   // the list plan's rows; the resident plan's learned start sweeps them too
@@ -437,14 +431,16 @@ int aq_fluid::solve_sweeps_done() const { return cfg.pressure_init == AQ_PRESSUR
 aq_status aq_fluid::enq_learned_start() {
   if (!net || !net_acts) return fail(AQ_ERR_INVALID_CONFIG, "AQ_PRESSURE_LEARNED needs a network (aq_fluid_set_warm_start)");
   AQ_TRY(unet_predict(net, stream, net_acts, rhs, type, pa));
-  // the two short starts: a cluster solve each where that is the plan, else
-  // one sweep per launch (the list plan when the solve itself is one launch)
+  // the two short starts: a cluster solve each where that is the plan and
+  // always holds the fluid, else one sweep per launch (the list plan when the
+  // solve itself is one launch)
   const JacobiPlan wp = whole_solve(plan) ? JacobiPlan{1, 3, 1} : plan;
-  const bool cluster = plan.by == 5;
+  const bool cluster = plan.by == 5 && !may_spill();
+  if (may_spill()) AQ_CUDA(launch_row_items(stream, d, bact, row_items, n_row_items));
   auto start = [&](float* a, float* b, double* part) -> aq_status {
     if (!cluster) return enqueue_sweeps_on(this, wp, a, b, kWarmSweeps, true, part);
-    AQ_CUDA(launch_cluster_solve(stream, d, plan.xc, a, b, rhs, type, cl_map, cl_list, cl_part, ss, kWarmSweeps, 0, 0,
-                                 0.0, part));
+    AQ_CUDA(launch_cluster_solve(stream, d, plan.xc, a, rhs, type, cl_map, cl_list, cl_part, ss, kWarmSweeps, 0, 0,
+                                 0.0, part, 0));
     return AQ_OK;
   };
   AQ_TRY(start(pa, pb, jpart));
@@ -477,11 +473,13 @@ static aq_status enqueue_resident(aq_fluid* f, int fixed_sweeps) {
   return AQ_OK;
 }
 
-// The whole solve as one launch of one cluster (plan.by == 5).
-static aq_status enqueue_cluster(aq_fluid* f, int fixed_sweeps) {
-  AQ_CUDA(launch_cluster_solve(f->stream, f->d, f->plan.xc, f->pa, f->pb, f->rhs, f->type, f->cl_map, f->cl_list,
-                               f->cl_part, f->ss, fixed_sweeps, f->cfg.check_interval, f->cfg.max_iterations,
-                               (double)f->cfg.rel_residual, nullptr));
+// The whole solve as one launch of one cluster (plan.by == 5); spill: the
+// condition of the graph that runs enq_sweeps_fixed or a loop of
+// enq_solve_body where the fluid does not fit.
+static aq_status enqueue_cluster(aq_fluid* f, int fixed_sweeps, unsigned long long spill) {
+  AQ_CUDA(launch_cluster_solve(f->stream, f->d, f->plan.xc, f->pa, f->rhs, f->type, f->cl_map, f->cl_list, f->cl_part,
+                               f->ss, fixed_sweeps, f->cfg.check_interval, f->cfg.max_iterations,
+                               (double)f->cfg.rel_residual, nullptr, spill));
   return AQ_OK;
 }
 
@@ -489,43 +487,57 @@ static aq_status enqueue_cluster(aq_fluid* f, int fixed_sweeps) {
 static aq_status enqueue_whole(aq_fluid* f, int fixed_sweeps) {
   return f->plan.by == 1   ? enqueue_persistent(f, fixed_sweeps)
          : f->plan.by == 4 ? enqueue_resident(f, fixed_sweeps)
-                           : enqueue_cluster(f, fixed_sweeps);
+                           : enqueue_cluster(f, fixed_sweeps, 0);
+}
+
+// The row list of a spilled fluid's sweeps, whose plan is not the fluid's own.
+static aq_status enqueue_wide_rows(aq_fluid* f) {
+  if (f->wide.by == 3) AQ_CUDA(launch_row_items(f->stream, f->d, f->bact, f->row_items, f->n_row_items));
+  return AQ_OK;
+}
+
+aq_status aq_fluid::enq_sweeps_fixed(const JacobiPlan& p, int sweeps) {
+  AQ_TRY(enqueue_sweeps_on(this, p, pa, pb, sweeps, true, jpart));
+  AQ_CUDA(launch_resid_finalize(stream, jpart, last_parts_of(this, p, sweeps), ss, sweeps, 0.0, 0, false, 0));
+  return AQ_OK;
 }
 
 aq_status aq_fluid::enq_solve_fixed(int sweeps) {
   if (sweeps <= 0) return AQ_OK;
-  if (whole_solve(plan)) return enqueue_whole(this, sweeps);
-  AQ_TRY(enqueue_sweeps(this, sweeps));
-  AQ_CUDA(launch_resid_finalize(stream, jpart, last_parts(this, sweeps), ss, sweeps, 0.0, 0, false, 0));
-  return AQ_OK;
+  if (may_spill()) {
+    AQ_TRY(enqueue_wide_rows(this));
+    return enq_sweeps_fixed(wide, sweeps);
+  }
+  return whole_solve(plan) ? enqueue_whole(this, sweeps) : enq_sweeps_fixed(plan, sweeps);
 }
 
-aq_status aq_fluid::enq_solve_body(bool set_cond, unsigned long long handle, int* launches) {
+aq_status aq_fluid::enq_solve_body(const JacobiPlan& plan, bool set_cond, unsigned long long handle, int* launches) {
   const int m = cfg.check_interval;
   if (separate_residual(plan) && d.sz % 4 == 0) {
     // plans whose residual is a separate pass: pass and check in one launch
-    AQ_TRY(enqueue_sweeps(this, m, false));
+    AQ_TRY(enqueue_sweeps_on(this, plan, pa, pb, m, false, jpart));
     if (plan.by == 3)
       AQ_CUDA(launch_resid_list_fin(stream, d, pa, rhs, type, row_items, n_row_items, jpart, resid_ticket, ss, m,
                                     (double)cfg.rel_residual, cfg.max_iterations, set_cond, handle));
     else
       AQ_CUDA(launch_resid_flat_fin(stream, d, pa, rhs, type, bact, jpart, resid_ticket, ss, m,
                                     (double)cfg.rel_residual, cfg.max_iterations, set_cond, handle));
-    if (launches) *launches = count_jacobi_launches(m) - 1;
+    if (launches) *launches = jacobi_launches(plan, m) - 1;
     return AQ_OK;
   }
-  AQ_TRY(enqueue_sweeps(this, m));
-  AQ_CUDA(launch_resid_finalize(stream, jpart, last_parts(this, m), ss, m, (double)cfg.rel_residual,
+  AQ_TRY(enqueue_sweeps_on(this, plan, pa, pb, m, true, jpart));
+  AQ_CUDA(launch_resid_finalize(stream, jpart, last_parts_of(this, plan, m), ss, m, (double)cfg.rel_residual,
                                 cfg.max_iterations, set_cond, handle));
-  if (launches) *launches = count_jacobi_launches(m);
+  if (launches) *launches = jacobi_launches(plan, m);
   return AQ_OK;
 }
 
 // Residual mode without a graph: the host reads the solve state after each block.
 aq_status aq_fluid::enq_solve_residual_eager() {
-  if (whole_solve(plan)) return enqueue_whole(this, 0);
+  if (whole_solve(plan) && !may_spill()) return enqueue_whole(this, 0);
+  if (may_spill()) AQ_TRY(enqueue_wide_rows(this));
   for (int guard = 0; guard < 1000000; ++guard) {
-    AQ_TRY(enq_solve_body(false, 0, nullptr));
+    AQ_TRY(enq_solve_body(may_spill() ? wide : plan, false, 0, nullptr));
     AQ_CUDA(cudaMemcpyAsync(ss_host, ss, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
     AQ_CUDA(cudaStreamSynchronize(stream));
     const SolveState& s = *ss_host;
@@ -676,95 +688,82 @@ aq_status aq_fluid::enable_ink() {
   return AQ_OK;
 }
 
-static aq_status leaves_of(cudaGraph_t g, std::vector<cudaGraphNode_t>& out) {
+aq_status aqb::add_conditional(cudaGraph_t g, cudaGraphConditionalHandle handle, bool loop, cudaGraphNode_t* node,
+                               cudaGraph_t* body) {
   size_t nn = 0;
   AQ_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
-  std::vector<cudaGraphNode_t> nodes(nn);
+  std::vector<cudaGraphNode_t> nodes(nn), leaves;
   AQ_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-  out.clear();
   for (cudaGraphNode_t nd : nodes) {
     size_t k = 0;
     AQ_CUDA(cudaGraphNodeGetDependentNodes(nd, nullptr, &k));
-    if (k == 0) out.push_back(nd);
+    if (k == 0) leaves.push_back(nd);
   }
+  cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
+  cp.conditional.handle = handle;
+  cp.conditional.type = loop ? cudaGraphCondTypeWhile : cudaGraphCondTypeIf;
+  cp.conditional.size = 1;
+  const cudaError_t e = cudaGraphAddNode(node, g, leaves.data(), leaves.size(), &cp);
+  if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("conditional node: ") + cudaGetErrorString(e));
+  *body = cp.conditional.phGraph_out[0];
   return AQ_OK;
 }
 
 // The whole step as one CUDA graph.  RESIDUAL mode puts the sweeps in a
 // conditional WHILE node whose body ends with the residual check that sets
-// the loop condition, so a step needs no host round trip.
+// the loop condition, so a step needs no host round trip.  Behind a cluster
+// solve that the fluid can outgrow stands a conditional node with the sweeps
+// over the whole machine; the cluster solve sets its condition.
 aq_status aq_fluid::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
   cudaGraph_t g = nullptr;
   AQ_CUDA(cudaGraphCreate(&g, 0));
-  int launches = 0;
-  auto capture = [&](cudaGraph_t into, const cudaGraphNode_t* deps, size_t nd, auto&& body) -> aq_status {
-    AQ_CUDA(cudaStreamBeginCaptureToGraph(stream, into, deps, nullptr, nd, cudaStreamCaptureModeThreadLocal));
-    aq_status st = body();
-    cudaGraph_t got = nullptr;
-    cudaError_t e = cudaStreamEndCapture(stream, &got);
-    if (st != AQ_OK) return st;
-    if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
-    return AQ_OK;
-  };
+  int launches = (n > 0 ? 6 : 3) + 2 + 2;  // particles (+3 scan kernels), p2g, slayer, divergence, b2
+  const bool residual = cfg.solve_mode == AQ_SOLVE_RESIDUAL;
+  const int fixed = residual ? 0 : cfg.pressure_iterations - solve_sweeps_done();
+  const bool spill = may_spill() && (residual || fixed > 0);
+  const bool loop = residual && (spill || !whole_solve(plan));
   auto before_solve = [&]() -> aq_status {
     if (sort) AQ_TRY(enq_sort());
     return rest ? enq_pre_solve() : AQ_OK;
   };
-  aq_status st = AQ_OK;
-  launches += (n > 0 ? 6 : 3) + 2 + 2;  // particles (+3 scan kernels), p2g, slayer, divergence, b2
-  if (!rest) {
-    st = capture(g, nullptr, 0, before_solve);
-  } else if (cfg.solve_mode == AQ_SOLVE_RESIDUAL && whole_solve(plan)) {
-    st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = before_solve();
-      if (s2 != AQ_OK) return s2;
-      s2 = enqueue_whole(this, 0);
-      if (s2 != AQ_OK) return s2;
-      return enq_post_solve();
-    });
-    launches += count_jacobi_launches(0);
+  auto build = [&]() -> aq_status {
+    if (!rest) return capture_into(stream, g, nullptr, 0, before_solve);
     body_launches = 0;
-  } else if (cfg.solve_mode == AQ_SOLVE_RESIDUAL) {
-    st = capture(g, nullptr, 0, before_solve);
-    if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
-    std::vector<cudaGraphNode_t> leaves;
-    st = leaves_of(g, leaves);
-    if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
-    cudaGraphConditionalHandle handle;
-    cudaError_t e = cudaGraphConditionalHandleCreate(&handle, g, 1, cudaGraphCondAssignDefault);
-    if (e != cudaSuccess) { cudaGraphDestroy(g); return fail(AQ_ERR_CUDA, cudaGetErrorString(e)); }
-    cudaGraphNodeParams cp = {cudaGraphNodeTypeConditional};
-    cp.conditional.handle = handle;
-    cp.conditional.type = cudaGraphCondTypeWhile;
-    cp.conditional.size = 1;
-    cudaGraphNode_t cnode;
-    e = cudaGraphAddNode(&cnode, g, leaves.data(), leaves.size(), &cp);
-    if (e != cudaSuccess) {
-      cudaGraphDestroy(g);
-      return fail(AQ_ERR_CUDA, std::string("conditional node: ") + cudaGetErrorString(e));
+    if (!spill && !loop) {
+      launches += residual || fixed > 0 ? count_jacobi_launches(fixed) : 0;
+      return capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
+        AQ_TRY(before_solve());
+        AQ_TRY(residual ? enqueue_whole(this, 0) : enq_solve_fixed(fixed));
+        return enq_post_solve();
+      });
     }
-    cudaGraph_t body = cp.conditional.phGraph_out[0];
+    cudaGraphConditionalHandle handle;
+    AQ_TRY(make_condition(g, spill ? 0 : 1, &handle));
+    AQ_TRY(capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
+      AQ_TRY(before_solve());
+      return spill ? enqueue_cluster(this, fixed, handle) : AQ_OK;
+    }));
+    cudaGraphNode_t node;
+    cudaGraph_t body;
+    AQ_TRY(add_conditional(g, handle, loop, &node, &body));
     int bl = 0;
-    st = capture(body, nullptr, 0, [&]() { return enq_solve_body(true, (unsigned long long)handle, &bl); });
-    if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
-    body_launches = bl;
-    st = capture(g, &cnode, 1, [&]() { return enq_post_solve(); });
-  } else {
-    st = capture(g, nullptr, 0, [&]() {
-      aq_status s2 = before_solve();
-      if (s2 != AQ_OK) return s2;
-      s2 = enq_solve_fixed(cfg.pressure_iterations - solve_sweeps_done());
-      if (s2 != AQ_OK) return s2;
-      return enq_post_solve();
-    });
-    const int rest = cfg.pressure_iterations - solve_sweeps_done();
-    launches += rest > 0 ? count_jacobi_launches(rest) : 0;
-    body_launches = 0;
-  }
+    AQ_TRY(capture_into(stream, body, nullptr, 0, [&]() -> aq_status {
+      if (spill) AQ_TRY(enqueue_wide_rows(this));
+      return residual ? enq_solve_body(spill ? wide : plan, true, handle, &bl) : enq_sweeps_fixed(wide, fixed);
+    }));
+    if (spill) launches += 1;  // the cluster solve; the branch that may follow it is not counted
+    else body_launches = bl;
+    return capture_into(stream, g, &node, 1, [&]() { return enq_post_solve(); });
+  };
+  const aq_status st = build();
   if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
   if (cfg.pressure_init == AQ_PRESSURE_LEARNED)  // network, two 20-sweep starts, pick, copy
     launches += kUNetForwardLaunches +
-                2 * (plan.by == 5 ? 1 : jacobi_launches(plan.by == 4 ? JacobiPlan{1, 3, 1} : plan, kWarmSweeps) - 1) + 2;
+                (may_spill() ? 1 : 0) +
+                2 * (plan.by == 5 && !may_spill()
+                         ? 1
+                         : jacobi_launches(whole_solve(plan) ? JacobiPlan{1, 3, 1} : plan, kWarmSweeps) - 1) +
+                2;
   launches += 1 + 3 + (multiphase ? cfg.diffusion_iterations : 0) + (ink_on && n_ink > 0 ? 1 : 0);
   if (sort && rest) graph_launches = launches;
   cudaError_t e = cudaGraphInstantiate(out, g, 0);
@@ -1730,15 +1729,28 @@ aq_status aq_fluid_benchmark_pressure(aq_fluid* f, int32_t sweeps, float* ms, in
   cudaSetDevice(f->device);
   // The sweeps are captured into a graph and replayed, as inside a step.
   cudaGraph_t g = nullptr;
-  AQ_CUDA(cudaStreamBeginCapture(f->stream, cudaStreamCaptureModeThreadLocal));
-  aq_status st = whole_solve(f->plan) ? enqueue_whole(f, sweeps) : enqueue_sweeps(f, sweeps, false);
-  cudaGraph_t got = nullptr;
-  cudaError_t ce = cudaStreamEndCapture(f->stream, &got);
-  if (st != AQ_OK) { if (got) cudaGraphDestroy(got); return st; }
-  if (ce != cudaSuccess) return fail(AQ_ERR_CUDA, cudaGetErrorString(ce));
-  g = got;
+  AQ_CUDA(cudaGraphCreate(&g, 0));
+  auto build = [&]() -> aq_status {
+    cudaGraphConditionalHandle handle = 0;
+    if (f->may_spill()) AQ_TRY(make_condition(g, 0, &handle));
+    AQ_TRY(capture_into(f->stream, g, nullptr, 0, [&]() -> aq_status {
+      if (f->may_spill()) return enqueue_cluster(f, sweeps, handle);
+      return whole_solve(f->plan) ? enqueue_whole(f, sweeps)
+                                  : enqueue_sweeps_on(f, f->plan, f->pa, f->pb, sweeps, false, f->jpart);
+    }));
+    if (!f->may_spill()) return AQ_OK;
+    cudaGraphNode_t node;
+    cudaGraph_t body;
+    AQ_TRY(add_conditional(g, handle, false, &node, &body));
+    return capture_into(f->stream, body, nullptr, 0, [&]() -> aq_status {
+      AQ_TRY(enqueue_wide_rows(f));
+      return f->enq_sweeps_fixed(f->wide, sweeps);
+    });
+  };
+  const aq_status st = build();
+  if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
   cudaGraphExec_t ex = nullptr;
-  ce = cudaGraphInstantiate(&ex, g, 0);
+  cudaError_t ce = cudaGraphInstantiate(&ex, g, 0);
   cudaGraphDestroy(g);
   if (ce != cudaSuccess) return fail(AQ_ERR_CUDA, cudaGetErrorString(ce));
   cudaEvent_t a, b;

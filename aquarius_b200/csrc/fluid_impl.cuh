@@ -17,6 +17,31 @@ namespace aqb {
 constexpr size_t kSplitBytes = 1u << 20;
 
 inline aq_status fail(aq_status st, const std::string& msg) { return set_last_error(st, msg); }
+
+// Captures what body enqueues on `stream` into g, behind deps.
+template <class F>
+aq_status capture_into(cudaStream_t stream, cudaGraph_t g, const cudaGraphNode_t* deps, size_t nd, F&& body) {
+  cudaError_t e = cudaStreamBeginCaptureToGraph(stream, g, deps, nullptr, nd, cudaStreamCaptureModeThreadLocal);
+  if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("begin capture: ") + cudaGetErrorString(e));
+  const aq_status st = body();
+  cudaGraph_t got = nullptr;
+  e = cudaStreamEndCapture(stream, &got);
+  if (st != AQ_OK) return st;
+  if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("capture: ") + cudaGetErrorString(e));
+  return AQ_OK;
+}
+
+// A condition of g with its value at each launch.
+inline aq_status make_condition(cudaGraph_t g, unsigned value, cudaGraphConditionalHandle* handle) {
+  const cudaError_t e = cudaGraphConditionalHandleCreate(handle, g, value, cudaGraphCondAssignDefault);
+  if (e != cudaSuccess) return fail(AQ_ERR_CUDA, std::string("condition: ") + cudaGetErrorString(e));
+  return AQ_OK;
+}
+
+// A conditional node of g behind all its last nodes; *body is the graph it runs.
+aq_status add_conditional(cudaGraph_t g, cudaGraphConditionalHandle handle, bool loop, cudaGraphNode_t* node,
+                          cudaGraph_t* body);
+
 struct UActs;
 struct MeshState;                  // surface mesher buffers (mesh.cu)
 void mesh_release(MeshState* s);
@@ -103,6 +128,7 @@ struct aq_fluid {
   double* cl_part = nullptr;
 
   JacobiPlan plan{4, 16, 32};
+  JacobiPlan wide{2, 16, 16};  // the grid's plan of sweeps over the whole machine (default without a cluster)
   // learned warm start (AQ_PRESSURE_LEARNED)
   aq_unet* net = nullptr;
   aqb::UActs* net_acts = nullptr;
@@ -171,13 +197,17 @@ struct aq_fluid {
 
   aq_status allocate();
   aq_status alloc_cluster();
+  // the plan is a cluster that the fluid can outgrow: a step's graph then also
+  // holds the sweeps of `wide`, and work outside of a graph runs those
+  bool may_spill() const { return plan.by == 5 && !aqb::cluster_solve_holds(d, plan.xc); }
   aq_status seed_and_init();
   // stage enqueues (eager or under capture)
   aq_status enq_particles(bool move);
   aq_status enq_p2g(bool forces);
   aq_status enq_divergence();
   aq_status enq_solve_fixed(int sweeps);
-  aq_status enq_solve_body(bool set_cond, unsigned long long handle, int* launches);
+  aq_status enq_sweeps_fixed(const JacobiPlan& p, int sweeps);  // sweeps and their residual
+  aq_status enq_solve_body(const JacobiPlan& p, bool set_cond, unsigned long long handle, int* launches);
   aq_status enq_solve_residual_eager();
   aq_status enq_learned_start();
   int solve_sweeps_done() const;  // sweeps the warm start already did (0 without it)

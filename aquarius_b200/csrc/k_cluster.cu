@@ -36,9 +36,10 @@
 // sums in index order, so a solve's decisions do not depend on the cluster
 // size (a scene in a batch stops where it stops alone).
 //
-// A fluid that spreads over more units than the cluster's shared memory holds
-// is swept by the same cluster through global memory (solve_global below):
-// the same results, many times slower.
+// A fluid may spread over more units than the cluster's shared memory holds (a
+// droplet occupies a whole unit).  The cluster then leaves the system as it is
+// and sets the graph condition that runs the solve's other branch, the sweeps
+// over the whole machine.
 #include <algorithm>
 #include <type_traits>
 
@@ -49,19 +50,19 @@ namespace {
 
 constexpr int kT = 512;                    // threads per CTA
 constexpr int kU = 4;                      // units per thread
-constexpr int kSlots = 2048;               // units per buffer, the last one zero
-constexpr int kZero = kSlots - 1;
-constexpr int kCap = 2016;                 // units per CTA (a multiple of 32)
+constexpr int kCap = 2048;                 // units per CTA (a multiple of 32): 16 CTAs hold any 64^3 fluid
+constexpr int kZero = kCap;                // the zero unit of a buffer
+constexpr int kSlots = kCap + 16;          // units per buffer
 constexpr int kHalf = kSlots * 16;         // bytes from quad A to quad B
 constexpr int kBufBytes = 2 * kHalf;
 constexpr int kSmem = 2 * kBufBytes;
 constexpr int kScanBits = 32;              // scan passes a thread remembers as one bit each
 constexpr int kSmallUnits = 1024;          // grids up to this many units (fluid or not) take one CTA
-static_assert(kCap <= kT * kU && kCap < kZero && kCap % 32 == 0, "a CTA's share must fit its threads");
+static_assert(kCap <= kT * kU && kCap % 32 == 0, "a CTA's share must fit its threads");
 
 struct ClusterScene {
   Dims d;
-  float *pa, *pb;
+  float* pa;
   const float* rhs;
   const int8_t* type;
   int *umap, *list;  // unit -> index among the fluid units (-1: none), and back
@@ -73,6 +74,8 @@ struct SolveArgs {
   int fixed_sweeps, check, max_iters;  // fixed_sweeps 0: residual mode
   double tol;
   double* r2_only;  // if set: where ||b - A p||^2 goes, and the solve state stays as it is
+  // set to 1 where the fluid's units do not fit; 0 where they always do
+  cudaGraphConditionalHandle spill;
 };
 
 // What every thread of the cluster knows of the running solve.
@@ -536,77 +539,6 @@ __device__ __forceinline__ void solve_shared(const ClusterScene& S, const SolveA
   cluster_sync(nr);  // no CTA leaves while another reads its buffers
 }
 
-// A unit's inputs from global memory (the iterate is rewritten by the
-// cluster's other CTAs between sweeps, so its loads go to L2).
-__device__ __forceinline__ UnitIn gload_unit(const Dims& d, const float* __restrict__ p, const UnitPos& q) {
-  const int plane = d.sy * d.sz, b = q.cell + plane;
-  UnitIn u;
-  u.a = load_cells(p, q.cell, q.len);
-  u.b = q.two ? load_cells(p, b, q.len) : u.a;
-  u.xm = q.x > 0 ? load_cells(p, q.cell - plane, q.len) : u.a;
-  u.xp = q.x + 2 < d.sx ? load_cells(p, b + plane, q.len) : u.b;
-  u.ypa = q.y + 1 < d.sy ? load_cells(p, q.cell + d.sz, q.len) : u.a;
-  u.yma = q.y > 0 ? load_cells(p, q.cell - d.sz, q.len) : u.a;
-  u.ypb = q.two && q.y + 1 < d.sy ? load_cells(p, b + d.sz, q.len) : u.b;
-  u.ymb = q.two && q.y > 0 ? load_cells(p, b - d.sz, q.len) : u.b;
-  const bool lo = q.zq > 0, hi = 4 * q.zq + 4 < d.sz;
-  u.zla = lo ? __ldcg(p + q.cell - 1) : unpack2(u.a.lo).x;
-  u.zha = hi ? __ldcg(p + q.cell + 4) : unpack2(u.a.hi).y;
-  u.zlb = lo && q.two ? __ldcg(p + b - 1) : unpack2(u.b.lo).x;
-  u.zhb = hi && q.two ? __ldcg(p + b + 4) : unpack2(u.b.hi).y;
-  return u;
-}
-
-// The solve through global memory, for a fluid of more units than the
-// cluster's shared memory holds.
-__device__ __noinline__ void solve_global(const ClusterScene& S, const SolveArgs& a, Solve& v, double* s_red) {
-  const Dims& d = S.d;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int nq = (d.sz + 3) / 4, plane = d.sy * d.sz;
-  const bool vec = d.sz % 4 == 0;
-  const int begin = (int)v.me * kT, stride = (int)v.nr * kT;
-  float* bufs[2] = {S.pa, S.pb};
-  int cur = 0;
-  solve_loop(
-      S, a, v, s_red,
-      [&](int todo) {
-        for (int k = 0; k < todo; ++k) {
-          for (int i = begin + tid; i < v.n; i += stride) {
-            const UnitPos p = unit_pos(d, nq, __ldcg(S.list + i));
-            const unsigned f = unit_fluid(d, S.type, p, vec);
-            UnitIn u = gload_unit(d, bufs[cur], p);
-            const Quad r0 = load_cells(S.rhs, p.cell, p.len);
-            update_unit(u, r0, p.two ? load_cells(S.rhs, p.cell + plane, p.len) : r0, sixths(f & 15u),
-                        sixths((f >> 4) & 15u));
-            store_cells(bufs[cur ^ 1], p.cell, p.len, u.a);
-            if (p.two) store_cells(bufs[cur ^ 1], p.cell + plane, p.len, u.b);
-          }
-          cur ^= 1;
-          cluster_sync(v.nr);
-        }
-      },
-      [&]() {
-        for (int i0 = begin + warp * 32; i0 < v.n; i0 += stride) {
-          double acc = 0.0;
-          if (i0 + lane < v.n) {
-            const UnitPos p = unit_pos(d, nq, __ldcg(S.list + i0 + lane));
-            const Quad r0 = load_cells(S.rhs, p.cell, p.len);
-            acc = resid_unit(gload_unit(d, bufs[cur], p), r0,
-                             p.two ? load_cells(S.rhs, p.cell + plane, p.len) : r0, unit_fluid(d, S.type, p, vec));
-          }
-          acc = warp_sum(acc);
-          if (lane == 0) S.part[i0 / 32] = acc;
-        }
-      });
-  if (cur) {
-    for (int i = begin + tid; i < v.n; i += stride) {
-      const UnitPos p = unit_pos(d, nq, __ldcg(S.list + i));
-      store_cells(S.pa, p.cell, p.len, load_cells(S.pb, p.cell, p.len));
-      if (p.two) store_cells(S.pa, p.cell + plane, p.len, load_cells(S.pb, p.cell + plane, p.len));
-    }
-  }
-}
-
 template <bool RAGGED>
 __device__ __forceinline__ void solve_units(const ClusterScene& S, const SolveArgs& a, Solve& v, double* s_red,
                                             unsigned smem) {
@@ -617,8 +549,29 @@ __device__ __forceinline__ void solve_units(const ClusterScene& S, const SolveAr
   else solve_shared<4, RAGGED>(S, a, v, s_red, smem);
 }
 
-// Starts from pa; the result is in pa.
-__device__ __forceinline__ void cluster_solve(const ClusterScene& S, const SolveArgs& a) {
+// The solve's end.  Called out of line, with the running values by address: they
+// then live on the stack between a solve's checks, and the sweeps' registers
+// hold their units without spilling.
+__device__ __noinline__ void record(const ClusterScene& S, const SolveArgs& a, const Solve& v) {
+  if (a.r2_only) {
+    *a.r2_only = v.r2;
+    return;
+  }
+  SolveState* ss = S.ss;
+  ss->iterations = v.it0 + v.done;
+  ss->bodies += v.checks;
+  ss->total_sweeps += v.done;
+  ss->total_bodies += v.checks;
+  ss->r2 = v.r2;
+  ss->rel_residual = v.rel;
+  const bool finite = isfinite(v.rel);
+  if (!finite) ss->nonfinite = ss->nonfinite_seen = 1;
+  ss->converged = finite && v.rel <= a.tol ? 1 : 0;
+}
+
+// Starts from pa; the result is in pa.  False where the fluid does not fit the
+// cluster, which leaves pa and the solve state alone.
+__device__ __forceinline__ bool cluster_solve(const ClusterScene& S, const SolveArgs& a) {
   extern __shared__ __align__(16) unsigned char cl_smem[];
   __shared__ double s_red[kT];
   __shared__ int s_warp[kT / 32];
@@ -681,41 +634,35 @@ __device__ __forceinline__ void cluster_solve(const ClusterScene& S, const Solve
   v.done = v.checks = 0;
   v.r2 = v.rel = -1.0;
   const unsigned smem = static_cast<unsigned>(__cvta_generic_to_shared(cl_smem));
-  if (v.per > kCap) solve_global(S, a, v, s_red);
-  else if (d.sx % 2 || !vec) solve_units<true>(S, a, v, s_red, smem);
-  else solve_units<false>(S, a, v, s_red, smem);
-  if (v.me == 0 && tid == 0 && a.r2_only) {
-    *a.r2_only = v.r2;
-  } else if (v.me == 0 && tid == 0) {
-    SolveState* ss = S.ss;
-    ss->iterations = v.it0 + v.done;
-    ss->bodies += v.checks;
-    ss->total_sweeps += v.done;
-    ss->total_bodies += v.checks;
-    ss->r2 = v.r2;
-    ss->rel_residual = v.rel;
-    const bool finite = isfinite(v.rel);
-    if (!finite) ss->nonfinite = ss->nonfinite_seen = 1;
-    ss->converged = finite && v.rel <= a.tol ? 1 : 0;
+  if (v.per > kCap) {  // the same in every CTA
+    if (v.me == 0 && tid == 0) cudaGraphSetConditional(a.spill, 1);
+    return false;
   }
+  if (d.sx % 2 || !vec) solve_units<true>(S, a, v, s_red, smem);
+  else solve_units<false>(S, a, v, s_red, smem);
+  if (v.me == 0 && tid == 0) record(S, a, v);
+  return true;
 }
 
-__global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__ ClusterScene S, SolveArgs a) {
+__global__ void __launch_bounds__(kT, 1)
+    k_cluster_solve(const __grid_constant__ ClusterScene S, const __grid_constant__ SolveArgs a) {
   cluster_solve(S, a);
 }
 
 // One cluster per scene of a batch: the clusters of the launch take the scenes
-// order[0], order[1], ... (largest first).
+// order[0], order[1], ... (largest first) that are live, and clear the mark of
+// those they solve.
 __global__ void __launch_bounds__(kT, 1) kb_cluster_solve(BatchIndex bi, const int* __restrict__ order,
-                                                        const int2* __restrict__ scratch, float* pa, float* pb,
+                                                        const int2* __restrict__ scratch, int* live, float* pa,
                                                         const float* rhs, const int8_t* type, int* umap, int* list,
-                                                        double* part, SolveState* ss, SolveArgs a) {
+                                                        double* part, SolveState* ss, const __grid_constant__ SolveArgs a) {
   const int s = order[blockIdx.x / cluster_size()];
+  if (!__ldcg(live + s)) return;  // the same in all CTAs of the cluster: none clears it before all have met
   const SceneDesc& D = bi.scenes[s];
   const int2 at = scratch[s];  // the scene's first unit and first residual partial
   const int c = D.c_off;
-  const ClusterScene S{D.d, pa + c, pb + c, rhs + c, type + c, umap + at.x, list + at.x, part + at.y, ss + s};
-  cluster_solve(S, a);
+  const ClusterScene S{D.d, pa + c, rhs + c, type + c, umap + at.x, list + at.x, part + at.y, ss + s};
+  if (cluster_solve(S, a) && cluster_rank() == 0 && threadIdx.x == 0) live[s] = 0;
 }
 
 // Launch configuration of `clusters` clusters of `width` CTAs.
@@ -759,6 +706,8 @@ long long cluster_solve_units(const Dims& d) { return (long long)((d.sx + 1) / 2
 // units rarely holds more than 300 fluid ones.
 int cluster_solve_width(const Dims& d) { return cluster_solve_units(d) <= kSmallUnits ? 1 : 16; }
 
+bool cluster_solve_holds(const Dims& d, int width) { return cluster_solve_units(d) <= (long long)width * kCap; }
+
 bool cluster_solve_takes(const Dims& d, int width) {
   return width >= 1 && width <= 16 && (width & (width - 1)) == 0 &&
          cluster_solve_units(d) <= (long long)width * kT * kScanBits;
@@ -784,35 +733,42 @@ bool cluster_solve_runs(int width) {
   return e == cudaSuccess && alone > 0 && batch > 0;
 }
 
-cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, float* pb, const float* rhs,
+cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, const float* rhs,
                                  const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
-                                 int fixed_sweeps, int check, int max_iters, double tol, double* r2_only) {
+                                 int fixed_sweeps, int check, int max_iters, double tol, double* r2_only,
+                                 unsigned long long spill) {
+  if (!spill && !cluster_solve_holds(d, width)) return cudaErrorInvalidValue;
   if (const cudaError_t e = allow_solve()) return e;
   ClusterLaunch l(st, 1, width);
-  const ClusterScene S{d, pa, pb, rhs, type, umap, list, part, ss};
-  return cudaLaunchKernelEx(&l.lc, k_cluster_solve, S, SolveArgs{fixed_sweeps, check, max_iters, tol, r2_only});
+  const ClusterScene S{d, pa, rhs, type, umap, list, part, ss};
+  return cudaLaunchKernelEx(&l.lc, k_cluster_solve, S,
+                            SolveArgs{fixed_sweeps, check, max_iters, tol, r2_only, spill});
 }
 
 // A batch fills the machine by its number of scenes, so a scene takes the
-// narrowest cluster that holds twice its initial fluid: a fluid that has
-// spread then still fits, and up to kU units to a thread cost a sweep 0.37 us
-// each against 0.45 us for the cluster's barrier.
+// narrowest cluster that holds twice its initial fluid (up to kU units to a
+// thread cost a sweep 0.37 us each against 0.45 us for the cluster's barrier).
+// Where the fluid has spread further the scene's solve goes to a cluster of 16
+// CTAs, and to the sweeps where even that does not hold it: the solve that the
+// scene has alone.
 int batch_cluster_width(const Dims& d, long long particles) {
+  if (!cluster_solve_fits(d, particles)) return 0;
   const long long units = std::min(cluster_solve_units(d), std::max(1LL, 2 * particles / 64));
   for (int w = 1; w <= 16; w *= 2)
-    if (units <= (long long)w * kCap && cluster_solve_takes(d, w)) return w;
+    if ((units <= (long long)w * kCap || w == 16) && cluster_solve_takes(d, w)) return w;
   return 0;
 }
 
 cudaError_t launch_batch_cluster_solve(cudaStream_t st, const BatchIndex& bi, int scenes, int width, const int* order,
-                                       const int2* scratch, float* pa, float* pb, const float* rhs,
+                                       const int2* scratch, int* live, float* pa, const float* rhs,
                                        const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
-                                       int fixed_sweeps, int check, int max_iters, double tol) {
+                                       int fixed_sweeps, int check, int max_iters, double tol,
+                                       unsigned long long spill) {
   if (scenes <= 0) return cudaSuccess;
   if (const cudaError_t e = allow_batch_solve()) return e;
   ClusterLaunch l(st, scenes, width);
-  return cudaLaunchKernelEx(&l.lc, kb_cluster_solve, bi, order, scratch, pa, pb, rhs, type, umap, list, part, ss,
-                            SolveArgs{fixed_sweeps, check, max_iters, tol, nullptr});
+  return cudaLaunchKernelEx(&l.lc, kb_cluster_solve, bi, order, scratch, live, pa, rhs, type, umap, list, part, ss,
+                            SolveArgs{fixed_sweeps, check, max_iters, tol, nullptr, spill});
 }
 
 }  // namespace aqb

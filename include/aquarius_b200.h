@@ -287,7 +287,11 @@ aq_status aq_selfcheck_division(int32_t device, uint64_t* mismatches);
  * sweeps (sz % 4 == 0).  rows = 5: the whole solve in one launch of one
  * thread-block cluster of x_planes (1, 2, 4, 8 or 16) CTAs with the iterate in
  * their shared memory (levels 1, any sz, at most 16384 units of 2 x 1 x 4
- * cells per CTA; the default where the fluid fits).  rows = 8, 16, 32:
+ * cells per CTA; the default where the fluid fits).  A fluid that comes to
+ * touch more units than the CTAs' shared memory holds (2048 each) is swept as by
+ * rows = 3 (sz % 4 == 0) or 16 instead, decided step by step on the device;
+ * steps outside of a graph (aq_fluid_set_graph_mode, aq_fluid_run_stage) sweep
+ * so on every grid of more units.  rows = 8, 16, 32:
  * the temporally blocked kernel with `levels` sweeps (1, 2, 4, 8) per launch
  * over tiles of that many rows and x_planes planes.  Chosen per grid by the
  * tuner; invalid plans are rejected. */
@@ -380,7 +384,8 @@ aq_status aq_batch_solve_stats(aq_batch* b, int32_t scene, aq_solve_stats* st);
 /* Kernel launches per step outside the residual loop, and per loop block, of
  * a step whose solve runs as row sweeps.  When every scene fits a
  * thread-block cluster the step's whole solve is at most five launches (one
- * per cluster size) instead, and no block launches anything. */
+ * per cluster size) instead, one more for the scenes that have outgrown theirs,
+ * and the row sweeps' only for scenes that outgrow that one too. */
 aq_status aq_batch_launch_counts(const aq_batch* b, int32_t* per_step, int32_t* per_block);
 /* Caps every batched launch at multiple x SMs CTAs (default 64, i.e. as many
  * as are resident at once; a batched launch never exceeds one resident wave).

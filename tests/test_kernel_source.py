@@ -43,7 +43,7 @@ def test_a_first_launch_waits_before_it_triggers(kernel):
     assert 0 <= body.find("griddepcontrol.wait") < body.find("griddepcontrol.launch_dependents")
 
 
-@pytest.mark.parametrize("array", ["umap", "list", "part", "pa", "pb"])
+@pytest.mark.parametrize("array", ["umap", "list", "part", "pa"])
 def test_cluster_solve_reads_what_it_writes_through_l2(array):
     """The cluster solve's CTAs exchange these arrays within one launch: the
     read-only path (__ldg) is for data that stays constant for a kernel's life."""
