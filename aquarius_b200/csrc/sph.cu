@@ -110,7 +110,6 @@ struct aq_sph {
   }
 
   // Fluid::simulationStep (Fluid_3D_PBF.cu:489-517, Fluid_3D_PCISPH.cu:424-448)
-  float* planes = nullptr;  // one particle array as planes (made by the first download)
   // neighbour lists of the density pass (null: not kept)
   int *near_count = nullptr, *near_list = nullptr;
 
@@ -416,13 +415,14 @@ aq_status aq_sph_download_state(aq_sph* s, aq_sph_state* st) {
   AQS_CUDA(cudaStreamSynchronize(s->stream));
   const size_t n = (size_t)s->n;
   st->physical_time = s->time;
-  if (n && !s->planes) AQS_TRY(s->alloc(&s->planes, 4 * n));
-  // one array, split into planes on the device; only what is asked for
+  // one array, split into planes on the device; only what is asked for.  The
+  // planes lie in the set of arrays that is not live: the next sort rewrites it.
+  float* const planes = reinterpret_cast<float*>(s->arr[1 - s->cur][A_P]);
   auto get = [&](int role, float* xyz, float* w) -> aq_status {
     if (!n || (!xyz && !w)) return AQ_OK;
-    AQS_CUDA(launch_sph_planes(s->stream, s->A(role), s->planes, s->n));
-    if (xyz) AQS_CUDA(cudaMemcpyAsync(xyz, s->planes, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost, s->stream));
-    if (w) AQS_CUDA(cudaMemcpyAsync(w, s->planes + 3 * n, sizeof(float) * n, cudaMemcpyDeviceToHost, s->stream));
+    AQS_CUDA(launch_sph_planes(s->stream, s->A(role), planes, s->n));
+    if (xyz) AQS_CUDA(cudaMemcpyAsync(xyz, planes, sizeof(float) * 3 * n, cudaMemcpyDeviceToHost, s->stream));
+    if (w) AQS_CUDA(cudaMemcpyAsync(w, planes + 3 * n, sizeof(float) * n, cudaMemcpyDeviceToHost, s->stream));
     return AQ_OK;
   };
   AQS_TRY(get(A_P, st->position, st->rest_density));

@@ -172,3 +172,26 @@ def test_crowded_particles_step_like_the_oracle(method, squeezed):
     a, b = s.get_state(FIELDS[method]), o.get_state(FIELDS[method])
     for f in FIELDS[method]:
         np.testing.assert_array_equal(a[f], b[f], err_msg=f)
+
+
+@pytest.mark.parametrize("method", ["pbf", "pcisph"])
+def test_a_first_read_back_allocates_nothing(method):
+    import torch
+    cfg = _abi.sph_config(METHODS[method], max_particle_count=3000000)
+    with torch.cuda.device(0):
+        other = aq.Sph(cfg)  # the process's first read-back, which loads its kernel
+        other.step(1)
+        want = other.get_state()
+        s = aq.Sph(cfg)
+        s.step(1)
+        s.synchronize()
+        before = torch.cuda.mem_get_info()[0]
+        got = s.get_state()
+        assert torch.cuda.mem_get_info()[0] == before
+        for f in FIELDS[method]:
+            np.testing.assert_array_equal(got[f], want[f], err_msg=f)
+        # and leaves the solver as it was
+        s.step(1)
+        other.step(1)
+        for f in FIELDS[method]:
+            np.testing.assert_array_equal(s.get_state([f])[f], other.get_state([f])[f], err_msg=f)
