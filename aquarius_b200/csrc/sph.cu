@@ -348,12 +348,22 @@ aq_status aq_sph_create(const aq_sph_config* cfg, aq_sph** out) {
   if (st == AQ_OK) st = s->alloc(&s->count, (size_t)s->cells + 1);
   if (st == AQ_OK) st = s->alloc(&s->off, (size_t)s->cells + 1);
   if (st == AQ_OK) st = s->alloc(&s->tiles, cell_scan_tiles(s->cells));
-  // neighbour lists, 260 bytes a particle; without them each pass searches
-  if (st == AQ_OK && n <= kListedParticles) {
-    st = s->alloc(&s->near_count, (size_t)n);
-    if (st == AQ_OK) st = s->alloc(&s->near_list, (size_t)n * kSphList);
-  }
   if (st != AQ_OK) return bail(st);
+  // neighbour lists, 260 bytes a particle; without them (more particles, or no
+  // memory left) each pass searches
+  if (n <= kListedParticles) {
+    void *counts = nullptr, *lists = nullptr;
+    if (cudaMalloc(&counts, std::max<size_t>(sizeof(int) * n, 16)) == cudaSuccess &&
+        cudaMalloc(&lists, std::max<size_t>(sizeof(int) * n * kSphList, 16)) == cudaSuccess) {
+      s->allocs.push_back(counts);
+      s->allocs.push_back(lists);
+      s->near_count = (int*)counts;
+      s->near_list = (int*)lists;
+    } else {
+      cudaGetLastError();
+      cudaFree(counts);
+    }
+  }
   // Particle(float3): position = lastPosition = predictedPosition, velocity 0
   std::vector<float4> h4((size_t)n);
   for (int i = 0; i < n; ++i) h4[i] = make_float4(pos[3 * (size_t)i], pos[3 * (size_t)i + 1], pos[3 * (size_t)i + 2], 0.f);

@@ -195,3 +195,32 @@ def test_a_first_read_back_allocates_nothing(method):
         other.step(1)
         for f in FIELDS[method]:
             np.testing.assert_array_equal(s.get_state([f])[f], other.get_state([f])[f], err_msg=f)
+
+
+@pytest.mark.parametrize("method", ["pbf", "pcisph"])
+def test_without_memory_for_neighbour_lists(method):
+    """A solver that finds memory for its particles but not for the neighbour
+    lists (260 bytes a particle) searches in every pass: the same steps."""
+    import torch
+    cfg = _abi.sph_config(METHODS[method], max_particle_count=10000000)
+    s = aq.Sph(cfg)
+    n, held = s.n, torch.cuda.mem_get_info()[0]
+    s.step(2)
+    want = s.get_state()
+    s.close()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    used = free - held  # with the lists
+    rest = used - 130 * n  # room for all but half of the lists
+    hog = torch.empty(free - rest, dtype=torch.uint8, device="cuda")
+    try:
+        s = aq.Sph(cfg)
+        assert torch.cuda.mem_get_info()[0] >= rest - (used - 250 * n)  # no lists
+        s.step(2)
+        got = s.get_state()
+        s.close()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    for f in FIELDS[method]:
+        np.testing.assert_array_equal(got[f], want[f], err_msg=f)
