@@ -481,8 +481,9 @@ struct RenderTri {
   int tl;
 };
 
+// *mixed (0 before) becomes nonzero if a fraction is neither 0 nor 1.
 cudaError_t launch_sprite_setup(cudaStream_t st, const RenderParams& P, const float* pts, int n, float4* spr,
-                                float4* frac, int* cnt, unsigned long long* total);
+                                float4* frac, int* cnt, unsigned long long* total, unsigned long long* mixed);
 cudaError_t launch_sprite_emit(cudaStream_t st, const RenderParams& P, const float4* spr, const int* off, int n,
                                unsigned* keys, int* vals);
 cudaError_t launch_tri_setup(cudaStream_t st, const RenderParams& P, const float* mesh, int ntri, RenderTri* tris,

@@ -421,11 +421,16 @@ __device__ __forceinline__ int block_x(int tx, int warp) { return tx * kT + (war
 __device__ __forceinline__ int block_y(int ty, int warp) { return ty * kT + (warp >> 1) * 4; }
 
 // ---------------------------------------------------------------- kernels
+// A fraction of a point whose phases have mixed.
+__device__ __forceinline__ bool partial_fraction(float f) { return !(f == 0.0f || f == 1.0f); }
+
 __global__ void __launch_bounds__(256) k_sprite_setup(RenderParams P, const float* __restrict__ pts, int n,
                                                       float4* __restrict__ spr, float4* __restrict__ frac,
-                                                      int* __restrict__ cnt, unsigned long long* __restrict__ total) {
+                                                      int* __restrict__ cnt, unsigned long long* __restrict__ total,
+                                                      unsigned long long* __restrict__ mixed) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   int c = 0;
+  bool part = false;
   if (i < n) {
     const float* p = pts + (size_t)i * 7;
     float4 s;
@@ -433,10 +438,13 @@ __global__ void __launch_bounds__(256) k_sprite_setup(RenderParams P, const floa
     if (sprite_setup(P, p, s) && sprite_pixels(s, P.W, P.H, i0, i1, j0, j1)) {
       c = tiles_of<kS>(i0, i1, j0, j1);
       spr[i] = s;
-      frac[i] = make_float4(p[3], p[4], p[5], p[6]);
+      const float4 f = make_float4(p[3], p[4], p[5], p[6]);
+      frac[i] = f;
+      part = partial_fraction(f.x) || partial_fraction(f.y) || partial_fraction(f.z) || partial_fraction(f.w);
     }
     cnt[i] = c;
   }
+  if (__syncthreads_or(part) && threadIdx.x == 0 && !__ldcg(mixed)) atomicExch(mixed, 1ull);
   unsigned long long v = (unsigned long long)c;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
@@ -631,7 +639,7 @@ __global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const fl
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         const float v = p[3 + k];
-        bad |= !(v == 0.0f || v == 1.0f);
+        bad |= partial_fraction(v);
         f[k] = v == 1.0f ? 1u : 0u;
       }
       add01 = f[0] | (f[1] << 16);
@@ -874,9 +882,9 @@ __global__ void __launch_bounds__(256) k_points_vbo(Particles cur, int n, int ph
 }  // namespace
 
 cudaError_t launch_sprite_setup(cudaStream_t st, const RenderParams& P, const float* pts, int n, float4* spr,
-                                float4* frac, int* cnt, unsigned long long* total) {
+                                float4* frac, int* cnt, unsigned long long* total, unsigned long long* mixed) {
   if (n <= 0) return cudaSuccess;
-  k_sprite_setup<<<(n + 255) / 256, 256, 0, st>>>(P, pts, n, spr, frac, cnt, total);
+  k_sprite_setup<<<(n + 255) / 256, 256, 0, st>>>(P, pts, n, spr, frac, cnt, total, mixed);
   return cudaGetLastError();
 }
 

@@ -128,6 +128,7 @@ struct aq_renderer {
   unsigned long long* totals_host = nullptr;
   int launches = 0;
   int last_w = 0, last_h = 0;
+  bool mixed = false;  // the last frame with a phase thickness met a fraction that is neither 0 nor 1
 
   ~aq_renderer() {
     if (device >= 0) cudaSetDevice(device);
@@ -360,8 +361,9 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
   AQR_CUDA(cudaMemsetAsync(r->totals.p, 0, 3 * sizeof(unsigned long long), st));
   AQR_CUDA(cudaMemsetAsync(r->srange.p, 0, sizeof(int2) * nstiles, st));
   AQR_CUDA(cudaMemsetAsync(r->trange.p, 0, sizeof(int2) * ntiles, st));
-  // the phase thickness by counting, unless phases have mixed
-  bool splat = P.use_phase && n_points <= kSplatPoints;
+  // the phase thickness by counting, unless phases have mixed (the last frame's
+  // tells where to start: a frame finds out for itself either way)
+  bool splat = P.use_phase && n_points <= kSplatPoints && !r->mixed;
   if (splat) {
     AQR_CUDA(cudaMemsetAsync(r->phase.p, 0, sizeof(float4) * npx, st));
     AQR_CUDA(launch_phase_splat(st, P, points, n_points, r->phase.p, r->totals.p + 2));
@@ -375,7 +377,8 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
     AQR_TRY(r->soff.ensure(n + 1));
     AQR_TRY(r->sscan.ensure(cell_scan_tiles(n_points)));
     AQR_CUDA(cudaMemsetAsync(r->scnt.p + n, 0, sizeof(int), st));
-    AQR_CUDA(launch_sprite_setup(st, P, points, n_points, r->spr.p, r->frac.p, r->scnt.p, r->totals.p));
+    AQR_CUDA(launch_sprite_setup(st, P, points, n_points, r->spr.p, r->frac.p, r->scnt.p, r->totals.p,
+                                 r->totals.p + 2));
     AQR_CUDA(launch_cell_scan(st, n_points, r->scnt.p, r->soff.p, r->sscan.p));
     r->launches += 4;
     return AQ_OK;
@@ -405,7 +408,8 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
   }
   if (need_spr || need_tri) {
     AQR_TRY(read_totals());
-    if (splat && r->totals_host[2]) {
+    if (P.use_phase) r->mixed = r->totals_host[2] != 0;
+    if (splat && r->mixed) {
       splat = false;
       AQR_TRY(sprites());
       AQR_TRY(read_totals());

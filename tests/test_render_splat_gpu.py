@@ -60,3 +60,24 @@ def test_counted_thickness_equals_the_ordered_sums(n, phases, shuffled, radius, 
     _, want2 = RenderOracle().frame(dc, pts2, None)
     np.testing.assert_array_equal(got2, want2)
     r.close()
+
+
+def test_frames_of_mixed_phases_start_with_the_lists():
+    """A renderer whose last frame met mixed phases does not count first: that
+    frame launches less than the first of its kind, and one whose phases are
+    apart again shows the same texture on either path."""
+    apart, mixed = _points(5000, 1, 4, False), _points(5000, 1, 4, False)
+    mixed[7, 3:] = (0.25, 0.75, 0.0, 0.0)
+    dc = aq.draw_command_default(320, 160, 10.0, 32)
+    dc.render_mode = _abi.RENDER_MULTIPHASE_MESH
+    r = aq.Renderer(0)
+    launches, got = [], []
+    for pts in (apart, mixed, mixed, apart, apart):
+        got.append(_draw(r, dc, pts, None)[1])
+        launches.append(r.launches())
+    r.close()
+    for k, pts in ((0, apart), (1, mixed)):
+        np.testing.assert_array_equal(got[k], RenderOracle().frame(dc, pts, None)[1])
+    for k, same in ((2, 1), (3, 0), (4, 0)):
+        np.testing.assert_array_equal(got[k], got[same])
+    assert launches[2] < launches[1] and launches[3] == launches[2] and launches[4] == launches[0]
