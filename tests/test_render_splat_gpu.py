@@ -81,3 +81,21 @@ def test_frames_of_mixed_phases_start_with_the_lists():
     for k, same in ((2, 1), (3, 0), (4, 0)):
         np.testing.assert_array_equal(got[k], got[same])
     assert launches[2] < launches[1] and launches[3] == launches[2] and launches[4] == launches[0]
+
+
+@pytest.mark.parametrize("n", [300, 20000])
+def test_large_sprites_take_the_lists(n):
+    """Counting visits every pixel of a sprite, the lists every 8 x 8 tile: from
+    some 20 pixels a side on the lists are faster.  The same texture."""
+    pts = _points(n, n, 2, False)
+    dc = aq.draw_command_default(640, 320, 10.0, 32)
+    dc.render_mode = _abi.RENDER_MULTIPHASE_MESH
+    launches = []
+    r = aq.Renderer(0)
+    for radius in (0.1, 3.0):  # 2 and 64 pixels a side
+        dc.point_radius = radius
+        _, got = _draw(r, dc, pts, None)
+        launches.append(r.launches())
+        np.testing.assert_array_equal(got, RenderOracle().frame(dc, pts, None)[1])
+    r.close()
+    assert launches[0] < launches[1]
