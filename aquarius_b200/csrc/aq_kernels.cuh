@@ -504,10 +504,11 @@ cudaError_t launch_phase(cudaStream_t st, const RenderParams& P, const int2* ran
                          const int* vals, const float4* spr, const float4* frac, float4* phase);
 // The same pass by counting, where every fraction is 0 or 1: adds to a zeroed
 // phase texture; *mixed (0 before) becomes nonzero if some fraction is neither,
-// and the texture is then void.  At most 2^24 points.
+// and the texture is then void.  At most 2^24 points; *total counts their
+// sprite-tile pairs, which a frame's limit is on whichever path it takes.
 constexpr int kSplatPoints = 1 << 24;
 cudaError_t launch_phase_splat(cudaStream_t st, const RenderParams& P, const float* pts, int n, float4* phase,
-                               unsigned long long* mixed);
+                               unsigned long long* total, unsigned long long* mixed);
 // load[t] = list length of sprite tile t, ids[t] = t
 cudaError_t launch_tile_load(cudaStream_t st, const int2* range, int n, unsigned* load, int* ids);
 cudaError_t launch_frame(cudaStream_t st, const RenderParams& P, const RenderTri* ctris, const int* clive,

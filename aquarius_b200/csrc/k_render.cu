@@ -618,13 +618,15 @@ __global__ void __launch_bounds__(64) k_phase(RenderParams P, const int2* __rest
 constexpr int kSplat = 512, kSplatBox = 5120;  // pixels; two words each
 __global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const float* __restrict__ pts, int n,
                                                        float* __restrict__ phase,
+                                                       unsigned long long* __restrict__ total,
                                                        unsigned long long* __restrict__ mixed) {
   __shared__ unsigned s_cnt[2][kSplatBox];  // phases 0, 1 and 2, 3 in 16-bit halves
-  __shared__ int s_box[4];
+  __shared__ int s_box[4], s_pairs;
   const int tid = threadIdx.x, i = blockIdx.x * kSplat + tid;
   if (tid == 0) {
     s_box[0] = s_box[2] = INT_MAX;
     s_box[1] = s_box[3] = -1;
+    s_pairs = 0;
   }
   // another CTA may set the flag at any time: one thread's look decides for all
   if (__syncthreads_or(tid == 0 && __ldcg(mixed) != 0)) return;
@@ -632,9 +634,11 @@ __global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const fl
   int i0 = 0, i1 = -1, j0 = 0, j1 = -1;
   unsigned add01 = 0, add23 = 0;
   bool bad = false;
+  int pairs = 0;
   if (i < n) {
     const float* p = pts + (size_t)i * 7;
     if (sprite_setup(P, p, s) && sprite_pixels(s, P.W, P.H, i0, i1, j0, j1)) {
+      pairs = tiles_of<kS>(i0, i1, j0, j1);
       unsigned f[4];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
@@ -657,13 +661,16 @@ __global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const fl
   const unsigned all = 0xffffffffu;
   const int bi0 = __reduce_min_sync(all, draws ? i0 : INT_MAX), bi1 = __reduce_max_sync(all, draws ? i1 : -1);
   const int bj0 = __reduce_min_sync(all, draws ? j0 : INT_MAX), bj1 = __reduce_max_sync(all, draws ? j1 : -1);
+  const int tiles = __reduce_add_sync(all, pairs);
   if ((tid & 31) == 0) {
+    atomicAdd(&s_pairs, tiles);
     atomicMin(&s_box[0], bi0);
     atomicMax(&s_box[1], bi1);
     atomicMin(&s_box[2], bj0);
     atomicMax(&s_box[3], bj1);
   }
   const int second = __syncthreads_or(add23 != 0);
+  if (tid == 0 && s_pairs) atomicAdd(total, (unsigned long long)s_pairs);
   const int ox = s_box[0], oy = s_box[2], w = s_box[1] - ox + 1, h = s_box[3] - oy + 1;
   if (s_box[1] < 0) return;  // nothing to draw
   const bool local = (long long)w * h <= kSplatBox;
@@ -927,9 +934,10 @@ cudaError_t launch_phase(cudaStream_t st, const RenderParams& P, const int2* ran
 }
 
 cudaError_t launch_phase_splat(cudaStream_t st, const RenderParams& P, const float* pts, int n, float4* phase,
-                               unsigned long long* mixed) {
+                               unsigned long long* total, unsigned long long* mixed) {
   if (n <= 0) return cudaSuccess;
-  k_phase_splat<<<(n + kSplat - 1) / kSplat, kSplat, 0, st>>>(P, pts, n, reinterpret_cast<float*>(phase), mixed);
+  k_phase_splat<<<(n + kSplat - 1) / kSplat, kSplat, 0, st>>>(P, pts, n, reinterpret_cast<float*>(phase), total,
+                                                               mixed);
   return cudaGetLastError();
 }
 

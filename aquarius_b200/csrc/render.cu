@@ -380,7 +380,7 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
   bool splat = P.use_phase && n_points <= kSplatPoints && !r->mixed && counting_pays(P, n_points);
   if (splat) {
     AQR_CUDA(cudaMemsetAsync(r->phase.p, 0, sizeof(float4) * npx, st));
-    AQR_CUDA(launch_phase_splat(st, P, points, n_points, r->phase.p, r->totals.p + 2));
+    AQR_CUDA(launch_phase_splat(st, P, points, n_points, r->phase.p, r->totals.p, r->totals.p + 2));
     ++r->launches;
   }
   auto sprites = [&]() -> aq_status {
@@ -425,6 +425,7 @@ aq_status aq_renderer_draw(aq_renderer* r, const aq_draw_command* dc, const floa
     if (P.use_phase) r->mixed = r->totals_host[2] != 0;
     if (splat && r->mixed) {
       splat = false;
+      AQR_CUDA(cudaMemsetAsync(r->totals.p, 0, sizeof(unsigned long long), st));  // counted anew
       AQR_TRY(sprites());
       AQR_TRY(read_totals());
     }

@@ -99,3 +99,27 @@ def test_large_sprites_take_the_lists(n):
         np.testing.assert_array_equal(got, RenderOracle().frame(dc, pts, None)[1])
     r.close()
     assert launches[0] < launches[1]
+
+
+def test_too_many_sprite_tile_pairs_are_refused():
+    """2^24 sprites of over 128 tiles each, close to the camera: more pairs than
+    a frame takes, also where the thickness is counted."""
+    import torch
+    dc = aq.draw_command_default(1728, 864, 10.0, 128)
+    dc.render_mode = _abi.RENDER_MULTIPHASE_MESH
+    dc.point_radius = 0.2  # 11.6 pixels a side at the container's centre, 18 away; 119 at 1.75
+    cam = np.array(list(dc.camera_position))
+    at = cam + (5.0 - cam) / np.linalg.norm(5.0 - cam) * 1.75
+    pts = torch.zeros(1 << 24, 7, device="cuda")
+    pts[:, :3] = torch.tensor(at, dtype=torch.float32)
+    pts[:, 3] = 1.0
+    torch.cuda.synchronize()
+    r = aq.Renderer(0)
+    with pytest.raises(aq.AquariusError, match="primitive-tile pairs"):
+        r.draw(dc, pts.data_ptr(), pts.shape[0], 0, 0)
+    few = pts[:100000].contiguous()
+    torch.cuda.synchronize()
+    r.draw(dc, few.data_ptr(), few.shape[0], 0, 0)
+    r.synchronize()
+    assert r.phase_thickness().max() == 100000.0
+    r.close()
