@@ -43,6 +43,31 @@ __device__ __forceinline__ void p2g_particle(int DX, int DY, int DZ, float qx, f
   bxyz = __fmul_rn(__fmul_rn(bx, by), bz);
 }
 
+// p2g_particle with the x factors already evaluated: ax = hat1(qx - fx) and
+// bx = hat1(qx - fxh), the same values (a staged plane shares the node x).
+__device__ __forceinline__ void p2g_particle_x(int DX, int DY, int DZ, float ax, float bx, float qy, float qz,
+                                               float vx, float vy, float vz, float fy, float fz, float fyh,
+                                               float fzh, float& su, float& sv, float& sw, float& wu, float& wv,
+                                               float& ww, float& bxyz) {
+  const float by = hat1(__fsub_rn(qy, fyh)), bz = hat1(__fsub_rn(qz, fzh));
+  if (DX < 1) {
+    const float w = __fmul_rn(__fmul_rn(ax, by), bz);
+    su = __fmaf_rn(w, vx, su);
+    wu = __fadd_rn(wu, w);
+  }
+  if (DY < 1) {
+    const float w = __fmul_rn(__fmul_rn(bx, hat1(__fsub_rn(qy, fy))), bz);
+    sv = __fmaf_rn(w, vy, sv);
+    wv = __fadd_rn(wv, w);
+  }
+  if (DZ < 1) {
+    const float w = __fmul_rn(__fmul_rn(bx, by), hat1(__fsub_rn(qz, fz)));
+    sw = __fmaf_rn(w, vz, sw);
+    ww = __fadd_rn(ww, w);
+  }
+  bxyz = __fmul_rn(__fmul_rn(bx, by), bz);
+}
+
 // The fractions' weighted sum of the node's own cell (transferVolumeFractionsToCell).
 __device__ __forceinline__ void p2g_fractions(float w, const float4& f, float4& fs, float& fw) {
   fs.x = __fmaf_rn(w, f.x, fs.x);
@@ -417,6 +442,123 @@ __global__ void __launch_bounds__(kP2gThreads, kP2gSlots <= 7 ? 6 : (kP2gSlots <
     a.own = own; a.left = left1; a.down = down; a.back = back;
     left1 = own;
   }
+}
+
+// The same gather for grids of few CTAs: a CTA owns the nodes of one x plane, 8 y
+// rows and 32 z columns, one per thread, and stages the three planes it reads one
+// after the other (10 rows of 34 cells, a thread its cells' particles).  A slot
+// holds the particle's two x hat factors (the CTA's nodes share one x), its y and
+// z in cell units and its velocity.  Where every CTA has an SM to itself the
+// time is a chain of three stagings and sums, and twice the threads to a CTA
+// shorten it against a chunk of one plane above (us, this / that: 16^3 27.3 /
+// 29.2, 20^3 27.2 / 31.2, 32^3 33.3 / 35.2); where some SMs get two CTAs the
+// marching kernel is ahead (48 x 32 x 32 42.6 / 36.1).
+constexpr int kTileY = 8, kTileCells = kP2gCols * (kTileY + 2);
+constexpr int p2g_tile_smem(int slots) { return 7 * slots * kTileCells * (int)sizeof(float); }
+
+template <bool FORCES, bool MULTI, int kP2gSlots>
+__global__ void __launch_bounds__(256, kP2gSlots <= 7 ? 3 : (kP2gSlots <= 11 ? 2 : 1))
+    k_p2g_tiled(Dims d, StepParams sp, Particles cur, const int* __restrict__ off, float* __restrict__ u0,
+                float* __restrict__ v0, float* __restrict__ w0, float* __restrict__ un, float* __restrict__ vn,
+                float* __restrict__ wn, int8_t* __restrict__ type, float* __restrict__ density,
+                float4* __restrict__ vf, float4* __restrict__ nvf) {
+  // hat1(qx - fx), hat1(qx - fxh), qy, qz, vx, vy, vz: [kP2gSlots][kTileCells] each (the x
+  // factors are per particle: the CTA's nodes share one x)
+  extern __shared__ float p2g_sm[];
+  __shared__ int s_beg[kTileCells], s_cnt[kTileCells];
+  constexpr int A = kP2gSlots * kTileCells;
+  float* const sax = p2g_sm;
+  float* const sbx = sax + A;
+  float* const sqy = sbx + A;
+  float* const sqz = sqy + A;
+  float* const svx = sqz + A;
+  float* const svy = svx + A;
+  float* const svz = svy + A;
+  const int lane = threadIdx.x, wy = threadIdx.y, tid = wy * 32 + lane;
+  const int z0 = blockIdx.x * 32, y0 = blockIdx.y * kTileY, x = blockIdx.z;
+  const int z = z0 + lane, y = y0 + wy;
+  const bool node = z < d.sz && y < d.sy;
+  const float fx = (float)x, fy = (float)y, fz = (float)z;
+  const float fxh = fx + 0.5f, fyh = fy + 0.5f, fzh = fz + 0.5f;
+  const float inv_h = d.inv_h;
+  float su = 0.f, sv = 0.f, sw = 0.f, wu = 0.f, wv = 0.f, ww = 0.f;
+  float4 fs = make_float4(0.f, 0.f, 0.f, 0.f);
+  float fw = 0.f;
+  int own = 0, left = 0, down = 0, back = 0;
+#pragma unroll
+  for (int dx = -1; dx <= 1; ++dx) {
+    const int X = x + dx;
+    if (X < 0 || X >= d.sx) continue;  // the same for the whole CTA
+    __syncthreads();                   // the previous plane's slots are consumed
+    for (int lc = tid; lc < kTileCells; lc += 256) {
+      const int Y = y0 - 1 + lc / kP2gCols, Z = z0 - 1 + lc % kP2gCols;
+      int b = 0, n = 0;
+      if (Y >= 0 && Y < d.sy && Z >= 0 && Z < d.sz) {
+        const int c = (X * d.sy + Y) * d.sz + Z;
+        b = __ldg(off + c);
+        n = __ldg(off + c + 1) - b;
+      }
+      s_beg[lc] = b;
+      s_cnt[lc] = n;
+      const int m = min(n, kP2gSlots);
+      for (int k = 0; k < m; ++k) {
+        const int j = b + k, sl = k * kTileCells + lc;
+        const float qx = __fmul_rn(__ldg(cur.px + j), inv_h);
+        sax[sl] = hat1(__fsub_rn(qx, fx));
+        sbx[sl] = hat1(__fsub_rn(qx, fxh));
+        sqy[sl] = __fmul_rn(__ldg(cur.py + j), inv_h);
+        sqz[sl] = __fmul_rn(__ldg(cur.pz + j), inv_h);
+        svx[sl] = __ldg(cur.vx + j);
+        svy[sl] = __ldg(cur.vy + j);
+        svz[sl] = __ldg(cur.vz + j);
+      }
+    }
+    __syncthreads();
+    if (!node) continue;
+    // dy and dz stay loops (the branches on them are uniform across the
+    // warp): 27 unrolled copies of the particle loop overflow the
+    // instruction cache
+#pragma unroll 1
+    for (int dy = -1; dy <= 1; ++dy) {
+      const int Y = y + dy;
+      if (Y < 0 || Y >= d.sy) continue;
+#pragma unroll 1
+      for (int dz = -1; dz <= 1; ++dz) {
+        const int Z = z + dz;
+        if (Z < 0 || Z >= d.sz) continue;
+        const int lc = (wy + 1 + dy) * kP2gCols + lane + 1 + dz;
+        const int b = s_beg[lc], n = s_cnt[lc];
+        if (dx == 0 && dy == 0 && dz == 0) own = n;
+        if (dx == -1 && dy == 0 && dz == 0) left = n;
+        if (dx == 0 && dy == -1 && dz == 0) down = n;
+        if (dx == 0 && dy == 0 && dz == -1) back = n;
+        const int m = min(n, kP2gSlots);
+        for (int k = 0; k < m; ++k) {  // the staged slots
+          const int sl = k * kTileCells + lc;
+          float bxyz;
+          p2g_particle_x(dx, dy, dz, sax[sl], sbx[sl], sqy[sl], sqz[sl], dx < 1 ? svx[sl] : 0.f,
+                         dy < 1 ? svy[sl] : 0.f, dz < 1 ? svz[sl] : 0.f, fy, fz, fyh, fzh, su, sv, sw, wu, wv, ww,
+                         bxyz);
+          if (MULTI && dx == 0 && dy == 0 && dz == 0) p2g_fractions(bxyz, cur.frac[b + k], fs, fw);
+        }
+        for (int k = m; k < n; ++k) {  // a crowded cell's particles beyond the slots
+          const int j = b + k;
+          float bxyz;
+          p2g_particle(dx, dy, dz, __fmul_rn(__ldg(cur.px + j), inv_h), __fmul_rn(__ldg(cur.py + j), inv_h),
+                       __fmul_rn(__ldg(cur.pz + j), inv_h), dx < 1 ? __ldg(cur.vx + j) : 0.f,
+                       dy < 1 ? __ldg(cur.vy + j) : 0.f, dz < 1 ? __ldg(cur.vz + j) : 0.f, fx, fy, fz, fxh, fyh, fzh,
+                       su, sv, sw, wu, wv, ww, bxyz);
+          if (MULTI && dx == 0 && dy == 0 && dz == 0) p2g_fractions(bxyz, cur.frac[j], fs, fw);
+        }
+      }
+    }
+  }
+  if (!node) return;
+  P2gAcc a;
+  a.su = su; a.sv = sv; a.sw = sw; a.wu = wu; a.wv = wv; a.ww = ww;
+  a.fs = fs; a.fw = fw;
+  a.own = own; a.left = left; a.down = down; a.back = back;
+  p2g_finish<FORCES, MULTI>(d, sp, x, y, z, a, u0, v0, w0, un, vn, wn, type, density, vf, nvf);
 }
 
 // node-grid virtual block -> (z block, y block, x plane) of one scene
@@ -970,7 +1112,8 @@ int p2g_variant() { return g_p2g_variant; }
 // over its air finish at once).  1400 CTAs or more are kept, at most 5 planes.
 // P2G in us at 1, 2, 3, 5 planes: 50^3 (1300 columns x planes) 50, 62, 65, 84;
 // 90 x 61 x 75 (4320) 130, 112, 93, 115; multiphase 96^3 (6912) 248, 201, 183,
-// 172; 128^3 (16384) 515, 334, 291, 267 and no better with more.
+// 172; 128^3 (16384) 515, 334, 291, 267 and no better with more.  Grids of at
+// most 148 CTAs of 8 rows take k_p2g_tiled.
 static int p2g_planes(const Dims& d) {
   const long long ctas = (long long)((d.sz + 31) / 32) * ((d.sy + kP2gY - 1) / kP2gY) * d.sx;
   return (int)std::min(std::max((ctas + 700) / 1400, 1LL), 5LL);
@@ -980,10 +1123,18 @@ template <bool F, bool M, int SLOTS>
 static cudaError_t launch_p2g_slots(cudaStream_t st, const Dims& d, const StepParams& sp, Particles cur,
                                     const int* off, float* u0, float* v0, float* w0, float* un, float* vn,
                                     float* wn, int8_t* type, float* density, float4* vf, float4* nvf) {
+  if (const dim3 tiles = node_grid(d); (long long)tiles.x * tiles.y * tiles.z <= 148) {
+    static_assert(kTileY == 8, "the node grid's rows");
+    constexpr int smem = p2g_tile_smem(SLOTS);
+    cudaError_t e = cudaFuncSetAttribute(k_p2g_tiled<F, M, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    k_p2g_tiled<F, M, SLOTS><<<tiles, dim3(32, kTileY), smem, st>>>(d, sp, cur, off, u0, v0, w0, un, vn, wn, type,
+                                                                    density, vf, nvf);
+    return cudaGetLastError();
+  }
   constexpr int smem = p2g_smem(SLOTS);
   cudaError_t e = cudaFuncSetAttribute(k_p2g_march<F, M, SLOTS>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   if (e != cudaSuccess) return e;
-  const int tiles = ((d.sz + 31) / 32) * ((d.sy + kP2gY - 1) / kP2gY);
   const int planes = p2g_planes(d);
   const dim3 grid((d.sz + 31) / 32, (d.sy + kP2gY - 1) / kP2gY, (d.sx + planes - 1) / planes);
   k_p2g_march<F, M, SLOTS><<<grid, dim3(32, kP2gY), smem, st>>>(d, sp, cur, off, u0, v0, w0, un, vn, wn, type, density,

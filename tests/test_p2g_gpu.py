@@ -110,3 +110,33 @@ def test_staged_p2g_chunks_of_planes(size, multi):
         _variant(1)
     for k in P2G_FIELDS:
         np.testing.assert_array_equal(b[k], a[k], err_msg=k)
+
+
+@pytest.mark.parametrize("multi", [False, True])
+@pytest.mark.parametrize("size", [(37, 29, 30), (38, 29, 30), (40, 40, 40)])
+def test_staged_p2g_at_the_line_of_the_small_grids(size, multi):
+    """148 CTAs of 8 rows, which take the small grids' kernel, four more, which
+    march in chunks of one plane, and crowded cells in both."""
+    cfg = ball_drop(size, pool=0.3, center=(0.5, 0.7, 0.5), radius=0.15, dt=0.005, phase_ball=1 if multi else 0,
+                    pressure_iterations=20)
+    st = _state(cfg, 1)
+    pos = st["position"].copy()
+    h = cfg.domain_size / cfg.size_y
+    rng = np.random.default_rng(1)
+    for first, count, cell in ((0, 40, (10, 3, 12)), (100, 13, (size[0] - 1, 0, size[2] - 1))):
+        for k in range(3):
+            pos[k, first:first + count] = (cell[k] + rng.uniform(0.05, 0.95, count)) * h
+    with aq.Fluid(cfg) as f:
+        f.upload_state(dict(st, position=pos))
+        f.run_stage(_abi.STAGE_SORT)
+        st = f.download_state()
+    try:
+        _variant(0)
+        a = _p2g(cfg, st)
+        for v in (2, 3, 1):
+            _variant(v)
+            b = _p2g(cfg, st)
+            for k in P2G_FIELDS:
+                np.testing.assert_array_equal(b[k], a[k], err_msg=f"{v} {k}")
+    finally:
+        _variant(1)
