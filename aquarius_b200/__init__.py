@@ -103,6 +103,9 @@ def load_library() -> ct.CDLL:
         "aq_batch_download_scene": (ct.c_int, [P, ct.c_int32, ct.POINTER(_abi.HostState)]),
         "aq_batch_solve_stats": (ct.c_int, [P, ct.c_int32, ct.POINTER(_abi.SolveStats)]),
         "aq_batch_launch_counts": (ct.c_int, [P, ct.POINTER(ct.c_int32), ct.POINTER(ct.c_int32)]),
+        "aq_batch_step_launches": (ct.c_int, [P, ct.POINTER(ct.c_int32)]),
+        "aq_batch_set_cluster_solve": (ct.c_int, [P, ct.c_int32]),
+        "aq_batch_get_cluster_solve": (ct.c_int, [P, ct.POINTER(ct.c_int32)]),
         "aq_batch_set_grid_multiple": (ct.c_int, [P, ct.c_int32]),
         "aq_batch_set_sweep_plan": (ct.c_int, [P, ct.c_int32, ct.c_int32]),
         "aq_batch_get_sweep_plan": (ct.c_int, [P, ct.POINTER(ct.c_int32), ct.POINTER(ct.c_int32)]),
@@ -746,6 +749,22 @@ class Batch:
         a, b = ct.c_int32(), ct.c_int32()
         _check(self._lib.aq_batch_launch_counts(self._h, ct.byref(a), ct.byref(b)))
         return a.value, b.value
+
+    def step_launches(self) -> int:
+        """Kernel launches of a step as it runs, outside its conditional parts."""
+        n = ct.c_int32()
+        _check(self._lib.aq_batch_step_launches(self._h, ct.byref(n)))
+        return n.value
+
+    def set_cluster_solve(self, clusters: bool):
+        """True (default where every scene fits): one thread-block cluster a scene;
+        False: row sweeps."""
+        _check(self._lib.aq_batch_set_cluster_solve(self._h, 1 if clusters else 0))
+
+    def cluster_solve(self) -> bool:
+        n = ct.c_int32()
+        _check(self._lib.aq_batch_get_cluster_solve(self._h, ct.byref(n)))
+        return bool(n.value)
 
     def set_grid_multiple(self, multiple: int):
         _check(self._lib.aq_batch_set_grid_multiple(self._h, multiple))

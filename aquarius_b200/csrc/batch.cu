@@ -82,7 +82,9 @@ struct aq_batch {
   // in a cluster of 16 CTAs, or else by the row sweeps (cl_spill, cl_spill16:
   // some scene can come to that).
   static constexpr int kWidths = 5;  // 1, 2, 4, 8, 16 CTAs
-  bool clusters = false, cl_spill = false, cl_spill16 = false;
+  bool cl_planned = false;  // every scene fits a cluster
+  bool clusters = false;    // and is solved in it
+  bool cl_spill = false, cl_spill16 = false;
   int cl_first[kWidths + 1] = {0};
   int* cl_order = nullptr;
   int2* cl_scratch = nullptr;
@@ -112,7 +114,8 @@ struct aq_batch {
   cudaGraphExec_t exec_sort = nullptr, exec_rest = nullptr;
   cudaStream_t copy = nullptr;
   cudaEvent_t sorted = nullptr, copied = nullptr;
-  int graph_launches = 0, body_launches = 0;
+  int graph_launches = 0, body_launches = 0;  // of a step of row sweeps
+  int step_launches = 0;                      // of a step as it runs, outside conditional nodes
   std::vector<void*> allocs;
 
   ~aq_batch() {
@@ -256,7 +259,7 @@ aq_status aq_batch::plan_clusters() {
   AQB_CUDA(cudaMemcpyAsync(cl_order, order.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, stream));
   AQB_CUDA(cudaMemcpyAsync(cl_scratch, scratch.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, stream));
   AQB_CUDA(cudaStreamSynchronize(stream));
-  clusters = true;
+  cl_planned = clusters = true;
   return AQ_OK;
 }
 
@@ -437,6 +440,13 @@ aq_status aq_batch::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
     cudaGraphNode_t node;
     cudaGraph_t body;
     const bool solve = residual || K > 0;
+    step_launches = pre_launches + post_launches;
+    if (clusters) {
+      step_launches -= 1;  // no row list
+      for (int k = 0; k < kWidths && solve; ++k) step_launches += cl_first[k + 1] > cl_first[k] ? 1 : 0;
+    } else if (!residual) {
+      step_launches = graph_launches;
+    }
     if (solve && clusters && !cl_spill) {
       return capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
         AQB_TRY(before_solve());
@@ -765,6 +775,30 @@ aq_status aq_batch_launch_counts(const aq_batch* b, int32_t* per_step, int32_t* 
   if (!b->exec) AQB_TRY(const_cast<aq_batch*>(b)->build_graph());
   if (per_step) *per_step = b->graph_launches;
   if (per_block) *per_block = b->body_launches;
+  return AQ_OK;
+}
+
+aq_status aq_batch_step_launches(const aq_batch* b, int32_t* launches) {
+  if (!b || !launches) return fail(AQ_ERR_INVALID_ARGUMENT, "bad argument");
+  if (!b->exec) AQB_TRY(const_cast<aq_batch*>(b)->build_graph());
+  *launches = b->step_launches;
+  return AQ_OK;
+}
+
+aq_status aq_batch_set_cluster_solve(aq_batch* b, int32_t clusters) {
+  if (!b) return fail(AQ_ERR_INVALID_ARGUMENT, "batch is NULL");
+  if (clusters && !b->cl_planned)
+    return fail(AQ_ERR_INVALID_ARGUMENT, "a scene of the batch does not fit a thread-block cluster");
+  cudaSetDevice(b->device);
+  AQB_CUDA(cudaStreamSynchronize(b->stream));
+  b->clusters = clusters != 0;
+  b->invalidate_graph();
+  return AQ_OK;
+}
+
+aq_status aq_batch_get_cluster_solve(const aq_batch* b, int32_t* clusters) {
+  if (!b || !clusters) return fail(AQ_ERR_INVALID_ARGUMENT, "bad argument");
+  *clusters = b->clusters ? 1 : 0;
   return AQ_OK;
 }
 

@@ -387,19 +387,29 @@ aq_status aq_batch_solve_stats(aq_batch* b, int32_t scene, aq_solve_stats* st);
  * per cluster size) instead, one more for the scenes that have outgrown theirs,
  * and the row sweeps' only for scenes that outgrow that one too. */
 aq_status aq_batch_launch_counts(const aq_batch* b, int32_t* per_step, int32_t* per_block);
+/* Kernel launches of a step as it runs, whichever solve it takes, outside the
+ * conditional parts of its graph (the residual loop of the row sweeps, the
+ * solves of scenes that have outgrown their cluster). */
+aq_status aq_batch_step_launches(const aq_batch* b, int32_t* launches);
+/* How the scenes are solved: 1, the default where every scene fits one, in a
+ * thread-block cluster each; 0 by the row sweeps.  1 is refused where a scene
+ * does not fit.  Iterates do not depend on it. */
+aq_status aq_batch_set_cluster_solve(aq_batch* b, int32_t clusters);
+aq_status aq_batch_get_cluster_solve(const aq_batch* b, int32_t* clusters);
 /* Caps every batched launch at multiple x SMs CTAs (default 64, i.e. as many
  * as are resident at once; a batched launch never exceeds one resident wave).
  * Results do not depend on it. */
 aq_status aq_batch_set_grid_multiple(aq_batch* b, int32_t multiple);
 /* Shape of the batched row sweep, which solves batches with a scene too large
- * for a thread-block cluster: x planes each warp streams (1, 2, 4 or
+ * for a thread-block cluster (or by aq_batch_set_cluster_solve): x planes each warp streams (1, 2, 4 or
  * 8; default 1) and, for more than one plane, whether the next plane's loads
  * are issued before the current plane's arithmetic.  Results do not depend
  * on it. */
 aq_status aq_batch_set_sweep_plan(aq_batch* b, int32_t x_planes, int32_t pipelined);
 aq_status aq_batch_get_sweep_plan(const aq_batch* b, int32_t* x_planes, int32_t* pipelined);
 /* Project-written autotuner of the batched sweep: times every sweep plan on
- * the current pressure systems (advances the iterates), keeps the fastest. */
+ * the current pressure systems (advances the iterates), keeps the fastest.
+ * How the scenes are solved stays as it is. */
 aq_status aq_batch_autotune(aq_batch* b, int32_t sweeps_per_trial, int32_t* x_planes, int32_t* pipelined,
                             float* sweep_us);
 /* Times `sweeps` batched Jacobi sweeps of the current pressure systems of all

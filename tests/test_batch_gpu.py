@@ -122,3 +122,56 @@ def test_batch_launch_counts_and_benchmark():
         r = b.benchmark_pressure(40)
         assert r["ms"] > 0
         assert 0 < r["cells_per_sweep"] <= b.totals()["cells"]
+
+
+@pytest.mark.parametrize("solver", [
+    dict(solve_mode=_abi.SOLVE_FIXED, pressure_init=_abi.PRESSURE_CARRY, pressure_iterations=37),
+    dict(solve_mode=_abi.SOLVE_FIXED, pressure_init=_abi.PRESSURE_ZERO, pressure_iterations=40),
+    dict(solve_mode=_abi.SOLVE_RESIDUAL, pressure_init=_abi.PRESSURE_CARRY, rel_residual=1e-4, max_iterations=300,
+         check_interval=10),
+], ids=["fixed-odd", "fixed-even", "residual"])
+@pytest.mark.parametrize("planes,pipe", [(1, False), (2, False), (4, True), (8, False)])
+def test_row_sweeps_equal_clusters(solver, planes, pipe):
+    """The batch's two solves, with a scene without fluid, scenes that stop at
+    different counts and row sweeps of every shape."""
+    cfgs = _mixed_configs(**solver)
+    with aq.Batch(cfgs) as rows, aq.Batch(cfgs) as clusters:
+        assert rows.cluster_solve() and clusters.cluster_solve()
+        rows.set_cluster_solve(False)
+        rows.set_sweep_plan(planes, pipe)
+        assert not rows.cluster_solve()
+        for b in (rows, clusters):
+            b.step(3)
+            b.synchronize()
+        for s in range(len(cfgs)):
+            x, y = rows.download_scene(s, FIELDS), clusters.download_scene(s, FIELDS)
+            for k in FIELDS:
+                np.testing.assert_array_equal(x[k], y[k], err_msg=f"scene {s} field {k}")
+            sa, sb = rows.solve_stats(s), clusters.solve_stats(s)
+            for k in ("iterations", "fluid_cells", "converged", "blocks", "total_sweeps", "total_blocks"):
+                assert sa[k] == sb[k], (s, k)
+            # the same FP64 terms in another order: under 1e5 of them, each sum within n * 2^-53
+            assert abs(sa["rel_residual"] - sb["rel_residual"]) <= 1e5 * 2.0 ** -53 * sb["rel_residual"]
+        # back to clusters: the same steps again
+        rows.set_cluster_solve(True)
+        rows.step(1)
+        clusters.step(1)
+        np.testing.assert_array_equal(rows.download_scene(0, FIELDS)["pressure"],
+                                      clusters.download_scene(0, FIELDS)["pressure"])
+
+
+def test_step_launches_are_those_of_the_solve_taken():
+    cfgs = batch_configs(3, seed=5, sizes=(16,), solve_mode=_abi.SOLVE_RESIDUAL, check_interval=20,
+                         max_iterations=200)
+    with aq.Batch(cfgs) as b:
+        assert b.step_launches() == 6 + 4 + 1 + 4  # sort; up to the solve; one cluster width; behind it
+        b.set_cluster_solve(False)
+        assert b.step_launches() == 6 + 5 + 4      # the row list; the loop's launches are launch_counts()'s
+    cfgs.append(_abi.make_config((160, 160, 160), [dict(shape="box", min=(0, 0, 0), max=(1, 0.05, 1))],
+                                 **{k: getattr(cfgs[0], k) for k in (
+                                     "timestep", "solve_mode", "pressure_init", "pressure_iterations", "rel_residual",
+                                     "max_iterations", "check_interval")}))
+    with aq.Batch(cfgs) as b:
+        assert not b.cluster_solve()
+        with pytest.raises(aq.AquariusError):
+            b.set_cluster_solve(True)
