@@ -193,6 +193,9 @@ def batch_traffic(cells: int):
         return None
 
 
+CLUSTER_UNIT_CLOCKS = 36  # shared-memory clocks of 32 units' sweep (16-byte rows, k_cluster.cu)
+
+
 def measured_hbm_peak():
     try:
         d = json.loads(MEASURED_PEAKS.read_text())
@@ -745,7 +748,7 @@ def run_batch(args, rank: int, world: int, dist):
         tune = b.autotune(50)
     b.step(1)
     b.synchronize()
-    per_step, per_block = b.launch_counts()
+    per_step, clusters = b.step_launches(), b.cluster_solve()
     s0 = [b.solve_stats(i) for i in range(b.scene_count)]
 
     clocks = ClockSampler(dev)
@@ -767,8 +770,8 @@ def run_batch(args, rank: int, world: int, dist):
     s1 = [b.solve_stats(i) for i in range(b.scene_count)]
     # the solve loop runs until its slowest scene stops: loop blocks = max over scenes
     loop_blocks = max(x["total_blocks"] - y["total_blocks"] for x, y in zip(s1, s0))
-    # the step's launches outside the solve loop: a lower bound, as the loop's own
-    # depend on whether the scenes are solved by rows or in clusters
+    # the step's launches outside conditional graph nodes: a lower bound where the
+    # scenes are solved by row sweeps, whose loop is one
     launches = args.steps * per_step
     value = weak_scaling_value(args.steps, world, ms_max)
     sweeps = [x["total_sweeps"] - y["total_sweeps"] for x, y in zip(s1, s0)]
@@ -797,6 +800,22 @@ def run_batch(args, rank: int, world: int, dist):
     sweep_ms = jb["ms"] / 200
     cells = jb["cells_per_sweep"]
     achieved = JACOBI_BYTES_PER_CELL * cells / (sweep_ms / 1000.0) / 1e9
+    max_sweeps = max(sweeps) / args.steps
+    row_sweep = {"bound": "hbm", "kernel": f"kb_jacobi_rows<{tune['x_planes']}, {'pipelined' if tune['pipelined'] else 'plain'}> "
+                 "(one sweep of every live scene per launch, packed rows)",
+                 "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
+                 "frac": achieved / hbm_peak, "traffic": batch_traffic(cells),
+                 "algorithmic_bytes": f"{JACOBI_BYTES_PER_CELL} B per updated cell per sweep x {cells} cells",
+                 "sweep_us": sweep_ms * 1000.0}
+    # in clusters the iterate stays on chip: what a sweep cannot do without is the
+    # shared-memory traffic of its units (8 cells each)
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    unit_sweeps = sum(x["fluid_cells"] / 8 * n for x, n in zip(s1, sweeps)) / args.steps
+    smem_ms = unit_sweeps * CLUSTER_UNIT_CLOCKS / 32 / (sms * (clk["sm_max_mhz"] or 1965) * 1e3)
+    cluster = {"bound": "shared memory", "kernel": "kb_cluster_solve (one thread-block cluster a scene, every sweep of "
+               "the solve in one launch)", "achieved": ms_max / args.steps, "peak": smem_ms,
+               "peak_kind": f"{CLUSTER_UNIT_CLOCKS} shared-memory clocks a warp of units and sweep, on {sms} SMs",
+               "unit": "ms a step (the solve's floor against the whole step)", "frac": smem_ms / (ms_max / args.steps)}
     line = {
         "metric": BATCH_METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": ms_max / args.steps, "higher_is_better": True, "scaling": "weak",
@@ -809,19 +828,15 @@ def run_batch(args, rank: int, world: int, dist):
                 "h2d_bytes_per_step": 2 * 12 * n, "d2h_bytes_per_step": 2 * 12 * n, "steps": e2e_steps,
                 "path": "aq_batch_step_host (C ABI), pinned host particle state of all scenes in and out"},
         "gpu_launches": int(launches),
-        "roofline": {"bound": "hbm", "kernel": f"kb_jacobi_rows<{tune['x_planes']}, {'pipelined' if tune['pipelined'] else 'plain'}> "
-                               "(one sweep of every live scene per launch, packed rows)",
-                     "achieved": achieved, "peak": hbm_peak, "peak_kind": peak_kind, "unit": "GB/s",
-                     "frac": achieved / hbm_peak, "traffic": batch_traffic(cells),
-                     "algorithmic_bytes": f"{JACOBI_BYTES_PER_CELL} B per updated cell per sweep x {cells} cells",
-                     "sweep_us": sweep_ms * 1000.0},
+        "roofline": cluster if clusters else row_sweep,
         "clocks": clk,
         "solver": {"mean_sweeps_per_scene_step": sum(sweeps) / len(sweeps) / args.steps,
-                   "max_sweeps_per_scene_step": max(sweeps) / args.steps,
+                   "max_sweeps_per_scene_step": max_sweeps,
                    "loop_blocks_per_step": loop_blocks / args.steps,
                    "scenes_converged_last_step": conv},
+        "solve": "one thread-block cluster a scene" if clusters else "row sweeps",
         "sweep_plan": {"x_planes_per_item": tune["x_planes"], "pipelined": tune["pipelined"],
-                       "tuned_sweep_us": tune["sweep_us"]},
+                       "tuned_sweep_us": tune["sweep_us"], "row_sweep_us": sweep_ms * 1000.0},
     }
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
         line["cpu_baseline"] = batch_cpu_sample(cfgs)
@@ -1049,6 +1064,7 @@ def run_profile_case(case: str):
     default plan; resident: the same system, 40 sweeps of the resident plan
     (one cooperative launch, 8x40x24 tiles, 384 threads); p2g: the same
     state, the particle-to-grid stage twice; batch-rows: 32 scenes of the batch set, 6 batched sweeps;
+    batch-clusters: the same scenes, 2 steps;
     conv: two U-Net inferences at 128^3 on seeded random inputs; mesh: two
     surface meshes of the 128^3 workload's initial particles; pbf / pcisph:
     one step of the solver at particle budget 3e6 (593k particles); render:
@@ -1088,6 +1104,13 @@ def run_profile_case(case: str):
         b.synchronize()
         b.set_sweep_plan(8, False)
         print(b.benchmark_pressure(6))
+        b.close()
+    elif case == "batch-clusters":
+        from aquarius_b200.scenes import batch_configs
+        b = aq.Batch(batch_configs(32, seed=BATCH_SEED, max_iterations=200))
+        b.step(2)
+        b.synchronize()
+        print(b.cluster_solve(), b.solve_stats(0))
         b.close()
     elif case in ("pbf", "pcisph"):
         from aquarius_b200 import _abi
@@ -1144,8 +1167,8 @@ def main():
     ap.add_argument("--no-reference-gpu", action="store_true",
                     help="skip timing the reference's own kernels (the plain-step comparator)")
     ap.add_argument("--reference-gpu-only", action="store_true", help=argparse.SUPPRESS)
-    ap.add_argument("--profile-case", choices=["jacobi", "resident", "p2g", "batch-rows", "conv", "mesh", "pbf",
-                                               "pcisph", "render"],
+    ap.add_argument("--profile-case", choices=["jacobi", "resident", "p2g", "batch-rows", "batch-clusters", "conv", "mesh",
+                                               "pbf", "pcisph", "render"],
                     default=None,
                     help="run one small fixed case for an ncu capture and exit")
     ap.add_argument("--workload", default="ball128",
