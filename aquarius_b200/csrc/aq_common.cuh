@@ -148,7 +148,8 @@ __device__ __forceinline__ u64 product2(u64 a, u64 b, u64 minus_zero) { return f
 // theorem: the first makes the quotient faithful, the second correct), where
 // nothing over- or underflows: |a| and |b| within 2^-60 .. 2^60, or a = 0.
 // Five FMAs and a check shared by up to three quotients, against a dozen
-// instructions and a branch each.
+// instructions and a branch each.  The remainders' signs are turned, which keeps
+// the sign of a zero quotient (for b > 0).
 struct Divisor {
   float b, y;
   bool ok;
@@ -158,8 +159,8 @@ __device__ __forceinline__ Divisor divisor(float b, float y) {
 }
 __device__ __forceinline__ float dvd_fast(float a, const Divisor& d) {
   const float q0 = __fmul_rn(a, d.y);
-  const float q1 = __fmaf_rn(__fmaf_rn(-q0, d.b, a), d.y, q0);
-  return __fmaf_rn(__fmaf_rn(-q1, d.b, a), d.y, q1);
+  const float q1 = __fmaf_rn(-__fmaf_rn(q0, d.b, -a), d.y, q0);
+  return __fmaf_rn(-__fmaf_rn(q1, d.b, -a), d.y, q1);
 }
 // 2 bits - 1 orders magnitudes, with 0 above all of them
 __device__ __forceinline__ unsigned mag_key(float a) { return 2u * __float_as_uint(a) - 1u; }

@@ -244,9 +244,12 @@ cudaError_t launch_resident_solve(cudaStream_t st, const Dims& d, int shape, int
                                   const float* rhs, const int8_t* type, const uint8_t* bact, int* tiles,
                                   int* n_tiles, unsigned int* bar, double* part, SolveState* ss, int fixed_sweeps,
                                   int check, int max_iters, double tol, BarrierTest bt);
-// Counts the float bit patterns where the resident sweep's division by 6
-// differs from the IEEE divide (*bad must start at 0).
+// Count the float bit patterns where a division by 6 differs from the IEEE
+// divide (added to *bad): the resident sweep's, the row sweeps' and the cluster
+// solve's, whose zeros may differ in sign.
 cudaError_t launch_div6_check(cudaStream_t st, unsigned long long* bad);
+cudaError_t launch_sixth4_check(cudaStream_t st, unsigned long long* bad);
+cudaError_t launch_cluster_div_check(cudaStream_t st, unsigned long long* bad);
 // fixed_sweeps > 0: that many sweeps then one residual; else residual mode.
 cudaError_t launch_persist_solve(cudaStream_t st, const Dims& d, int ctas, float* pa, float* pb, const float* rhs,
                                  const int8_t* type, const int* items, const int* n_items, unsigned int* bar,

@@ -1416,6 +1416,8 @@ aq_status aq_selfcheck_division(int32_t device, uint64_t* mismatches) {
   AQ_CUDA(cudaMalloc(&bad, sizeof(unsigned long long)));
   cudaError_t e = cudaMemset(bad, 0, sizeof(unsigned long long));
   if (e == cudaSuccess) e = launch_div6_check(nullptr, bad);
+  if (e == cudaSuccess) e = launch_sixth4_check(nullptr, bad);
+  if (e == cudaSuccess) e = launch_cluster_div_check(nullptr, bad);
   unsigned long long h = 0;
   if (e == cudaSuccess) e = cudaMemcpy(&h, bad, sizeof(h), cudaMemcpyDeviceToHost);
   cudaFree(bad);

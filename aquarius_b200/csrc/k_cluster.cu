@@ -221,7 +221,9 @@ __device__ __forceinline__ Quad sum_quad(const Quad& xp, const Quad& xm, const Q
 // (Markstein's; aq_selfcheck_division compares it with the IEEE divide over
 // all floats): exact for 0 and for finite |s| >= 2^-123, other sums divide.
 // r is 1/6 on fluid cells and 0 elsewhere, which makes the quotient of a
-// finite sum 0 there.
+// finite sum 0 there.  The sign of a zero may be another one than the divide's
+// (packed operands cannot be negated for nothing): a sum with a nonzero term
+// does not see it, and the solve's end stores zeros as +0.
 __device__ __forceinline__ Quad update_quad(const Quad& xp, const Quad& xm, const Quad& yp, const Quad& ym,
                                             const Quad& c, float zh, float zl, const Quad& rhs, const Quad& r) {
   const Quad s = sum_quad(xp, xm, yp, ym, c, zh, zl, rhs);
@@ -335,8 +337,9 @@ __device__ __forceinline__ Quad load_cells(const float* __restrict__ v, int cell
   r.w = len > 3 ? __ldcg(v + cell + 3) : r.z;
   return pack4(r);
 }
+// -0 is stored as +0, which the other plans write.
 __device__ __forceinline__ void store_cells(float* __restrict__ v, int cell, int len, const Quad& q) {
-  const float4 o = unpack4(q);
+  const float4 o = unpack4({add2(q.lo, 0ull), add2(q.hi, 0ull)});
   v[cell] = o.x;
   if (len > 1) v[cell + 1] = o.y;
   if (len > 2) v[cell + 2] = o.z;
@@ -665,6 +668,25 @@ __global__ void __launch_bounds__(kT, 1) kb_cluster_solve(BatchIndex bi, const i
   if (cluster_solve(S, a) && cluster_rank() == 0 && threadIdx.x == 0) live[s] = 0;
 }
 
+// Self-check of update_quad's quotients against the IEEE divide over all 2^32
+// bit patterns (zeros compare equal, NaN equal to NaN).
+__global__ void k_cluster_div_check(unsigned long long* bad) {
+  unsigned long long local = 0;
+  const unsigned stride = gridDim.x * blockDim.x;
+  const Quad none = pack4(make_float4(-0.f, -0.f, -0.f, -0.f));
+  for (unsigned long long i = blockIdx.x * blockDim.x + threadIdx.x; i <= 0xffffffffull; i += stride) {
+    const float x = __uint_as_float((unsigned)i);
+    const float4 q = unpack4(update_quad(pack4(make_float4(x, 1.f, 0.f, -x)), none, none, none, none, -0.f, -0.f, none,
+                                         sixths(15u)));
+    const float a[2] = {q.x, q.w}, e[2] = {__fdiv_rn(x, 6.f), __fdiv_rn(-x, 6.f)};
+    for (int k = 0; k < 2; ++k)
+      if (!(isnan(a[k]) && isnan(e[k])) && !(a[k] == 0.f && e[k] == 0.f) &&
+          __float_as_uint(a[k]) != __float_as_uint(e[k]))
+        ++local;
+  }
+  if (local) atomicAdd(bad, local);
+}
+
 // Launch configuration of `clusters` clusters of `width` CTAs.
 struct ClusterLaunch {
   cudaLaunchConfig_t lc = {};
@@ -743,6 +765,11 @@ cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, floa
   const ClusterScene S{d, pa, rhs, type, umap, list, part, ss};
   return cudaLaunchKernelEx(&l.lc, k_cluster_solve, S,
                             SolveArgs{fixed_sweeps, check, max_iters, tol, r2_only, spill});
+}
+
+cudaError_t launch_cluster_div_check(cudaStream_t st, unsigned long long* bad) {
+  k_cluster_div_check<<<148 * 8, 256, 0, st>>>(bad);
+  return cudaGetLastError();
 }
 
 // A batch fills the machine by its number of scenes, so a scene takes the

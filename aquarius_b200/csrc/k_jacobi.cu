@@ -191,7 +191,8 @@ __host__ __device__ __forceinline__ int resid_flat_parts_dev(const Dims& d) {
 }
 
 // RN(s / 6) for four sums: the corrected reciprocal product (see
-// k_resident.cu's div6_fast) where it is exact, else the divide.  One check
+// k_resident.cu's div6_fast) where it is exact, else the divide; the remainder
+// with its sign turned, which keeps the sign of a zero quotient.  One check
 // for the four instead of a branch in each divide: a sweep of the 128^3
 // workload's rows takes 2.65 us instead of 3.00.
 __device__ __forceinline__ float4 sixth4(const float4& s) {
@@ -202,7 +203,7 @@ __device__ __forceinline__ float4 sixth4(const float4& s) {
     const float r = 0x1.555556p-3f;
     auto q = [r](float v) {
       const float q0 = __fmul_rn(v, r);
-      return __fmaf_rn(__fmaf_rn(-q0, 6.0f, v), r, q0);
+      return __fmaf_rn(-__fmaf_rn(q0, 6.0f, -v), r, q0);
     };
     return make_float4(q(s.x), q(s.y), q(s.z), q(s.w));
   }
@@ -1730,6 +1731,29 @@ cudaError_t launch_batch_solve_condition(cudaStream_t st, const int* live, int n
 }  // namespace aqb
 
 namespace aqb {
+namespace {
+
+// Self-check of sixth4 against the IEEE divide over all 2^32 bit patterns, beside
+// sums that take its fast path where the pattern does (NaN equal to NaN).
+__global__ void k_sixth4_check(unsigned long long* bad) {
+  unsigned long long local = 0;
+  const unsigned stride = gridDim.x * blockDim.x;
+  for (unsigned long long i = blockIdx.x * blockDim.x + threadIdx.x; i <= 0xffffffffull; i += stride) {
+    const float x = __uint_as_float((unsigned)i);
+    const float4 q = sixth4(make_float4(x, 1.f, 0.f, -x));
+    const float a[2] = {q.x, q.w}, e[2] = {__fdiv_rn(x, 6.f), __fdiv_rn(-x, 6.f)};
+    for (int k = 0; k < 2; ++k)
+      if (!(isnan(a[k]) && isnan(e[k])) && __float_as_uint(a[k]) != __float_as_uint(e[k])) ++local;
+  }
+  if (local) atomicAdd(bad, local);
+}
+
+}  // namespace
+
+cudaError_t launch_sixth4_check(cudaStream_t st, unsigned long long* bad) {
+  k_sixth4_check<<<148 * 8, 256, 0, st>>>(bad);
+  return cudaGetLastError();
+}
 
 int row_items_capacity(const Dims& d) { return d.sx * d.sy * ((d.sz / 4 + 31) / 32); }
 

@@ -267,10 +267,11 @@ aq_status aq_fluid_test_barrier_timeout(aq_fluid* f, int32_t withhold_cta, uint3
  * (transferToCellAccumPhase, Fluid/Fluid_3D_FLIP.cu:8-70). */
 aq_status aq_p2g_set_variant(int32_t variant);
 
-/* Self-check of the resident solve's division by 6 (an FMA-corrected
- * reciprocal product on normal quotients) against the IEEE divide over all
- * 2^32 float bit patterns on `device`; *mismatches receives the count of
- * differing results (NaN equal to NaN).  No counterpart in the reference. */
+/* Self-check of the solves' divisions by 6 (FMA-corrected reciprocal products
+ * on normal quotients: the resident sweep's, the row sweeps' and the cluster
+ * solve's) against the IEEE divide over all 2^32 float bit patterns on `device`;
+ * *mismatches receives the count of differing results (NaN equal to NaN; in the
+ * cluster solve +0 equal to -0).  No counterpart in the reference. */
 aq_status aq_selfcheck_division(int32_t device, uint64_t* mismatches);
 
 /* Plan of the Jacobi kernels.  rows = 0: one vectorised sweep per launch

@@ -59,3 +59,16 @@ def test_cluster_solve_without_fluid():
         f.step(2)
         s = f.solve_stats()
         assert s["converged"] and s["iterations"] == 20 and s["rel_residual"] == 0.0
+
+
+def test_cluster_solve_writes_zeros_as_the_sweeps_do():
+    """Cells without fluid beside fluid ones hold +0 after a solve, whatever the
+    sign of the sums around them: bit patterns, not values, are compared."""
+    def pressure(plan):
+        with aq.Fluid(ball_drop((24, 20, 28), pool=0.4, pressure_iterations=30)) as f:
+            f.set_jacobi_plan(*plan)
+            f.step(4)
+            return f.download_state(["pressure"])["pressure"]
+    want = pressure((1, 3, 1))
+    assert (want < 0).any()
+    np.testing.assert_array_equal(pressure((1, 5, 16)).view(np.uint32), want.view(np.uint32))
