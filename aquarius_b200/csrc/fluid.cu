@@ -765,7 +765,7 @@ aq_status aq_fluid::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
                          : jacobi_launches(whole_solve(plan) ? JacobiPlan{1, 3, 1} : plan, kWarmSweeps) - 1) +
                 2;
   launches += 1 + 3 + (multiphase ? cfg.diffusion_iterations : 0) + (ink_on && n_ink > 0 ? 1 : 0);
-  if (sort && rest) graph_launches = launches;
+  if (rest) graph_launches = launches;  // of the whole step, also where the sort is a graph of its own
   cudaError_t e = cudaGraphInstantiate(out, g, 0);
   cudaGraphDestroy(g);
   if (e != cudaSuccess) { *out = nullptr; return fail(AQ_ERR_CUDA, std::string("instantiate: ") + cudaGetErrorString(e)); }

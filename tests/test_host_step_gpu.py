@@ -60,3 +60,13 @@ def test_batch_host_steps_equal_steps(sizes):
             np.testing.assert_array_equal(pos[:, at:at + m], want["position"])
             np.testing.assert_array_equal(vel[:, at:at + m], want["velocity_p"])
             at += m
+
+
+def test_launch_counts_after_host_steps_alone():
+    cfg = ball_drop((40, 36, 42), pool=0.5, pressure_iterations=30)
+    with aq.Fluid(cfg) as a, aq.Fluid(cfg) as b:
+        pos = np.empty((3, a.particleCount), np.float32)
+        a.step_host(1, None, None, pos, None)
+        b.step(1)
+        assert a.launch_counts() == b.launch_counts() != (0, 0)
+        assert a.launches_per_step() == b.launches_per_step()
