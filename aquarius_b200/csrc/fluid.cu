@@ -490,7 +490,7 @@ static aq_status enqueue_whole(aq_fluid* f, int fixed_sweeps) {
                            : enqueue_cluster(f, fixed_sweeps, 0);
 }
 
-// The row list of a spilled fluid's sweeps, whose plan is not the fluid's own.
+// The row list of an outgrown cluster's sweeps, whose plan is not the fluid's own.
 static aq_status enqueue_wide_rows(aq_fluid* f) {
   if (f->wide.by == 3) AQ_CUDA(launch_row_items(f->stream, f->d, f->bact, f->row_items, f->n_row_items));
   return AQ_OK;
@@ -504,10 +504,7 @@ aq_status aq_fluid::enq_sweeps_fixed(const JacobiPlan& p, int sweeps) {
 
 aq_status aq_fluid::enq_solve_fixed(int sweeps) {
   if (sweeps <= 0) return AQ_OK;
-  if (may_spill()) {
-    AQ_TRY(enqueue_wide_rows(this));
-    return enq_sweeps_fixed(wide, sweeps);
-  }
+  if (may_spill()) return enq_spilling(sweeps);
   return whole_solve(plan) ? enqueue_whole(this, sweeps) : enq_sweeps_fixed(plan, sweeps);
 }
 
@@ -534,10 +531,10 @@ aq_status aq_fluid::enq_solve_body(const JacobiPlan& plan, bool set_cond, unsign
 
 // Residual mode without a graph: the host reads the solve state after each block.
 aq_status aq_fluid::enq_solve_residual_eager() {
-  if (whole_solve(plan) && !may_spill()) return enqueue_whole(this, 0);
-  if (may_spill()) AQ_TRY(enqueue_wide_rows(this));
+  if (may_spill()) return enq_spilling(0);
+  if (whole_solve(plan)) return enqueue_whole(this, 0);
   for (int guard = 0; guard < 1000000; ++guard) {
-    AQ_TRY(enq_solve_body(may_spill() ? wide : plan, false, 0, nullptr));
+    AQ_TRY(enq_solve_body(plan, false, 0, nullptr));
     AQ_CUDA(cudaMemcpyAsync(ss_host, ss, sizeof(SolveState), cudaMemcpyDeviceToHost, stream));
     AQ_CUDA(cudaStreamSynchronize(stream));
     const SolveState& s = *ss_host;
@@ -709,6 +706,50 @@ aq_status aqb::add_conditional(cudaGraph_t g, cudaGraphConditionalHandle handle,
   return AQ_OK;
 }
 
+// Captures into g what `before` enqueues, the cluster solve (fixed sweeps, or 0:
+// residual mode) and, in a conditional node whose condition the cluster solve
+// sets, the sweeps over the whole machine of a fluid that it does not hold.
+template <class F>
+static aq_status capture_spilling(aq_fluid* f, cudaGraph_t g, int fixed, cudaGraphNode_t* last, F&& before) {
+  cudaGraphConditionalHandle handle;
+  cudaGraph_t body;
+  AQ_TRY(make_condition(g, 0, &handle));
+  AQ_TRY(capture_into(f->stream, g, nullptr, 0, [&]() -> aq_status {
+    AQ_TRY(before());
+    return enqueue_cluster(f, fixed, handle);
+  }));
+  AQ_TRY(add_conditional(g, handle, fixed == 0, last, &body));
+  return capture_into(f->stream, body, nullptr, 0, [&]() -> aq_status {
+    AQ_TRY(enqueue_wide_rows(f));
+    return fixed == 0 ? f->enq_solve_body(f->wide, true, handle, nullptr) : f->enq_sweeps_fixed(f->wide, fixed);
+  });
+}
+
+// Such a solve outside of a step's graph, as a graph of its own; its sweeps
+// where the stream is being captured and cannot launch one.
+aq_status aq_fluid::enq_spilling(int fixed) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  AQ_CUDA(cudaStreamIsCapturing(stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) {
+    if (fixed == 0) return fail(AQ_ERR_CUDA, "a residual solve cannot be captured");
+    AQ_TRY(enqueue_wide_rows(this));
+    return enq_sweeps_fixed(wide, fixed);
+  }
+  if (!exec_solve) {
+    cudaGraph_t g = nullptr;
+    cudaGraphNode_t last;
+    AQ_CUDA(cudaGraphCreate(&g, 0));
+    const aq_status st = capture_spilling(this, g, fixed, &last, [] { return AQ_OK; });
+    const cudaError_t e = st == AQ_OK ? cudaGraphInstantiate(&exec_solve, g, 0) : cudaSuccess;
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) exec_solve = nullptr;
+    AQ_TRY(st);
+    AQ_CUDA(e);
+  }
+  AQ_CUDA(cudaGraphLaunch(exec_solve, stream));
+  return AQ_OK;
+}
+
 // The whole step as one CUDA graph.  RESIDUAL mode puts the sweeps in a
 // conditional WHILE node whose body ends with the residual check that sets
 // the loop condition, so a step needs no host round trip.  Behind a cluster
@@ -737,22 +778,19 @@ aq_status aq_fluid::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
         return enq_post_solve();
       });
     }
-    cudaGraphConditionalHandle handle;
-    AQ_TRY(make_condition(g, spill ? 0 : 1, &handle));
-    AQ_TRY(capture_into(stream, g, nullptr, 0, [&]() -> aq_status {
-      AQ_TRY(before_solve());
-      return spill ? enqueue_cluster(this, fixed, handle) : AQ_OK;
-    }));
     cudaGraphNode_t node;
-    cudaGraph_t body;
-    AQ_TRY(add_conditional(g, handle, loop, &node, &body));
-    int bl = 0;
-    AQ_TRY(capture_into(stream, body, nullptr, 0, [&]() -> aq_status {
-      if (spill) AQ_TRY(enqueue_wide_rows(this));
-      return residual ? enq_solve_body(spill ? wide : plan, true, handle, &bl) : enq_sweeps_fixed(wide, fixed);
-    }));
-    if (spill) launches += 1;  // the cluster solve; the branch that may follow it is not counted
-    else body_launches = bl;
+    if (spill) {
+      launches += 1;  // the cluster solve; the branch that may follow it is not counted
+      AQ_TRY(capture_spilling(this, g, fixed, &node, before_solve));
+    } else {
+      cudaGraphConditionalHandle handle;
+      cudaGraph_t body;
+      AQ_TRY(make_condition(g, 1, &handle));
+      AQ_TRY(capture_into(stream, g, nullptr, 0, before_solve));
+      AQ_TRY(add_conditional(g, handle, true, &node, &body));
+      AQ_TRY(capture_into(stream, body, nullptr, 0,
+                          [&]() { return enq_solve_body(plan, true, handle, &body_launches); }));
+    }
     return capture_into(stream, g, &node, 1, [&]() { return enq_post_solve(); });
   };
   const aq_status st = build();
@@ -1732,24 +1770,14 @@ aq_status aq_fluid_benchmark_pressure(aq_fluid* f, int32_t sweeps, float* ms, in
   // The sweeps are captured into a graph and replayed, as inside a step.
   cudaGraph_t g = nullptr;
   AQ_CUDA(cudaGraphCreate(&g, 0));
-  auto build = [&]() -> aq_status {
-    cudaGraphConditionalHandle handle = 0;
-    if (f->may_spill()) AQ_TRY(make_condition(g, 0, &handle));
-    AQ_TRY(capture_into(f->stream, g, nullptr, 0, [&]() -> aq_status {
-      if (f->may_spill()) return enqueue_cluster(f, sweeps, handle);
-      return whole_solve(f->plan) ? enqueue_whole(f, sweeps)
-                                  : enqueue_sweeps_on(f, f->plan, f->pa, f->pb, sweeps, false, f->jpart);
-    }));
-    if (!f->may_spill()) return AQ_OK;
-    cudaGraphNode_t node;
-    cudaGraph_t body;
-    AQ_TRY(add_conditional(g, handle, false, &node, &body));
-    return capture_into(f->stream, body, nullptr, 0, [&]() -> aq_status {
-      AQ_TRY(enqueue_wide_rows(f));
-      return f->enq_sweeps_fixed(f->wide, sweeps);
-    });
-  };
-  const aq_status st = build();
+  cudaGraphNode_t last;
+  const aq_status st =
+      f->may_spill() ? capture_spilling(f, g, sweeps, &last, [] { return AQ_OK; })
+                     : capture_into(f->stream, g, nullptr, 0, [&]() -> aq_status {
+                         return whole_solve(f->plan)
+                                    ? enqueue_whole(f, sweeps)
+                                    : enqueue_sweeps_on(f, f->plan, f->pa, f->pb, sweeps, false, f->jpart);
+                       });
   if (st != AQ_OK) { cudaGraphDestroy(g); return st; }
   cudaGraphExec_t ex = nullptr;
   cudaError_t ce = cudaGraphInstantiate(&ex, g, 0);

@@ -149,6 +149,7 @@ struct aq_fluid {
   // The step in two graphs, split behind the sort: aq_fluid_step_host copies
   // the particles out (on `copy`) while the rest of its last step runs.
   cudaGraphExec_t exec_sort = nullptr, exec_rest = nullptr;
+  cudaGraphExec_t exec_solve = nullptr;  // enq_spilling's
   cudaStream_t copy = nullptr;
   cudaEvent_t sorted = nullptr, copied = nullptr;
   bool use_graph = true;
@@ -197,8 +198,8 @@ struct aq_fluid {
 
   aq_status allocate();
   aq_status alloc_cluster();
-  // the plan is a cluster that the fluid can outgrow: a step's graph then also
-  // holds the sweeps of `wide`, and work outside of a graph runs those
+  // the plan is a cluster that the fluid can outgrow: a solve is then a graph
+  // (the step's, or exec_solve outside of it) that also holds the sweeps of `wide`
   bool may_spill() const { return plan.by == 5 && !aqb::cluster_solve_holds(d, plan.xc); }
   aq_status seed_and_init();
   // stage enqueues (eager or under capture)
@@ -207,6 +208,7 @@ struct aq_fluid {
   aq_status enq_divergence();
   aq_status enq_solve_fixed(int sweeps);
   aq_status enq_sweeps_fixed(const JacobiPlan& p, int sweeps);  // sweeps and their residual
+  aq_status enq_spilling(int fixed);                            // may_spill(); 0: residual mode
   aq_status enq_solve_body(const JacobiPlan& p, bool set_cond, unsigned long long handle, int* launches);
   aq_status enq_solve_residual_eager();
   aq_status enq_learned_start();
@@ -234,7 +236,7 @@ struct aq_fluid {
                               const std::vector<float>& dens);
   int count_jacobi_launches(int sweeps) const;
   void invalidate_graph() {
-    for (cudaGraphExec_t* e : {&exec, &exec_sort, &exec_rest}) {
+    for (cudaGraphExec_t* e : {&exec, &exec_sort, &exec_rest, &exec_solve}) {
       if (*e) cudaGraphExecDestroy(*e);
       *e = nullptr;
     }

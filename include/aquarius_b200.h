@@ -290,9 +290,8 @@ aq_status aq_selfcheck_division(int32_t device, uint64_t* mismatches);
  * their shared memory (levels 1, any sz, at most 16384 units of 2 x 1 x 4
  * cells per CTA; the default where the fluid fits).  A fluid that comes to
  * touch more units than the CTAs' shared memory holds (2048 each) is swept as by
- * rows = 3 (sz % 4 == 0) or 16 instead, decided step by step on the device;
- * steps outside of a graph (aq_fluid_set_graph_mode, aq_fluid_run_stage) sweep
- * so on every grid of more units.  rows = 8, 16, 32:
+ * rows = 3 (sz % 4 == 0) or 16 instead, decided step by step on the device.
+ * rows = 8, 16, 32:
  * the temporally blocked kernel with `levels` sweeps (1, 2, 4, 8) per launch
  * over tiles of that many rows and x_planes planes.  Chosen per grid by the
  * tuner; invalid plans are rejected. */

@@ -77,6 +77,18 @@ def test_strewn_fluid_is_solved_by_the_machine_wide_sweeps(size, wide, mode):
     assert secs[1] <= 1.5 * secs[0]
 
 
+def test_stages_solve_a_pool_in_the_cluster():
+    """Outside of a step's graph too: the pressure stage of a fluid that its
+    cluster holds takes less than the tiled sweeps' (some 0.2 of it)."""
+    def stage(plan):
+        with aq.Fluid(ball_drop((90, 61, 75), pool=0.2, dt=0.001, pressure_iterations=200)) as f:
+            if plan is not None:
+                f.set_jacobi_plan(*plan)
+            f.step(2)
+            return min(f.profile_step()["pressure"] for _ in range(5))
+    assert stage(None) < 0.7 * stage((2, 16, 16))
+
+
 @pytest.mark.parametrize("mode", MODES)
 def test_strewn_scenes_of_a_batch_stay_the_scenes_alone(mode):
     sizes = [(16, 16, 16), (32, 32, 32), (96, 64, 96), (24, 32, 48)]  # 32^3: a wider cluster; 96 x 64 x 96: row sweeps
