@@ -212,13 +212,13 @@ bool cluster_solve_holds(const Dims& d, int width);               // whatever th
 bool cluster_solve_runs(int width);  // the current device holds such a cluster, alone and in a batch
 // fixed_sweeps > 0: that many sweeps then one residual; else residual mode.
 // part: one double per 32 units.  Starts from pa, result in pa.  r2_only (may
-// be null): the squared residual goes there and *ss is only read.  spill: the
-// graph condition that a fluid of too many units sets, whose solve is then
-// still to be done (0 only where cluster_solve_holds).
+// be null): the squared residual goes there and *ss is only read.  *spilled
+// becomes 1 for a fluid of too many units, whose solve is then still to be done
+// (null only where cluster_solve_holds).
 cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, const float* rhs,
                                  const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
                                  int fixed_sweeps, int check, int max_iters, double tol, double* r2_only,
-                                 unsigned long long spill);
+                                 int* spilled);
 // The same for the live scenes of order[0 .. scenes) of a batch, one cluster
 // each; a solved scene is no longer live.  scratch[s]: scene s's first entry in
 // umap and list, and in part.
@@ -227,7 +227,9 @@ cudaError_t launch_batch_cluster_solve(cudaStream_t st, const BatchIndex& bi, in
                                        const int2* scratch, int* live, float* pa, const float* rhs,
                                        const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
                                        int fixed_sweeps, int check, int max_iters, double tol,
-                                       unsigned long long spill);
+                                       int* spilled);
+// The graph condition `handle` from *spilled, which is 0 again.
+cudaError_t launch_spill_condition(cudaStream_t st, int* spilled, unsigned long long handle);
 // ---- resident solve (k_resident.cu) ------------------------------------------
 // Plan rows = 4: the whole solve in one cooperative launch, one CTA per SM;
 // a CTA keeps a tile (plan.xc selects the TX x TY x TZ shape) plus a K-cell

@@ -90,6 +90,7 @@ struct aq_batch {
   int2* cl_scratch = nullptr;
   int *cl_map = nullptr, *cl_list = nullptr;
   double* cl_part = nullptr;
+  int* cl_spilled = nullptr;  // some scene did not fit its cluster; one of 16 CTAs
   cudaStream_t cl_stream[kWidths] = {nullptr};
   cudaEvent_t cl_event[kWidths + 1] = {nullptr};
 
@@ -161,7 +162,7 @@ struct aq_batch {
   aq_status allocate();
   aq_status plan_clusters();
   aq_status enq_clusters(unsigned long long spill);
-  aq_status enq_wide_clusters(unsigned long long spill);
+  aq_status enq_wide_clusters(unsigned long long rows);
   aq_status add_scene(int s, aq_fluid* f);
   aq_status enq_sort();       // the step's particle stage
   aq_status enq_pre_solve();  // the rest up to the solve
@@ -256,6 +257,7 @@ aq_status aq_batch::plan_clusters() {
   AQB_TRY(alloc(&cl_map, (size_t)units));
   AQB_TRY(alloc(&cl_list, (size_t)units));
   AQB_TRY(alloc(&cl_part, (size_t)parts));
+  AQB_TRY(alloc(&cl_spilled, 2));
   AQB_CUDA(cudaMemcpyAsync(cl_order, order.data(), sizeof(int) * ns, cudaMemcpyHostToDevice, stream));
   AQB_CUDA(cudaMemcpyAsync(cl_scratch, scratch.data(), sizeof(int2) * ns, cudaMemcpyHostToDevice, stream));
   AQB_CUDA(cudaStreamSynchronize(stream));
@@ -273,20 +275,24 @@ aq_status aq_batch::enq_clusters(unsigned long long spill) {
     AQB_CUDA(cudaStreamWaitEvent(cl_stream[k], cl_event[kWidths], 0));
     AQB_CUDA(launch_batch_cluster_solve(cl_stream[k], bi, n, 1 << k, cl_order + cl_first[k], cl_scratch, live, pa, rhs,
                                         type, cl_map, cl_list, cl_part, ss, fixed, solver.check_interval,
-                                        solver.max_iterations, (double)solver.rel_residual, spill));
+                                        solver.max_iterations, (double)solver.rel_residual,
+                                        spill ? cl_spilled : nullptr));
     AQB_CUDA(cudaEventRecord(cl_event[k], cl_stream[k]));
     AQB_CUDA(cudaStreamWaitEvent(stream, cl_event[k], 0));
   }
+  if (spill) AQB_CUDA(launch_spill_condition(stream, cl_spilled, spill));
   return AQ_OK;
 }
 
-// The scenes still live, a cluster of 16 CTAs each.
-aq_status aq_batch::enq_wide_clusters(unsigned long long spill) {
+// The scenes still live, a cluster of 16 CTAs each; rows: the condition of the
+// row sweeps (0: 16 CTAs hold every scene).
+aq_status aq_batch::enq_wide_clusters(unsigned long long rows) {
   AQB_CUDA(launch_batch_cluster_solve(stream, bi, ns, 1 << (kWidths - 1), cl_order, cl_scratch, live, pa, rhs, type,
                                       cl_map, cl_list, cl_part, ss,
                                       solver.solve_mode == AQ_SOLVE_RESIDUAL ? 0 : solver.pressure_iterations,
                                       solver.check_interval, solver.max_iterations, (double)solver.rel_residual,
-                                      spill));
+                                      rows ? cl_spilled + 1 : nullptr));
+  if (rows) AQB_CUDA(launch_spill_condition(stream, cl_spilled + 1, rows));
   return AQ_OK;
 }
 
@@ -444,6 +450,7 @@ aq_status aq_batch::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
     if (clusters) {
       step_launches -= 1;  // no row list
       for (int k = 0; k < kWidths && solve; ++k) step_launches += cl_first[k + 1] > cl_first[k] ? 1 : 0;
+      if (solve && cl_spill) step_launches += 1;  // their condition
     } else if (!residual) {
       step_launches = graph_launches;
     }

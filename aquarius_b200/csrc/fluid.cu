@@ -318,6 +318,7 @@ aq_status aq_fluid::alloc_cluster() {
   const size_t q = (size_t)cluster_solve_units(d);
   AQ_TRY(alloc(&cl_list, q));
   AQ_TRY(alloc(&cl_part, q / 32 + 1));
+  AQ_TRY(alloc(&cl_spilled, 1));
   return alloc(&cl_map, q);
 }
 
@@ -440,7 +441,7 @@ aq_status aq_fluid::enq_learned_start() {
   auto start = [&](float* a, float* b, double* part) -> aq_status {
     if (!cluster) return enqueue_sweeps_on(this, wp, a, b, kWarmSweeps, true, part);
     AQ_CUDA(launch_cluster_solve(stream, d, plan.xc, a, rhs, type, cl_map, cl_list, cl_part, ss, kWarmSweeps, 0, 0,
-                                 0.0, part, 0));
+                                 0.0, part, nullptr));
     return AQ_OK;
   };
   AQ_TRY(start(pa, pb, jpart));
@@ -475,11 +476,12 @@ static aq_status enqueue_resident(aq_fluid* f, int fixed_sweeps) {
 
 // The whole solve as one launch of one cluster (plan.by == 5); spill: the
 // condition of the graph that runs enq_sweeps_fixed or a loop of
-// enq_solve_body where the fluid does not fit.
+// enq_solve_body where the fluid does not fit (0: it always does).
 static aq_status enqueue_cluster(aq_fluid* f, int fixed_sweeps, unsigned long long spill) {
   AQ_CUDA(launch_cluster_solve(f->stream, f->d, f->plan.xc, f->pa, f->rhs, f->type, f->cl_map, f->cl_list, f->cl_part,
                                f->ss, fixed_sweeps, f->cfg.check_interval, f->cfg.max_iterations,
-                               (double)f->cfg.rel_residual, nullptr, spill));
+                               (double)f->cfg.rel_residual, nullptr, spill ? f->cl_spilled : nullptr));
+  if (spill) AQ_CUDA(launch_spill_condition(f->stream, f->cl_spilled, spill));
   return AQ_OK;
 }
 
@@ -780,7 +782,7 @@ aq_status aq_fluid::capture_step(bool sort, bool rest, cudaGraphExec_t* out) {
     }
     cudaGraphNode_t node;
     if (spill) {
-      launches += 1;  // the cluster solve; the branch that may follow it is not counted
+      launches += 2;  // the cluster solve and its condition; the branch that may follow is not counted
       AQ_TRY(capture_spilling(this, g, fixed, &node, before_solve));
     } else {
       cudaGraphConditionalHandle handle;

@@ -126,6 +126,7 @@ struct aq_fluid {
   // cluster solve (plan rows 5): numbering of the fluid quads, residual partials
   int *cl_map = nullptr, *cl_list = nullptr;
   double* cl_part = nullptr;
+  int* cl_spilled = nullptr;  // 1: the fluid did not fit
 
   JacobiPlan plan{4, 16, 32};
   JacobiPlan wide{2, 16, 16};  // the grid's plan of sweeps over the whole machine (default without a cluster)

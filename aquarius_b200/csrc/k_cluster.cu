@@ -38,8 +38,8 @@
 //
 // A fluid may spread over more units than the cluster's shared memory holds (a
 // droplet occupies a whole unit).  The cluster then leaves the system as it is
-// and sets the graph condition that runs the solve's other branch, the sweeps
-// over the whole machine.
+// and sets a mark, from which a graph condition runs the solve's other branch, the
+// sweeps over the whole machine.
 #include <algorithm>
 #include <type_traits>
 
@@ -74,8 +74,7 @@ struct SolveArgs {
   int fixed_sweeps, check, max_iters;  // fixed_sweeps 0: residual mode
   double tol;
   double* r2_only;  // if set: where ||b - A p||^2 goes, and the solve state stays as it is
-  // set to 1 where the fluid's units do not fit; 0 where they always do
-  cudaGraphConditionalHandle spill;
+  int* spilled;     // set to 1 where the fluid's units do not fit (null: they always do)
 };
 
 // What every thread of the cluster knows of the running solve.
@@ -552,24 +551,15 @@ __device__ __forceinline__ void solve_units(const ClusterScene& S, const SolveAr
   else solve_shared<4, RAGGED>(S, a, v, s_red, smem);
 }
 
-// The solve's end.  Called out of line, with the running values by address: they
-// then live on the stack between a solve's checks, and the sweeps' registers
-// hold their units without spilling.
-__device__ __noinline__ void record(const ClusterScene& S, const SolveArgs& a, const Solve& v) {
-  if (a.r2_only) {
-    *a.r2_only = v.r2;
-    return;
-  }
-  SolveState* ss = S.ss;
-  ss->iterations = v.it0 + v.done;
-  ss->bodies += v.checks;
-  ss->total_sweeps += v.done;
-  ss->total_bodies += v.checks;
-  ss->r2 = v.r2;
-  ss->rel_residual = v.rel;
-  const bool finite = isfinite(v.rel);
-  if (!finite) ss->nonfinite = ss->nonfinite_seen = 1;
-  ss->converged = finite && v.rel <= a.tol ? 1 : 0;
+// The fluid does not fit.  Called out of line, with the running values by
+// address: they then live on the stack between a solve's checks and the sweeps'
+// registers hold their units without spilling (a sweep of 64 x 24 x 64 with 90k
+// fluid cells 1.28 us, 1.44 with 44 bytes spilled).  For the same reason another
+// kernel sets the graph's condition: a call of the device runtime in this one
+// costs registers.
+__device__ __noinline__ void outgrown(const SolveArgs& a, Solve& v) {
+  if (v.me == 0 && threadIdx.x == 0) *a.spilled = 1;
+  v.n = 0;
 }
 
 // Starts from pa; the result is in pa.  False where the fluid does not fit the
@@ -638,17 +628,29 @@ __device__ __forceinline__ bool cluster_solve(const ClusterScene& S, const Solve
   v.r2 = v.rel = -1.0;
   const unsigned smem = static_cast<unsigned>(__cvta_generic_to_shared(cl_smem));
   if (v.per > kCap) {  // the same in every CTA
-    if (v.me == 0 && tid == 0) cudaGraphSetConditional(a.spill, 1);
+    outgrown(a, v);
     return false;
   }
   if (d.sx % 2 || !vec) solve_units<true>(S, a, v, s_red, smem);
   else solve_units<false>(S, a, v, s_red, smem);
-  if (v.me == 0 && tid == 0) record(S, a, v);
+  if (v.me == 0 && tid == 0 && a.r2_only) {
+    *a.r2_only = v.r2;
+  } else if (v.me == 0 && tid == 0) {
+    SolveState* ss = S.ss;
+    ss->iterations = v.it0 + v.done;
+    ss->bodies += v.checks;
+    ss->total_sweeps += v.done;
+    ss->total_bodies += v.checks;
+    ss->r2 = v.r2;
+    ss->rel_residual = v.rel;
+    const bool finite = isfinite(v.rel);
+    if (!finite) ss->nonfinite = ss->nonfinite_seen = 1;
+    ss->converged = finite && v.rel <= a.tol ? 1 : 0;
+  }
   return true;
 }
 
-__global__ void __launch_bounds__(kT, 1)
-    k_cluster_solve(const __grid_constant__ ClusterScene S, const __grid_constant__ SolveArgs a) {
+__global__ void __launch_bounds__(kT, 1) k_cluster_solve(const __grid_constant__ ClusterScene S, SolveArgs a) {
   cluster_solve(S, a);
 }
 
@@ -658,7 +660,7 @@ __global__ void __launch_bounds__(kT, 1)
 __global__ void __launch_bounds__(kT, 1) kb_cluster_solve(BatchIndex bi, const int* __restrict__ order,
                                                         const int2* __restrict__ scratch, int* live, float* pa,
                                                         const float* rhs, const int8_t* type, int* umap, int* list,
-                                                        double* part, SolveState* ss, const __grid_constant__ SolveArgs a) {
+                                                        double* part, SolveState* ss, SolveArgs a) {
   const int s = order[blockIdx.x / cluster_size()];
   if (!__ldcg(live + s)) return;  // the same in all CTAs of the cluster: none clears it before all have met
   const SceneDesc& D = bi.scenes[s];
@@ -666,6 +668,12 @@ __global__ void __launch_bounds__(kT, 1) kb_cluster_solve(BatchIndex bi, const i
   const int c = D.c_off;
   const ClusterScene S{D.d, pa + c, rhs + c, type + c, umap + at.x, list + at.x, part + at.y, ss + s};
   if (cluster_solve(S, a) && cluster_rank() == 0 && threadIdx.x == 0) live[s] = 0;
+}
+
+// The condition from the mark of the cluster solves before, which it clears.
+__global__ void k_spill_condition(int* spilled, cudaGraphConditionalHandle handle) {
+  cudaGraphSetConditional(handle, *spilled ? 1 : 0);
+  *spilled = 0;
 }
 
 // Self-check of update_quad's quotients against the IEEE divide over all 2^32
@@ -758,13 +766,18 @@ bool cluster_solve_runs(int width) {
 cudaError_t launch_cluster_solve(cudaStream_t st, const Dims& d, int width, float* pa, const float* rhs,
                                  const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
                                  int fixed_sweeps, int check, int max_iters, double tol, double* r2_only,
-                                 unsigned long long spill) {
-  if (!spill && !cluster_solve_holds(d, width)) return cudaErrorInvalidValue;
+                                 int* spilled) {
+  if (!spilled && !cluster_solve_holds(d, width)) return cudaErrorInvalidValue;
   if (const cudaError_t e = allow_solve()) return e;
   ClusterLaunch l(st, 1, width);
   const ClusterScene S{d, pa, rhs, type, umap, list, part, ss};
   return cudaLaunchKernelEx(&l.lc, k_cluster_solve, S,
-                            SolveArgs{fixed_sweeps, check, max_iters, tol, r2_only, spill});
+                            SolveArgs{fixed_sweeps, check, max_iters, tol, r2_only, spilled});
+}
+
+cudaError_t launch_spill_condition(cudaStream_t st, int* spilled, unsigned long long handle) {
+  k_spill_condition<<<1, 1, 0, st>>>(spilled, (cudaGraphConditionalHandle)handle);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_cluster_div_check(cudaStream_t st, unsigned long long* bad) {
@@ -790,12 +803,12 @@ cudaError_t launch_batch_cluster_solve(cudaStream_t st, const BatchIndex& bi, in
                                        const int2* scratch, int* live, float* pa, const float* rhs,
                                        const int8_t* type, int* umap, int* list, double* part, SolveState* ss,
                                        int fixed_sweeps, int check, int max_iters, double tol,
-                                       unsigned long long spill) {
+                                       int* spilled) {
   if (scenes <= 0) return cudaSuccess;
   if (const cudaError_t e = allow_batch_solve()) return e;
   ClusterLaunch l(st, scenes, width);
   return cudaLaunchKernelEx(&l.lc, kb_cluster_solve, bi, order, scratch, live, pa, rhs, type, umap, list, part, ss,
-                            SolveArgs{fixed_sweeps, check, max_iters, tol, nullptr, spill});
+                            SolveArgs{fixed_sweeps, check, max_iters, tol, nullptr, spilled});
 }
 
 }  // namespace aqb
