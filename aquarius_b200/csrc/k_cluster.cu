@@ -383,8 +383,10 @@ __device__ __forceinline__ void solve_loop(const ClusterScene& S, const SolveArg
 template <int U, bool RAGGED>
 __device__ __forceinline__ void solve_shared(const ClusterScene& S, const SolveArgs& a, Solve& v, double* s_red,
                                              unsigned smem) {
-  // 31 registers a unit with its iterate and its reciprocals, 15 with neither
-  constexpr bool KEEP_C = U <= 3, KEEP_R = U <= 2;
+  // 31 registers a unit with its iterate and its reciprocals, 15 with neither; two
+  // units with both leave no room to overlap them (64 x 24 x 64, 90k fluid cells:
+  // 1.41 us a sweep, 1.28 with the reciprocals made anew)
+  constexpr bool KEEP_C = U <= 3, KEEP_R = U <= 1;
   const Dims& d = S.d;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int nq = (d.sz + 3) / 4, plane = d.sy * d.sz;
@@ -553,13 +555,12 @@ __device__ __forceinline__ void solve_units(const ClusterScene& S, const SolveAr
 
 // The fluid does not fit.  Called out of line, with the running values by
 // address: they then live on the stack between a solve's checks and the sweeps'
-// registers hold their units without spilling (a sweep of 64 x 24 x 64 with 90k
-// fluid cells 1.28 us, 1.44 with 44 bytes spilled).  For the same reason another
+// registers hold their units with hardly a spill.  For the same reason another
 // kernel sets the graph's condition: a call of the device runtime in this one
-// costs registers.
+// costs registers (with both 192 bytes spilled and 12% longer sweeps).
 __device__ __noinline__ void outgrown(const SolveArgs& a, Solve& v) {
   if (v.me == 0 && threadIdx.x == 0) *a.spilled = 1;
-  v.n = 0;
+  v.n = -1;
 }
 
 // Starts from pa; the result is in pa.  False where the fluid does not fit the
@@ -627,12 +628,10 @@ __device__ __forceinline__ bool cluster_solve(const ClusterScene& S, const Solve
   v.done = v.checks = 0;
   v.r2 = v.rel = -1.0;
   const unsigned smem = static_cast<unsigned>(__cvta_generic_to_shared(cl_smem));
-  if (v.per > kCap) {  // the same in every CTA
-    outgrown(a, v);
-    return false;
-  }
-  if (d.sx % 2 || !vec) solve_units<true>(S, a, v, s_red, smem);
+  if (v.per > kCap) outgrown(a, v);  // the same in every CTA
+  else if (d.sx % 2 || !vec) solve_units<true>(S, a, v, s_red, smem);
   else solve_units<false>(S, a, v, s_red, smem);
+  if (v.n < 0) return false;
   if (v.me == 0 && tid == 0 && a.r2_only) {
     *a.r2_only = v.r2;
   } else if (v.me == 0 && tid == 0) {
