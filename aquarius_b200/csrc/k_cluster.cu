@@ -12,8 +12,8 @@
 // sweep per launch takes 1.6 us at 16^3 (row list) and 6.1 us at 50^3 (tiled
 // kernel, z not a multiple of 4); a cluster barrier with a read of another
 // CTA's shared memory takes 0.4 us at 16 CTAs (0.05 us at one CTA).  Measured
-// here, a sweep: 16^3 0.39 us (one CTA), 50^3 with 27k fluid cells 0.81 us,
-// 64^3 with 111k 1.53 us (row list 2.05), 90x61x75 with 132k 2.1 us (tiled
+// here, a sweep: 16^3 0.39 us (one CTA), 50^3 with 27k fluid cells 0.80 us,
+// 64^3 with 111k 1.50 us (row list 2.05), 90x61x75 with 132k 2.10 us (tiled
 // 6.2).  What bounds it now is the latency of a unit's dependent instructions
 // (few warps per scheduler) and the barrier.
 //
@@ -786,7 +786,7 @@ cudaError_t launch_cluster_div_check(cudaStream_t st, unsigned long long* bad) {
 
 // A batch fills the machine by its number of scenes, so a scene takes the
 // narrowest cluster that holds twice its initial fluid (up to kU units to a
-// thread cost a sweep 0.37 us each against 0.45 us for the cluster's barrier).
+// thread cost a sweep 0.37 us each against 0.4 us for the cluster's barrier).
 // Where the fluid has spread further the scene's solve goes to a cluster of 16
 // CTAs, and to the sweeps where even that does not hold it: the solve that the
 // scene has alone.

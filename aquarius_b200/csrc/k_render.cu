@@ -613,8 +613,9 @@ __global__ void __launch_bounds__(64) k_phase(RenderParams P, const int2* __rest
 // close on the screen; a box too large is counted in global memory) and adds
 // the box to the texture.  The tests are k_phase's, pixel for pixel.  A CTA
 // that meets another fraction sets *mixed; the texture is then void.
-// 5.2M sprites in a 1728x864 window: 342 us, against 1.3 ms of k_phase and
-// the 0.5 ms of the lists and their sort.
+// 5.2M sprites in a 1728x864 window: 345 us, against 1.3 ms of k_phase and
+// the 0.5 ms of the lists and their sort.  Frames of large sprites are faster by
+// the lists (counting_pays in render.cu).
 constexpr int kSplat = 512, kSplatBox = 5120;  // pixels; two words each
 __global__ void __launch_bounds__(kSplat) k_phase_splat(RenderParams P, const float* __restrict__ pts, int n,
                                                        float* __restrict__ phase,

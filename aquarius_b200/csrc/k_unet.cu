@@ -387,9 +387,9 @@ __host__ __device__ constexpr int tmem_cols(int n) {
 // shared memory: two being loaded, one whose MMAs run, one that waits; finished
 // output planes are written meanwhile.  The weights are loaded once a CTA.
 // 128^3 in us, against a CTA that loaded a 2-plane halo and all weights, issued
-// an MMA a tap and stored: 48 -> 16 channels 427 -> 231 (400 with the wide MMAs
-// alone), 16 -> 16 148 -> 98, 64^3 32 -> 32 82 -> 41; the network's inference
-// 1.23 -> 0.80 ms.
+// an MMA a tap and stored: 48 -> 16 channels 427 -> 219 (400 with the wide MMAs
+// alone), 16 -> 16 148 -> 96, 64^3 32 -> 32 82 -> 41; the network's inference
+// 1.23 -> 0.78 ms.
 constexpr int kUY = 16, kUZ = 8;
 constexpr int kUHY = kUY + 2, kUHZ = kUZ + 2;
 constexpr int kUChunk = kUHY * kUHZ * 16;  // bytes of one 8-channel chunk of a halo plane
@@ -421,7 +421,7 @@ __host__ __device__ constexpr bool umma_fits() {
 
 // SKIP > 0: the input's last SKIP channels are read from `skip`, the others from
 // `in` at half the resolution (the concatenation that k_upcat writes, without
-// writing it: 128^3, 32 + 16 channels, 245 us against 67 + 231).
+// writing it: 128^3, 32 + 16 channels, 236 us against 67 + 219).
 template <int CIN, int COUT, bool RELU, bool BIAS, int SKIP = 0>
 __global__ void __launch_bounds__(256) k_conv3_fwd_umma(const bf16* __restrict__ in, const bf16* __restrict__ skip,
                                                        const bf16* __restrict__ w, const float* __restrict__ bias,

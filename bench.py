@@ -1061,7 +1061,7 @@ def run_multiphase(args, rank: int, world: int, dist):
 def run_profile_case(case: str):
     """Small, fixed cases for single-kernel ncu captures (no JSON line):
     jacobi: the 128^3 workload's system after 3 steps, 6 sweeps of the
-    default plan; resident: the same system, 40 sweeps of the resident plan
+    default plan; cluster: a 50^3 ball drop's system, 100 sweeps in one cluster; resident: the 128^3 system, 40 sweeps of the resident plan
     (one cooperative launch, 8x40x24 tiles, 384 threads); p2g: the same
     state, the particle-to-grid stage twice; batch-rows: 32 scenes of the batch set, 6 batched sweeps;
     batch-clusters: the same scenes, 2 steps;
@@ -1089,6 +1089,13 @@ def run_profile_case(case: str):
             f.run_stage(_abi.STAGE_P2G)
         f.synchronize()
         print("p2g ok")
+        f.close()
+    elif case == "cluster":
+        from aquarius_b200 import _abi
+        f = aq.Fluid(_abi.make_config((50, 50, 50)))
+        f.step(3)
+        f.synchronize()
+        print(f.jacobi_plan(), f.benchmark_pressure(100), f.solve_stats()["fluid_cells"])
         f.close()
     elif case == "resident":
         f = aq.Fluid(workload_config(128, "zero"))
@@ -1167,7 +1174,7 @@ def main():
     ap.add_argument("--no-reference-gpu", action="store_true",
                     help="skip timing the reference's own kernels (the plain-step comparator)")
     ap.add_argument("--reference-gpu-only", action="store_true", help=argparse.SUPPRESS)
-    ap.add_argument("--profile-case", choices=["jacobi", "resident", "p2g", "batch-rows", "batch-clusters", "conv", "mesh",
+    ap.add_argument("--profile-case", choices=["jacobi", "cluster", "resident", "p2g", "batch-rows", "batch-clusters", "conv", "mesh",
                                                "pbf", "pcisph", "render"],
                     default=None,
                     help="run one small fixed case for an ncu capture and exit")
